@@ -1017,6 +1017,10 @@ __global__ void empty_pattern_kernel(const uint8_t* __restrict__ in, unsigned lo
 namespace {
 
 constexpr int kNBuf = 2;
+// Regions with up to this many matches are written as pieces: a piece costs about as many
+// instructions as an eighth of the scatter of a region (with 8 matches in most regions, 16 MiB of
+// ACGT took 58 us as pieces and 43 us scattered).
+constexpr uint32_t kPieceMax = 4;
 constexpr int kMaxSub = 8;
 
 
@@ -1025,34 +1029,33 @@ struct LayoutS {
   uint32_t masks_set, srec_set, wtab_set, wrec_set, subrec_set;  // bytes of one set of per-super-tile tables
   uint32_t mtab;                    // kModeMulti: the stage's pair table
   uint32_t rs, inbytes;
-  uint32_t wstage_words;  // padded staging words per warp (its 2 KiB of input may grow 3x)
+  uint32_t gmask;         // literal and kept-start masks of a warp's segments (emit_region)
+  uint32_t wstage_words;  // staging words per warp (kModeMulti: with padding words)
   uint32_t wstage_cap;    // bytes one warp can stage (before the padding words)
 };
 
-// Output bytes one 16 KiB sub-tile can produce, capped at three times its input.
-__host__ __device__ __forceinline__ uint32_t stage_ratio(uint32_t L, uint32_t R) {
-  if (L == 0 || R <= L) return 1;
-  const uint32_t r = (R + L - 1) / L;
-  return r < 3 ? r : 3;
-}
-
-// ratio: output staging per input byte (0: from L and R; a segmented launch passes the largest).
+// ratio: kModeMulti, output staging per input byte (1..3). The other modes stage 2 KiB per warp
+// whatever R is: a region whose output is larger is staged and written in rounds.
 // sets: per-super-tile tables held at once (2 when one super-tile's pass A overlaps the
 // previous one's look-back and pass B).
 __host__ __device__ __forceinline__ LayoutS make_layout_s(uint32_t mode, uint32_t L, uint32_t R, uint32_t nsub,
-                                                          uint32_t ratio = 0, uint32_t sets = 1) {
+                                                          uint32_t ratio = 1, uint32_t sets = 1) {
   LayoutS s{};
   uint32_t off = 0;
   s.inbytes = align_up_u32(kTile + (L > 1 ? L - 1 : 0), 16) + 32;
   s.in0 = off;
   off += kNBuf * s.inbytes;
   {
-    const uint32_t words = (2048u * (ratio ? ratio : stage_ratio(L, R)) + 48u) / 4u;
-    s.wstage_words = words + words / 32u + 2u;
+    const uint32_t words = (2048u * ratio + 48u) / 4u;
+    s.wstage_words = mode == kModeMulti ? words + words / 32u + 2u : words;  // (a multiple of 4: 16-byte rows)
     s.wstage_cap = words * 4u;
   }
   s.outb = off;
   off += align_up_u32(kWarps * s.wstage_words * 4u, 16);
+  if (mode != kModeMulti) {
+    s.gmask = off;
+    off += kWarps * 32u * 16u;
+  }
   s.masks = off;
   s.masks_set = nsub * kThreads * 8;
   off += sets * s.masks_set;
@@ -1382,33 +1385,6 @@ __device__ __forceinline__ void emit_literal(Emitter& e, const uint8_t* src, uin
   uint32_t i = 0;
   for (; i + 4 <= len; i += 4) e.append4(ld_u32_unaligned(src + i));
   for (; i < len; ++i) e.append1(src[i]);
-}
-
-// r copies of the replacement: rrep holds the replacement repeated (at least R + 8 bytes);
-// step4 = 4 mod R. When R divides 4 every word of the run is the same.
-__device__ __forceinline__ void emit_repeat(Emitter& e, const uint8_t* rrep, uint32_t R, uint32_t step4,
-                                            uint32_t r) {
-  uint32_t total = r * R;
-  if (step4 == 0u) {
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(rrep);
-    for (; total >= 4; total -= 4) e.append4(w);
-  } else {
-    uint32_t ph = 0;
-    for (; total >= 4; total -= 4) {
-      e.append4(ld_u32_unaligned(rrep + ph));
-      ph += step4;
-      if (ph >= R) ph -= R;
-    }
-    for (; total; --total) {
-      e.append1(rrep[ph]);
-      if (++ph == R) ph = 0;
-    }
-    return;
-  }
-  for (uint32_t ph = 0; total; --total) {
-    e.append1(rrep[ph]);
-    if (++ph == R) ph = 0;
-  }
 }
 
 // ---- short bordered patterns (L <= 4): segment functions packed in registers.
@@ -2158,6 +2134,85 @@ __device__ __forceinline__ void warp_emit_replace(uint8_t* out, const uint4* t16
   if (ok) out[b] = rs[mod_small((uint32_t)(b - g0) + ph0, R, rmag)];
 }
 
+// Staging bytes of segments [s0, s1) of a warp's region. gm[s]: segment s's literal bytes (x: low 32,
+// z: high 32) and kept starts (y, w); pk (lane s): staging position of its first byte in bits 0-15 and
+// the output length of its first 32 bytes in bits 16-31. A lane takes one byte of each 32: a
+// population count of the masks below it places the byte, so every step is the same few
+// instructions in every lane whatever the matches, and the 32 stores of a step are contiguous.
+// Bound by instruction issue; before, each lane walked its own matches and emitted words one after
+// the other, which cost a warp as much as its busiest lane at every step: 64 MiB of text, every
+// blank replaced by three bytes, 340 -> 115 us; line ends made CRLF, 149 -> 97 us.
+// ONE: L = 1 and every byte valid (literal = not kept). RC: R, or 5 for any R > 4.
+template <bool ONE, int RC>
+__device__ __forceinline__ void scatter_segments(uint8_t* stg, const uint8_t* src, const uint4* gm, uint32_t pk,
+                                                 uint32_t s0, uint32_t s1, uint32_t R, const uint8_t* rs) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t bit = 1u << lane, below = bit - 1u;
+  const uint32_t r4 = *reinterpret_cast<const uint32_t*>(rs);
+#pragma unroll 1
+  for (uint32_t s = s0; s < s1; ++s) {
+    const uint4 q = gm[s];
+    const uint32_t b = __shfl_sync(0xffffffffu, pk, s);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t C = h ? q.z : q.x, K = h ? q.w : q.y;
+      const uint32_t base = h ? (b & 0xFFFFu) + (b >> 16) : (b & 0xFFFFu);
+      const uint32_t kb = (uint32_t)__popc(K & below);
+      uint8_t* d = stg + base + (ONE ? lane - kb : (uint32_t)__popc(C & below)) +
+                   (RC == 5 ? kb * R : kb * (uint32_t)RC);
+      const uint8_t v = src[64u * s + 32u * (uint32_t)h + lane];
+      const bool mat = (K & bit) != 0u, lit = ONE ? !mat : (C & bit) != 0u;
+      if (RC == 0) {
+        if (lit) *d = v;
+      } else {
+        if (lit || mat) *d = mat ? (uint8_t)r4 : v;
+        if (RC >= 2 && mat) {
+          d[1] = (uint8_t)(r4 >> 8);
+          if (RC >= 3) d[2] = (uint8_t)(r4 >> 16);
+          if (RC >= 4) d[3] = (uint8_t)(r4 >> 24);
+          if (RC >= 5)
+            for (uint32_t r = 4; r < R; ++r) d[r] = rs[r];
+        }
+      }
+    }
+  }
+}
+
+template <bool ONE>
+__device__ __noinline__ void scatter_by_length(uint8_t* stg, const uint8_t* src, const uint4* gm, uint32_t pk,
+                                                  uint32_t s0, uint32_t s1, uint32_t R, const uint8_t* rs) {
+  switch (R) {  // the same in every lane
+    case 0: scatter_segments<ONE, 0>(stg, src, gm, pk, s0, s1, R, rs); break;
+    case 1: scatter_segments<ONE, 1>(stg, src, gm, pk, s0, s1, R, rs); break;
+    case 2: scatter_segments<ONE, 2>(stg, src, gm, pk, s0, s1, R, rs); break;
+    case 3: scatter_segments<ONE, 3>(stg, src, gm, pk, s0, s1, R, rs); break;
+    case 4: scatter_segments<ONE, 4>(stg, src, gm, pk, s0, s1, R, rs); break;
+    default: scatter_segments<ONE, 5>(stg, src, gm, pk, s0, s1, R, rs); break;
+  }
+}
+
+// A warp's staged bytes to out[g0, g0 + len): staging byte (g0 & 15) + i holds output byte i. Whole
+// 16-byte chunks as one store each; the partial chunks at both ends one byte per lane (the
+// neighbouring regions own their other bytes).
+__device__ __forceinline__ void warp_copy_staged(uint8_t* out, const uint8_t* stg, unsigned long long g0, uint32_t len) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const unsigned long long ga = g0 & ~15ull, gend = g0 + len;
+  const uint32_t c0 = (uint32_t)((g0 - ga + 15ull) >> 4);  // first whole chunk
+  const uint32_t c1 = (uint32_t)((gend - ga) >> 4);        // end of the whole chunks
+  for (uint32_t c = c0 + lane; c < c1; c += 32u)
+    st_out16(out + ga + ((unsigned long long)c << 4), *reinterpret_cast<const uint4*>(stg + (c << 4)));
+  unsigned long long b;
+  bool ok;
+  if (c0 < c1) {
+    b = lane < 16u ? g0 + lane : ga + ((unsigned long long)c1 << 4) + (lane - 16u);
+    ok = lane < 16u ? (b < ga + ((unsigned long long)c0 << 4)) : (b < gend);
+  } else {  // no whole chunk: fewer than 32 bytes
+    b = g0 + lane;
+    ok = b < gend;
+  }
+  if (ok) out[b] = stg[(uint32_t)(b - ga)];
+}
+
 // Input length, output range and super-tile count of the job described by p.
 struct JobDims {
   unsigned long long n_all, n, n16;
@@ -2261,8 +2316,8 @@ __global__ void __launch_bounds__(kThreads, 3)
   unsigned int* const sched = SEG ? sl.sched : &pk.res->tile_counter;  // claim counter, then finished CTAs
   const uint32_t nsub = SEG ? sl.nsub : pk.nsub;
   const LayoutS lay =
-      SEG ? make_layout_s(MODE, sl.Lmax, sl.Rmax, nsub, 3u)
-          : make_layout_s(MODE, pk.L, pk.R, nsub, MODE == kModeMulti ? pk.multi_ratio : 0u, 2u);
+      SEG ? make_layout_s(MODE, sl.Lmax, sl.Rmax, nsub)
+          : make_layout_s(MODE, pk.L, pk.R, nsub, MODE == kModeMulti ? pk.multi_ratio : 1u, 2u);
   uint8_t* ps = smem + lay.pat;
   uint8_t* rs = smem + lay.rep;
   uint8_t* ob = smem + lay.outb;
@@ -2274,7 +2329,7 @@ __global__ void __launch_bounds__(kThreads, 3)
   const uint32_t sb = tid * kSeg;
   const unsigned long long S = (unsigned long long)nsub * kTile;
   // the job's dimensions and pattern: once (one apply) or whenever the job changes (segmented)
-  uint32_t L = 0, R = 0, NT = 0, carry0 = 0, want_a = 0, step4 = 0, step512 = 0, rmag = 0;
+  uint32_t L = 0, R = 0, NT = 0, carry0 = 0, want_a = 0, step512 = 0, rmag = 0;
   unsigned long long n_all = 0, n = 0, n16 = 0;
   bool rep_table = false;
   bool run_pat = false;  // the pattern's first min(L, 4) bytes are its first byte repeated
@@ -2290,7 +2345,6 @@ __global__ void __launch_bounds__(kThreads, 3)
     R = p.R;
     rep_table = R >= 1u && R <= 64u;
     run_pat = ((p.p4 ^ ((p.p4 & 0xFFu) * 0x01010101u)) & p.m4) == 0u;
-    step4 = R ? 4u % R : 0u;
     step512 = R ? 512u % R : 0u;
     rmag = mod_magic(R);
     const uint8_t* psrc = (!SEG && L <= (uint32_t)kInlineMax) ? p.pat : p.pat_ext;
@@ -2509,8 +2563,8 @@ __global__ void __launch_bounds__(kThreads, 3)
             // (kModeMulti: the replacements differ, so no region is a run of one replacement)
             const bool full = MODE != kModeMulti && 2048u - wcov - wc * L + over == 0u;
             ok = __all_sync(0xffffffffu, !act || full);
-            // (kModeFree: a region with at most 16 matches is written as pieces in mode 2)
-            tin = __all_sync(0xffffffffu, !act || full || wc == 0u || (MODE == kModeFree && wc <= 16u));
+            // (kModeFree: emit_region writes any region in mode 2)
+            tin = __all_sync(0xffffffffu, !act || full || wc == 0u || MODE == kModeFree);
           }
         }
 #pragma unroll
@@ -2625,7 +2679,7 @@ __global__ void __launch_bounds__(kThreads, 3)
                          unsigned long long g0, uint32_t wtot) -> bool {
     const uint32_t cnt = (uint32_t)__popcll(kept);
     const uint32_t M = __reduce_add_sync(0xffffffffu, cnt);
-    if (M > 16u) return false;
+    if (M > (MODE == kModeMulti ? 16u : kPieceMax)) return false;
     uint32_t* desc = reinterpret_cast<uint32_t*>(ob) + (size_t)warp * lay.wstage_words;
     const uint32_t mb = warp_incl_scan(cnt, OpSum()) - cnt;  // this lane's first match index
     uint32_t i = 0;
@@ -2674,6 +2728,74 @@ __global__ void __launch_bounds__(kThreads, 3)
     }
     __syncwarp();
     return true;
+  };
+
+  // Output of one warp region (kModeFree, kModeSmall) that mixes literal bytes and replacements:
+  // out[g0, g0 + wtot). This thread's segment of the sub-tile at tb has the kept starts `kept`, its
+  // first x_in bytes covered by an earlier match and V valid bytes. Equal lengths: the replacements
+  // are written over the matches in shared memory and the region copied. At most kPieceMax
+  // matches: literal runs between replacements (emit_pieces). Otherwise the bytes are scattered
+  // into the warp's staging area (scatter_segments) and copied out, in rounds of as many segments
+  // as fit it (a segment that alone outgrows it goes straight to global memory).
+  // Lengths that do not add up to wtot (which the arithmetic rules out) report an error.
+  auto emit_region = [&](const uint8_t* tb, uint64_t kept, unsigned long long gseg, uint32_t x_in, uint32_t V,
+                         unsigned long long g0, uint32_t wtot) {
+    const uint32_t x0r = __shfl_sync(0xffffffffu, x_in, 0);
+    if (R == L) {
+      uint8_t* w = const_cast<uint8_t*>(tb) + sb;  // (a match may run past the segment: those bytes are its own)
+      for (uint64_t km = kept; km; km &= km - 1ull) {
+        const uint32_t b = (uint32_t)(__ffsll((long long)km) - 1);
+        for (uint32_t r = 0; r < R; ++r) w[b + r] = rs[r];
+      }
+      fence_proxy_async_smem();  // the buffer is loaded again by the async proxy
+      __syncwarp();
+      warp_emit_literal(p.out, tb, g0, wtot, warp * 2048u + x0r);
+      return;
+    }
+    if (emit_pieces(tb, kept, gseg, x0r, __reduce_add_sync(0xffffffffu, V), g0, wtot)) return;
+    // literal bytes: valid, not covered by the carry-in or by a match of this segment
+    uint64_t C = kept;
+    {
+      const uint32_t Lc = L < 64u ? L : 64u;
+      uint32_t w = 1;
+      for (; 2u * w <= Lc; w *= 2u) C |= C << w;
+      if (w < Lc) C |= C << (Lc - w);
+      C = ~C & ~low_bits(x_in) & low_bits(V);
+    }
+    const uint32_t low = (uint32_t)__popc((uint32_t)C) + (uint32_t)__popc((uint32_t)kept) * R;
+    const uint32_t olen = low + (uint32_t)__popc((uint32_t)(C >> 32)) + (uint32_t)__popc((uint32_t)(kept >> 32)) * R;
+    const uint32_t end = warp_incl_scan(olen, OpSum()), start = end - olen;
+    if (__shfl_sync(0xffffffffu, end, 31) != wtot) {
+      if (lane == 0) set_error(p);
+      return;
+    }
+    uint4* gm = reinterpret_cast<uint4*>(smem + lay.gmask) + warp * 32u;
+    uint8_t* stg = ob + (size_t)warp * lay.wstage_words * 4u;
+    gm[lane] = make_uint4((uint32_t)C, (uint32_t)kept, (uint32_t)(C >> 32), (uint32_t)(kept >> 32));
+    const bool one = __all_sync(0xffffffffu, L == 1u && V == 64u && x_in == 0u);
+    const uint8_t* src = tb + warp * 2048u;
+#pragma unroll 1
+    for (uint32_t s0 = 0; s0 < 32u;) {
+      const uint32_t from = __shfl_sync(0xffffffffu, start, s0);
+      const uint32_t over = __ballot_sync(0xffffffffu, lane >= s0 && end - from + 15u > lay.wstage_cap);
+      uint32_t s1 = over ? (uint32_t)__ffs(over) - 1u : 32u;
+      const bool direct = s1 == s0;  // one segment alone outgrows the staging (R > 32)
+      if (direct) ++s1;
+      const uint32_t to = __shfl_sync(0xffffffffu, end, s1 - 1u);
+      const unsigned long long gr = g0 + from;
+      const uint32_t pk = ((uint32_t)(gr & 15ull) + start - from) | (low << 16);
+      __syncwarp();  // the masks (and the last round's copies) are done
+      if (direct)
+        scatter_segments<false, 5>(p.out + (gr & ~15ull), src, gm, pk, s0, s1, R, rs);
+      else if (one)
+        scatter_by_length<true>(stg, src, gm, pk, s0, s1, R, rs);
+      else
+        scatter_by_length<false>(stg, src, gm, pk, s0, s1, R, rs);
+      __syncwarp();
+      if (to > from && !direct) warp_copy_staged(p.out, stg, gr, to - from);
+      s0 = s1;
+    }
+    __syncwarp();
   };
 
   // look-back, pass B and records of super-tile t, whose pass A filled set `set`; after the
@@ -2756,6 +2878,8 @@ __global__ void __launch_bounds__(kThreads, 3)
     unsigned long long O =
         p.len_bias + (unsigned long long)((long long)(tstart + cin) - (long long)carry0 + dprefix);
     const bool failed = s_fail != 0;
+    // a region's output of any length is staged in rounds (emit_region)
+    const bool stage_rounds = MODE != kModeMulti && R <= 64u;
 
     // ================= pass B, table-driven: every warp region of this whole super-tile is a run of
     // replacements, empty, or (mode 2) a copy of its input. Mode 2: lane r stands for region
@@ -2837,9 +2961,9 @@ __global__ void __launch_bounds__(kThreads, 3)
           0xffffffffu, wc ? (MODE == kModeFree ? jr * (uint32_t)kTile + we - L + 1u
                                                : jr * (uint32_t)kTile + wr * 2048u + x0 + (wc - 1u) * L + 1u)
                           : 0u);
-      // a region not shown by the fold: literal bytes beside kept matches (kModeFree: beside
-      // more than 16 of them; fewer are written as pieces)
-      const bool odd = __any_sync(0xffffffffu, olen_r != wc * R && wc > (MODE == kModeFree ? 16u : 0u));
+      // a region not shown by the fold: literal bytes beside kept matches (kModeFree: emit_region
+      // writes those)
+      const bool odd = MODE != kModeFree && __any_sync(0xffffffffu, olen_r != wc * R && wc > 0u);
       const bool fits_t = (O + total <= p.out_cap) && (O <= p.out_cap);
       if (!fits_t && tid == 0) atomicExch(&p.res->overflow_epoch, p.epoch);
       if (odd && tid == 0) set_error(p);
@@ -2859,9 +2983,13 @@ __global__ void __launch_bounds__(kThreads, 3)
             warp_emit_replace(p.out, reinterpret_cast<const uint4*>(smem + lay.tab16), rs, R, step512, rmag,
                               O + of, ol);
           } else if constexpr (MODE == kModeFree) {
-            // matches beside literal bytes (at most 16, as the fold checked; all kept in free mode)
-            emit_pieces(tb, masks_s[j * kThreads + tid], tstart + (unsigned long long)j * kTile + sb, xr, 2048u,
-                        O + of, ol);
+            // matches beside literal bytes; all are kept in free mode, and only the previous segment's
+            // last match reaches into a segment (L <= 64)
+            const uint64_t kept = masks_s[j * kThreads + tid];
+            const uint32_t e = kept ? 63u - (uint32_t)__clzll((long long)kept) + L : 0u;
+            const uint32_t pe = __shfl_up_sync(0xffffffffu, e, 1);
+            emit_region(tb, kept, tstart + (unsigned long long)j * kTile + sb,
+                        lane == 0 ? xr : (pe > 64u ? pe - 64u : 0u), 64u, O + of, ol);
           }
         }
         __syncthreads();
@@ -2937,8 +3065,8 @@ __global__ void __launch_bounds__(kThreads, 3)
           wbase = __shfl_sync(0xffffffffu, wbase, warp);
           sub_total = __shfl_sync(0xffffffffu, sub_total, 7);
           const bool fits0 = (O + sub_total <= p.out_cap) && (O <= p.out_cap);
-          const bool stage0 =
-              __reduce_max_sync(0xffffffffu, lane < 8u ? wolen : 0u) + 15u <= lay.wstage_cap;
+          const bool stage0 = stage_rounds ||
+                              __reduce_max_sync(0xffffffffu, lane < 8u ? wolen : 0u) + 15u <= lay.wstage_cap;
           const uint32_t wcw = __shfl_sync(0xffffffffu, ewc, warp);
           const uint32_t wlw = __shfl_sync(0xffffffffu, wolen, warp);
           const uint32_t x0w = __shfl_sync(0xffffffffu, ewcov, warp);  // bytes covered at the region start
@@ -3064,7 +3192,8 @@ __global__ void __launch_bounds__(kThreads, 3)
       // every warp's output of this sub-tile fits its staging area (with the up to 15 bytes of
       // alignment in front): the warp paths; otherwise the whole block writes windows. Lanes
       // 0-7 of every warp hold the eight lengths, so the choice is the same in every warp.
-      const bool warp_stage = __reduce_max_sync(0xffffffffu, lane < 8u ? wolen : 0u) + 15u <= lay.wstage_cap;
+      const bool warp_stage = stage_rounds ||
+                              __reduce_max_sync(0xffffffffu, lane < 8u ? wolen : 0u) + 15u <= lay.wstage_cap;
       if (!fits && tid == 0) atomicExch(&p.res->overflow_epoch, p.epoch);
       // kModeMulti: the warp's own sum of its threads' lengths must equal the length its slot was
       // given from the pass-A sums, or it would write over its neighbour; a mismatch (which the
@@ -3090,14 +3219,10 @@ __global__ void __launch_bounds__(kThreads, 3)
                             wtot);
         }
       } else if (fits && !failed && warp_stage) {
-        if (len_ok) {
-        bool pieces_done = false;
-        if constexpr (kFreeLike) {
-          // few matches in the region: literal runs between replacements
-          pieces_done = emit_pieces(tb, kept, gseg, __shfl_sync(0xffffffffu, x_in, 0),
-                                    __reduce_add_sync(0xffffffffu, V), O + wbase, wtot);
-        }
-        if (!pieces_done) {
+        if constexpr (MODE != kModeMulti) {
+        emit_region(tb, kept, gseg, x_in, V, O + wbase, wtot);
+        } else if (len_ok && !emit_pieces(tb, kept, gseg, __shfl_sync(0xffffffffu, x_in, 0),
+                                          __reduce_add_sync(0xffffffffu, V), O + wbase, wtot)) {
         uint32_t W[17];
         load_seg_words(tb + sb, W);
         // ---- this warp's output: assemble in its padded staging area, then copy out
@@ -3136,21 +3261,10 @@ __global__ void __launch_bounds__(kThreads, 3)
             if (nk > V) nk = V;
             if (nk > pos) emit_literal(e, src + pos, nk - pos);
             if (nk >= V) break;
-            if constexpr (MODE == kModeMulti) {  // this match's own replacement
-              const int k = multi_identify(MT, src + nk, n_all - (gseg + nk));
-              if (k < 0) break;  // cannot happen: pass A found this pattern here
-              emit_literal(e, MT.rep[k], MT.R[k]);
-              pos = nk + MT.L[k];
-              continue;
-            }
-            uint32_t r = 1;  // kept starts nk, nk+L, ... with nothing literal between them
-            if (L < 64u) {
-              const uint64_t holes = p.stride_mask & ~(kept >> nk);
-              const uint32_t h = holes ? (uint32_t)(__ffsll((long long)holes) - 1) : 64u;
-              r = ((h + L - 1) * p.inv_l) >> 16;
-            }
-            if (R) emit_repeat(e, rs, R, step4, r);
-            pos = nk + r * L;
+            const int k = multi_identify(MT, src + nk, n_all - (gseg + nk));  // this match's own replacement
+            if (k < 0) break;  // cannot happen: pass A found this pattern here
+            emit_literal(e, MT.rep[k], MT.R[k]);
+            pos = nk + MT.L[k];
           }
           e.finish();
         }
@@ -3186,8 +3300,7 @@ __global__ void __launch_bounds__(kThreads, 3)
             p.out[b] = sbytes[stg_pad(sbi >> 2) * 4u + (sbi & 3u)];
           }
         }
-        }  // !pieces_done
-        }  // len_ok
+        }  // kModeMulti, more than 16 matches
       } else if (fits && !failed) {
         // very large expansions: windows of the sub-tile output, byte by byte (the windows
         // share the staging area with the warps' own staging, which the block barrier at the
@@ -3593,7 +3706,7 @@ template <int MODE>
 cudaError_t launch_super_mode(const ReplaceParams& p, cudaStream_t st, int* grid_out) {
   static std::mutex mu;
   static unsigned long long attr_dev_mask = 0;
-  const uint32_t smem = make_layout_s(MODE, p.L, p.R, p.nsub, 0u, 2u).total;  // two sets of tables
+  const uint32_t smem = make_layout_s(MODE, p.L, p.R, p.nsub, 1u, 2u).total;  // two sets of tables
   int dev = 0;
   cudaGetDevice(&dev);
   {
@@ -3662,7 +3775,7 @@ cudaError_t launch_move_tail(const uint8_t* buf, const unsigned long long* total
   return cudaGetLastError();
 }
 
-uint32_t seg_smem_bytes(const SegLaunch& sl) { return make_layout_s(sl.mode, sl.Lmax, sl.Rmax, sl.nsub, 3u).total; }
+uint32_t seg_smem_bytes(const SegLaunch& sl) { return make_layout_s(sl.mode, sl.Lmax, sl.Rmax, sl.nsub).total; }
 
 namespace {
 template <int MODE>
