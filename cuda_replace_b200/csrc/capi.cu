@@ -488,7 +488,7 @@ int apply_one(Session* s, const uint8_t* pat, int pat_len, const uint8_t* rep, i
   memset(&p, 0, sizeof(p));
   crb::prepare_pattern_fields(p, pat, L);
   p.R = R;
-  p.nsub = crb::super_nsub(p.mode, L);
+  p.nsub = crb::super_nsub(p.mode, L, n);
   const size_t tile_bytes = (size_t)crb::kTile * (p.nsub ? p.nsub : 1u);
   const size_t tiles = (n + tile_bytes - 1) / tile_bytes;
   if (tiles > 0xFFFFFFF0ull) return (int)cudaErrorInvalidValue;
@@ -599,7 +599,7 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
       p.R = 0;
       p.agg_entries = 1;
       p.multi_ratio = T.ratio;
-      p.nsub = crb::super_nsub(crb::kModeFree, 1);
+      p.nsub = crb::super_nsub(crb::kModeMulti, 1, b);
       bnext = (size_t)crb::multi_output_bound(T, b);
       // the look-back sums sum(R - L) plus a bias per super-tile in 38-bit fields
       if ((b / ((size_t)crb::kTile * p.nsub) + 2) * crb::kMultiBias + bnext >= (1ull << 37)) return kFallback;
@@ -607,7 +607,7 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
       const int pl = pat_lens[k], rl = rep_lens[k];
       crb::prepare_pattern_fields(p, pats[k], (uint32_t)pl);
       p.R = (uint32_t)rl;
-      p.nsub = crb::super_nsub(p.mode, p.L);
+      p.nsub = crb::super_nsub(p.mode, p.L, b);
       if (!p.nsub) return kFallback;
       memcpy(p.pat, pats[k], (size_t)pl);
       if (rl) memcpy(p.rep, reps[k], (size_t)rl);
@@ -1025,7 +1025,7 @@ CR_EXPORT int cuda_replace_apply_device_async(void* h, const uint8_t* d_in, size
   memset(&p, 0, sizeof(p));
   crb::prepare_pattern_fields(p, pat, L);
   p.R = R;
-  p.nsub = crb::super_nsub(p.mode, L);
+  p.nsub = crb::super_nsub(p.mode, L, n);
   const size_t tile_bytes = (size_t)crb::kTile * (p.nsub ? p.nsub : 1u);
   const size_t tiles = (n + tile_bytes - 1) / tile_bytes;
   if (tiles > 0xFFFFFFF0ull) return (int)cudaErrorInvalidValue;
@@ -1118,7 +1118,8 @@ int unified_chunked(Session* s, const uint8_t* src, size_t n, const uint8_t* pat
   memset(&proto, 0, sizeof(proto));
   crb::prepare_pattern_fields(proto, pat, L);
   proto.R = R;
-  proto.nsub = crb::super_nsub(proto.mode, L);
+  const size_t chunk = std::max<size_t>((size_t)32 << 20, round_up((n + kUnifiedChunks - 1) / kUnifiedChunks, 1u << 20));
+  proto.nsub = crb::super_nsub(proto.mode, L, chunk);
   if (!proto.nsub) return kFallback;
   const size_t bound = output_bound(n, L, R);
   if (bound > 4 * n + ((size_t)64 << 20)) return kFallback;  // a large expansion: the single-launch path sizes it
@@ -1126,7 +1127,6 @@ int unified_chunked(Session* s, const uint8_t* src, size_t n, const uint8_t* pat
   memcpy(proto.pat, pat, L);
   if (R) memcpy(proto.rep, rep, R);
   const size_t P = L - 1;  // bytes held back at the end of every chunk but the last
-  const size_t chunk = std::max<size_t>((size_t)32 << 20, round_up((n + kUnifiedChunks - 1) / kUnifiedChunks, 1u << 20));
   // Chunk k uploads input [bnd(k), bnd(k + 1)) with bnd(k) = k * chunk + P for 0 < k: its
   // replace then starts P bytes earlier, at k * chunk, a 16-byte boundary as the loads need.
   size_t nchunks = (n + chunk - 1) / chunk;

@@ -1866,15 +1866,10 @@ __device__ __forceinline__ void ks_compose_n(uint32_t& t0, uint32_t& t1, uint32_
 
 // Kogge-Stone scan of the warp's 32 segment functions (L = LL <= 4): srec row of this
 // segment (carry into it for each warp carry-in) and, from lane 31, the warp function.
-// *dense (written by lane 0) tells whether the region is all candidates; then no table is
-// written and every reader uses the closed forms.
 template <int LL>
 __device__ __forceinline__ void ks_warp_tables(uint64_t mask, uint32_t inv_l, uint64_t stride, uint8_t* srec_row,
-                                               uint32_t* wtab_row, uint8_t* dense) {
+                                               uint32_t* wtab_row) {
   const uint32_t lane = threadIdx.x & 31u;
-  const bool all = __all_sync(0xffffffffu, mask == ~0ull);
-  if (lane == 0) *dense = all ? 1u : 0u;
-  if (all) return;  // closed forms (dense_region_entry, dense_seg_carry): no tables
   uint32_t ent[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
   for (uint32_t c = 0; c < (uint32_t)LL; ++c) {
@@ -1904,6 +1899,16 @@ __device__ __forceinline__ void ks_warp_tables(uint64_t mask, uint32_t inv_l, ui
       wtab_row[c] = (v & 0x3FFFu) | ((v >> 14) << 16);
     }
   }
+}
+
+// The same unless the region is all candidates: then no table is written, *dense is set and every
+// reader uses the closed forms (dense_region_entry, dense_seg_carry).
+template <int LL>
+__device__ __forceinline__ void ks_warp_tables(uint64_t mask, uint32_t inv_l, uint64_t stride, uint8_t* srec_row,
+                                               uint32_t* wtab_row, uint8_t* dense) {
+  const bool all = __all_sync(0xffffffffu, mask == ~0ull);
+  if ((threadIdx.x & 31u) == 0) *dense = all ? 1u : 0u;
+  if (!all) ks_warp_tables<LL>(mask, inv_l, stride, srec_row, wtab_row);
 }
 
 // 16 bytes starting r = 4q + sh/8 bytes into the 32 bytes (A, B); q is warp-uniform.
@@ -2179,7 +2184,7 @@ __device__ __forceinline__ void scatter_segments(uint8_t* stg, const uint8_t* sr
 }
 
 template <bool ONE>
-__device__ __noinline__ void scatter_by_length(uint8_t* stg, const uint8_t* src, const uint4* gm, uint32_t pk,
+__device__ __forceinline__ void scatter_by_length(uint8_t* stg, const uint8_t* src, const uint4* gm, uint32_t pk,
                                                   uint32_t s0, uint32_t s1, uint32_t R, const uint8_t* rs) {
   switch (R) {  // the same in every lane
     case 0: scatter_segments<ONE, 0>(stg, src, gm, pk, s0, s1, R, rs); break;
@@ -3475,6 +3480,1142 @@ __global__ void __launch_bounds__(kThreads, 3)
   }
 }
 
+// ============================================================================ region kernel
+// One apply in one launch, warp-specialised: a persistent CTA per SM of 24 worker warps and three
+// control warps. A super-tile is 48 KiB (nsub = 3), a 2 KiB region per worker warp, and stays in shared
+// memory from its single load until its output is written. The loader fills three slots by 1-D TMA bulk
+// copies, a whole super-tile ahead. For super-tile i a worker finds its region's candidates (pass A,
+// chunks in registers); the publisher folds the regions and publishes the super-tile's function; the
+// look-back warp resolves what the super-tiles before leave and places the regions' outputs, while
+// the workers write super-tile i - 1 (pass B, from shared memory) and search i + 1. Nobody but the
+// look-back warp waits for another CTA, and warps meet only at mbarriers, never at a block barrier.
+//
+// Why: with the input read twice (for the search and, after the look-back, for the output) the
+// second read came from L2 only while every CTA's super-tiles in flight fitted it (64 KiB super-tiles
+// read by three CTAs per SM with registers as the only staging read DRAM twice), each sub-tile
+// ended at a block barrier and the look-back's round trip stopped all eight warps of a CTA.
+namespace {
+
+constexpr uint32_t kRegion = 2048;
+constexpr uint32_t kWorkers = 24;                        // worker warps = regions of a super-tile
+// control warps (the look-backs of successive super-tiles alternate between two warps: one takes
+// 3500 cycles, most of it the round trip to the records, a super-tile at DRAM speed 4400)
+constexpr uint32_t kLoader = kWorkers, kPublisher = kWorkers + 1, kLookback = kWorkers + 2, kLookbacks = 2;
+constexpr uint32_t kRegionThreads = (kWorkers + 2 + kLookbacks) * 32;
+constexpr uint32_t kRegionSub = kWorkers * kRegion / kTile;  // nsub of the region kernel
+constexpr uint32_t kHaloMax = 272;                       // bytes after a super-tile held with it
+constexpr uint32_t kSlot = kWorkers * kRegion + kHaloMax + 48;
+constexpr uint32_t kSlots = 3;
+constexpr uint32_t kRegionPieces = 4;                    // regions with up to this many matches: pieces
+constexpr unsigned long long kPipeLimitNs = 6000000000ull;  // bounded wait inside a CTA (a look-back may take 2 s)
+static_assert(kRegionSub * kTile == kWorkers * kRegion, "super-tiles are whole sub-tiles (query kernel)");
+
+struct LayoutW {
+  uint32_t slots, masks, scratch, pat, rep, tab16, srec, wtab, wrec, total;
+  uint32_t srec_set, wtab_set, wrec_set;  // bytes per slot
+  uint32_t stage;                         // staged output bytes per worker
+};
+
+__host__ __device__ __forceinline__ LayoutW make_layout_w(uint32_t mode, uint32_t L, uint32_t R) {
+  LayoutW s{};
+  uint32_t off = 0;
+  s.slots = off;
+  off += kSlots * kSlot;
+  s.masks = off;
+  off += kSlots * kWorkers * 256u;
+  s.scratch = off;
+  s.stage = (mode == kModeFree && L <= 256u && R <= 256u) ? 1552u : 1040u;
+  off += kWorkers * (s.stage + 512u);  // and the segments' masks
+  s.pat = off;
+  off += align_up_u32(L ? L : 1, 16);
+  s.rep = off;
+  off += align_up_u32(R + 16, 16);
+  s.tab16 = off;  // replacement repeated, 16 bytes from every phase (R <= 64)
+  off += (R >= 1 && R <= 64) ? R * 16 : 0;
+  if (mode == kModeSmall) {
+    if (L <= 4u) {
+      s.srec = off;
+      s.srec_set = kWorkers * 32u * L;
+      off += kSlots * s.srec_set;
+    }
+    s.wtab = off;  // per region and carry: kept count (low half), carry-out
+    s.wtab_set = kWorkers * L * (L <= 4u ? 4u : 2u);
+    off += align_up_u32(kSlots * s.wtab_set, 16);
+    s.wrec = off;
+    s.wrec_set = kWorkers * L;
+    off += align_up_u32(kSlots * s.wrec_set, 16);
+  }
+  s.total = off;
+  return s;
+}
+
+// The four bytes at 4i of a chunk compared with the first NB pattern bytes at all four offsets:
+// a byte of the result is zero where all NB match (w: the word, wn: the next one; r[k]: pattern
+// byte k in every byte).
+template <int NB>
+__device__ __forceinline__ uint32_t diff_word(uint32_t w, uint32_t wn, const uint32_t r[4]) {
+  uint32_t d = w ^ r[0];
+  if (NB >= 2) d |= __funnelshift_r(w, wn, 8) ^ r[1];
+  if (NB >= 3) d |= __funnelshift_r(w, wn, 16) ^ r[2];
+  if (NB >= 4) d |= __funnelshift_r(w, wn, 24) ^ r[3];
+  return d;
+}
+// Nonzero in some bit 7 when a byte of some d folded in is zero (borrows only spread above a
+// real zero byte, so the answer for "any" is exact).
+__device__ __forceinline__ uint32_t zero_fold(uint32_t acc, uint32_t d) { return acc | ((d - 0x01010101u) & ~d); }
+// Bit i: byte i of d is zero (exact: no carry between bytes).
+__device__ __forceinline__ uint32_t zero_nibble(uint32_t d) {
+  const uint32_t nz = ((d & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | d;
+  return ((~nz & 0x80808080u) * 0x00204081u) >> 28;
+}
+template <int NB>
+__device__ __forceinline__ uint32_t detect_chunk(uint32_t acc, const uint4& q, uint32_t nx, const uint32_t r[4]) {
+  acc = zero_fold(acc, diff_word<NB>(q.x, q.y, r));
+  acc = zero_fold(acc, diff_word<NB>(q.y, q.z, r));
+  acc = zero_fold(acc, diff_word<NB>(q.z, q.w, r));
+  return zero_fold(acc, diff_word<NB>(q.w, nx, r));
+}
+template <int NB>
+__device__ __forceinline__ uint32_t mask_chunk(const uint4& q, uint32_t nx, const uint32_t r[4]) {
+  return zero_nibble(diff_word<NB>(q.x, q.y, r)) | (zero_nibble(diff_word<NB>(q.y, q.z, r)) << 4) |
+         (zero_nibble(diff_word<NB>(q.z, q.w, r)) << 8) | (zero_nibble(diff_word<NB>(q.w, nx, r)) << 12);
+}
+
+// A region in registers: lane l holds the 16-byte chunks l, l + 32, l + 64 and l + 96.
+struct RegionWords {
+  uint4 q0, q1, q2, q3;
+};
+__device__ __forceinline__ RegionWords load_region(const uint8_t* s) {
+  const uint4* v = reinterpret_cast<const uint4*>(s) + (threadIdx.x & 31u);
+  return RegionWords{v[0], v[32], v[64], v[96]};
+}
+// The first word after each of the lane's chunks (the next lane's chunk; for lane 31 the next row's
+// first one, held by lane 0, or the first word after the region).
+__device__ __forceinline__ void next_words(const RegionWords& w, uint32_t after, uint32_t nx[4]) {
+  const uint32_t lane = threadIdx.x & 31u, from = (lane + 1u) & 31u;
+  nx[0] = __shfl_sync(0xffffffffu, lane ? w.q0.x : w.q1.x, from);
+  nx[1] = __shfl_sync(0xffffffffu, lane ? w.q1.x : w.q2.x, from);
+  nx[2] = __shfl_sync(0xffffffffu, lane ? w.q2.x : w.q3.x, from);
+  nx[3] = __shfl_sync(0xffffffffu, lane ? w.q3.x : after, from);
+}
+template <int NB>
+__device__ __forceinline__ bool detect_region(const RegionWords& w, const uint32_t nx[4], const uint32_t r[4]) {
+  uint32_t acc = detect_chunk<NB>(0u, w.q0, nx[0], r);
+  acc = detect_chunk<NB>(acc, w.q1, nx[1], r);
+  acc = detect_chunk<NB>(acc, w.q2, nx[2], r);
+  acc = detect_chunk<NB>(acc, w.q3, nx[3], r);
+  return __any_sync(0xffffffffu, (acc & 0x80808080u) != 0u);
+}
+// Candidate masks of the lane's chunks (16 bits each: rows 0, 1 and rows 2, 3).
+template <int NB>
+__device__ __forceinline__ uint2 mask_region(const RegionWords& w, const uint32_t nx[4], const uint32_t r[4]) {
+  return make_uint2(mask_chunk<NB>(w.q0, nx[0], r) | (mask_chunk<NB>(w.q1, nx[1], r) << 16),
+                    mask_chunk<NB>(w.q2, nx[2], r) | (mask_chunk<NB>(w.q3, nx[3], r) << 16));
+}
+__device__ __forceinline__ uint32_t or_diff(uint32_t acc, const uint4& q, uint32_t rep) {
+  return acc | (q.x ^ rep) | (q.y ^ rep) | (q.z ^ rep) | (q.w ^ rep);
+}
+
+// Start of every run of L set bits in the 128 bits (hi, lo), for starts in lo (L <= 64).
+__device__ __forceinline__ uint64_t runs_of(uint64_t lo, uint64_t hi, uint32_t L) {
+  uint32_t w = 1;
+#pragma unroll 1
+  while (w < L) {
+    const uint32_t s = 2u * w <= L ? w : L - w;  // 1..32
+    lo &= (lo >> s) | (hi << (64u - s));
+    hi &= hi >> s;
+    w += s;
+  }
+  return lo;
+}
+
+// One step of the greedy over segments: blocked until x (relative to the region), segment s with
+// candidates `mask`. Adds the kept count to *cnt, returns the new x (patterns of 5..64 bytes: at most
+// 13 kept starts in a segment).
+__device__ __forceinline__ uint32_t walk_segment(uint32_t x, uint32_t s, uint64_t mask, uint32_t L, uint32_t* cnt) {
+  uint32_t y = x > 64u * s ? x - 64u * s : 0u;
+  bool any = false;
+  while (y < 64u) {
+    const uint64_t mm = mask >> y;
+    if (!mm) break;
+    y += (uint32_t)__ffsll((long long)mm) - 1u + L;
+    ++*cnt;
+    any = true;
+  }
+  return any ? 64u * s + y : x;
+}
+// The kept starts of that walk.
+__device__ __forceinline__ uint64_t walk_kept(uint32_t y, uint64_t mask, uint32_t L) {
+  uint64_t kept = 0;
+  while (y < 64u) {
+    const uint64_t mm = mask >> y;
+    if (!mm) break;
+    y += (uint32_t)__ffsll((long long)mm) - 1u;
+    kept |= 1ull << y;
+    y += L;
+  }
+  return kept;
+}
+
+// Bounded wait inside the CTA.
+__device__ __forceinline__ bool pipe_wait(const ReplaceParams& p, uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = global_ns();
+  for (;;) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (global_ns() - t0 > kPipeLimitNs) {
+      set_error(p);
+      return false;
+    }
+  }
+}
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// Look-back of kModeFree in the region kernel. Its carry-in is the reach recorded by the super-tile
+// before (no pattern is as long as a super-tile, so no older carry passes through one); its prefix is the
+// sum of the counts back to the nearest inclusive record. A window is 160 predecessors (with a
+// CTA per SM at most 148 super-tiles are between claim and record), five words per lane in one
+// round trip: windows of 32 took up to five round trips, which bounded the whole pipeline.
+struct SumWindow {
+  static constexpr int kPer = 5;
+  unsigned long long w[kPer];  // first record words of super-tiles base - lane - 32k
+  unsigned long long carry;    // lane 0, first window: the second word of the nearest record
+
+  __device__ __forceinline__ void load(const ReplaceParams& p, long long base, bool first) {
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const long long j = base - (long long)lane - 32 * k;
+      w[k] = 0;
+      if (j < 0) continue;
+      if (k == 0 && first && lane == 0)
+        rec_load(p.rec, (uint32_t)j, &w[0], &carry);
+      else
+        asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(w[k]) : "l"(p.rec + 2ull * (unsigned long long)j) : "memory");
+    }
+  }
+};
+__device__ __forceinline__ bool lookback_sum(const ReplaceParams& p, uint32_t t, unsigned long long* K_out,
+                                             uint32_t* c_out, uint32_t carry0) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const unsigned long long tag = p.epoch & 0xFFFFFFu;
+  unsigned long long acc = 0, t0 = 0;
+  long long base = (long long)t - 1;
+  bool first = true;
+  uint32_t ns = 32;
+  SumWindow W;
+  W.load(p, base, true);
+  for (;;) {
+    uint32_t D = 32u * SumWindow::kPer;  // distance of the nearest inclusive record
+    bool ready = true;
+    uint32_t part = 0;
+    unsigned long long Kd = 0;
+#pragma unroll
+    for (int k = 0; k < SumWindow::kPer; ++k) {
+      const long long j = base - (long long)lane - 32 * k;
+      const unsigned long long v = W.w[k];
+      uint32_t st = (v >> 40) == tag ? (uint32_t)(v >> 38) & 3u : 0u;
+      if (k == 0 && first && lane == 0 && ((W.carry >> 40) != tag || ((uint32_t)(W.carry >> 38) & 3u) != st)) st = 0;
+      if (j < 0) st = kStInc;  // the virtual super-tile before the first: nothing kept
+      const uint32_t okm = __ballot_sync(0xffffffffu, st != 0u), inc = __ballot_sync(0xffffffffu, st == (uint32_t)kStInc);
+      if (D == 32u * SumWindow::kPer) {  // (the same in every lane)
+        const uint32_t pl = inc ? (uint32_t)__ffs(inc) - 1u : 32u;
+        const uint32_t need = pl >= 31u ? 0xffffffffu : ((2u << pl) - 1u);
+        ready = ready && (okm & need) == need;
+        if (lane < pl) part += (uint32_t)rec_data(v);
+        if (inc) {
+          D = 32u * (uint32_t)k + pl;
+          Kd = __shfl_sync(0xffffffffu, j < 0 ? 0ull : rec_data(v), pl);
+        }
+      }
+    }
+    if (ready) {
+      if (first) {
+        const uint32_t c = base < 0 ? carry0 : (uint32_t)rec_data(W.carry);
+        *c_out = __shfl_sync(0xffffffffu, c, 0);
+        first = false;
+      }
+      acc += __reduce_add_sync(0xffffffffu, part);
+      if (D < 32u * SumWindow::kPer) {
+        *K_out = acc + Kd;
+        return true;
+      }
+      base -= 32 * SumWindow::kPer;
+    } else {
+      if (aborted(p)) return false;
+      const unsigned long long now = global_ns();
+      if (t0 == 0) {
+        t0 = now;
+      } else if (now - t0 > kSpinLimitNs) {
+        if (lane == 0) set_error(p);
+        return false;
+      }
+      __nanosleep(ns);
+      if (ns < 128) ns <<= 1;
+    }
+    W.load(p, base, first);
+  }
+}
+
+// Look-back for patterns of 5..64 bytes with a border: super-tile functions are tables over
+// carries in global memory; lane c holds entries c and (NE = 2) c + 32. 32 / NE predecessors per
+// window, their loads in flight together.
+template <int NE>
+__device__ __forceinline__ bool lookback_table(const ReplaceParams& p, uint32_t t, uint32_t L, unsigned long long* K_out,
+                                               uint32_t* c_out, uint32_t carry0) {
+  constexpr uint32_t W = 32u / NE;
+  const uint32_t lane = threadIdx.x & 31u;
+  unsigned long long acc_cnt[NE];  // function of the super-tiles between the window and t
+  uint32_t acc_carry[NE];
+#pragma unroll
+  for (int k = 0; k < NE; ++k) {
+    acc_cnt[k] = 0;
+    acc_carry[k] = lane + 32u * (uint32_t)k;
+  }
+  long long base = (long long)t - 1;
+  for (;;) {
+    uint32_t st;
+    const int plr = warp_wait_window(p, base, &st);
+    if (plr < 0) return false;
+    const uint32_t pl = min((uint32_t)plr, W);
+    uint32_t e[W][NE];
+#pragma unroll
+    for (uint32_t i = 0; i < W; ++i)
+#pragma unroll
+      for (uint32_t k = 0; k < (uint32_t)NE; ++k) {
+        e[i][k] = 0;
+        const uint32_t c = lane + 32u * k;
+        if (i < pl && c < L) {
+          const unsigned long long v = __ldcg(p.agg + (unsigned long long)(base - i) * L + c);
+          e[i][k] = (uint32_t)(v & 0x00FFFFFFull) | ((uint32_t)(v >> 32) << 24);
+        }
+      }
+    auto entry = [&](const uint32_t (&v)[NE], uint32_t x) -> uint32_t {
+      uint32_t r = __shfl_sync(0xffffffffu, v[0], x & 31u);
+      if (NE == 2) {
+        const uint32_t r1 = __shfl_sync(0xffffffffu, v[NE - 1], x & 31u);
+        if (x >= 32u) r = r1;
+      }
+      return r;
+    };
+    auto entry64 = [&](const unsigned long long (&v)[NE], uint32_t x) -> unsigned long long {
+      unsigned long long r = __shfl_sync(0xffffffffu, v[0], x & 31u);
+      if (NE == 2) {
+        const unsigned long long r1 = __shfl_sync(0xffffffffu, v[NE - 1], x & 31u);
+        if (x >= 32u) r = r1;
+      }
+      return r;
+    };
+    if (pl < W) {
+      unsigned long long K = 0;
+      uint32_t x = carry0;
+      const long long jp = base - (long long)pl;
+      if (jp >= 0) {
+        K = __ldcg(&p.incl[jp].kept);
+        x = __ldcg(&p.incl[jp].carry);
+      }
+#pragma unroll
+      for (int i = (int)W - 1; i >= 0; --i) {
+        if ((uint32_t)i < pl) {
+          const uint32_t v = entry(e[i], x);
+          K += v & 0x00FFFFFFu;
+          x = v >> 24;
+        }
+      }
+      *K_out = K + entry64(acc_cnt, x);
+      *c_out = entry(acc_carry, x);
+      return true;
+    }
+    // the whole window holds aggregates: compose it and put it in front of acc
+    unsigned long long wc[NE];
+    uint32_t y[NE];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const uint32_t c = lane + 32u * (uint32_t)k;
+      wc[k] = 0;
+      y[k] = c < L ? c : 0u;
+    }
+#pragma unroll
+    for (int i = (int)W - 1; i >= 0; --i)
+#pragma unroll
+      for (int k = 0; k < NE; ++k) {
+        const uint32_t v = entry(e[i], y[k]);
+        wc[k] += v & 0x00FFFFFFu;
+        y[k] = v >> 24;
+      }
+    unsigned long long ac[NE];
+    uint32_t ax[NE];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      ac[k] = wc[k] + entry64(acc_cnt, y[k]);
+      ax[k] = entry(acc_carry, y[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      acc_cnt[k] = ac[k];
+      acc_carry[k] = ax[k];
+    }
+    base -= W;
+  }
+}
+
+// Fold of up to 32 regions for patterns of LL <= 4 bytes (one warp): lane r holds region r's function
+// (the identity beyond nreg). A scan over the lanes gives the carry into every region for each
+// carry into the super-tile (wrec) and the super-tile's function (entry `lane`).
+template <int LL>
+__device__ __forceinline__ void fold_regions(const uint32_t* wt, const uint8_t* kind, uint8_t* wrec, uint32_t nreg,
+                                             uint32_t* sup_cnt, uint32_t* sup_carry) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t g[4];
+#pragma unroll
+  for (uint32_t y = 0; y < (uint32_t)LL; ++y) {
+    g[y] = y << 24;
+    if (lane < nreg) {
+      const uint32_t k = kind[lane];
+      const uint32_t v = k == 0u ? 0u : (k == 2u ? dense_region_entry(y, LL) : wt[lane * LL + y]);
+      g[y] = (v & 0xFFFFu) | ((v >> 16) << 24);
+    }
+  }
+  fn_scan_up<LL>(g, 1, 32, lane);
+  fn_scan_up<LL>(g, 2, 32, lane);
+  fn_scan_up<LL>(g, 4, 32, lane);
+  fn_scan_up<LL>(g, 8, 32, lane);
+  fn_scan_up<LL>(g, 16, 32, lane);
+#pragma unroll
+  for (uint32_t y = 0; y < (uint32_t)LL; ++y) {
+    uint32_t x = __shfl_up_sync(0xffffffffu, g[y], 1);
+    if (lane == 0) x = y << 24;
+    if (lane < nreg) wrec[lane * LL + y] = (uint8_t)(x >> 24);
+    const uint32_t e = __shfl_sync(0xffffffffu, g[y], 31);
+    if (lane == y) {
+      *sup_cnt = e & 0xFFFFFFu;
+      *sup_carry = e >> 24;
+    }
+  }
+}
+
+// The scatter of scatter_segments by R and shape; kept out of line: its twelve loops would crowd the
+// kernel's instruction cache (inlined, sparse inputs measured 3-4% slower).
+__device__ __noinline__ void scatter_any(uint8_t* stg, const uint8_t* src, const uint4* gm, uint32_t pk, uint32_t s0,
+                                         uint32_t s1, uint32_t R, const uint8_t* rs, bool one) {
+  if (one)
+    scatter_by_length<true>(stg, src, gm, pk, s0, s1, R, rs);
+  else
+    scatter_by_length<false>(stg, src, gm, pk, s0, s1, R, rs);
+}
+
+}  // namespace
+
+template <int MODE>
+__global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const __grid_constant__ ReplaceParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  // per slot: its load has landed; every worker's pass A is done; its function is known; its outputs
+  // are placed; every worker's pass B is done
+  __shared__ __align__(8) uint64_t s_full[kSlots], s_adone[kSlots], s_folded[kSlots], s_ready[kSlots], s_bdone[kSlots];
+  __shared__ uint32_t s_tile[kSlots];
+  __shared__ uint32_t s_wcnt[kSlots][kWorkers], s_wend[kSlots][kWorkers];  // kModeFree: kept count, end of the last match
+  __shared__ uint8_t s_kind[kSlots][kWorkers];  // kModeSmall: 0 no candidate, 1 mixed, 2 all candidates
+  // per region: output offset in the super-tile's, length, first byte not covered by an earlier
+  // match (relative to the super-tile), kept count
+  __shared__ uint4 s_reg[kSlots][kWorkers];
+  __shared__ unsigned long long s_O[kSlots];  // where the super-tile's output starts
+  __shared__ uint32_t s_total[kSlots], s_flags[kSlots], s_cin[kSlots];
+  __shared__ unsigned long long s_kept[kSlots];  // kept through the super-tile
+  __shared__ uint32_t s_supc[kSlots][64], s_supx[kSlots][64];  // its function: kept count, carry-out (kModeFree: entry 0)
+  __shared__ uint32_t s_last1[kSlots], s_cutlen[kSlots];  // kModeSmall: last kept start + 1; cut region's length
+  constexpr uint32_t kNone = 0xFFFFFFFFu;
+  constexpr uint32_t kWrite = 1u, kRuns = 2u, kCut = 4u;  // s_flags: write; all replacements; the region at n is cut
+
+  const uint32_t L = p.L, R = p.R;
+  const LayoutW lay = make_layout_w(MODE, L, R);
+  uint8_t* const ps = smem + lay.pat;
+  uint8_t* const rs = smem + lay.rep;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  constexpr unsigned long long S = (unsigned long long)kWorkers * kRegion;
+  const JobDims dims = job_dims(p, S);
+  const unsigned long long n_all = dims.n_all, n = dims.n, n16 = dims.n16;
+  const uint32_t NT = dims.NT, carry0 = dims.carry0;
+  const uint32_t halo = align_up_u32((L <= kHaloMax && L > 65u) ? L - 1u : 64u, 16);
+
+  // ---- loader warp, lane 0: load super-tile t into slot `slot` (kNone: no more)
+  auto issue = [&](uint32_t slot, uint32_t t) {
+    s_tile[slot] = t;
+    if (t == kNone) {
+      mbar_arrive(&s_full[slot]);
+      return;
+    }
+    const unsigned long long a = (unsigned long long)t * S;
+    const uint32_t bytes = (uint32_t)min(S + halo, n16 - a);
+    mbar_arrive_expect_tx(&s_full[slot], bytes);
+    bulk_load_hint(smem + lay.slots + slot * kSlot, p.in + a, bytes, &s_full[slot], l2_policy_evict_first());
+  };
+  auto claim = [&]() -> uint32_t {
+    const uint32_t c = atomicAdd(&p.res->tile_counter, 1u);
+    return c < NT ? c : kNone;
+  };
+  uint32_t issued = 0;  // loader: super-tiles and end marks issued
+  uint32_t marks = 0;   // ... end marks among them (one for each look-back warp)
+  if (tid == kLoader * 32u) {
+    for (uint32_t s = 0; s < kSlots; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&s_adone[s], kWorkers);
+      mbar_init(&s_folded[s], 1);
+      mbar_init(&s_ready[s], 1);
+      mbar_init(&s_bdone[s], kWorkers);
+      s_last1[s] = 0;
+      s_cutlen[s] = 0;
+    }
+    fence_mbar_init();
+    // one super-tile when every CTA gets at most one (none is taken from a CTA that starts late),
+    // else up to three ahead
+    const uint32_t share = (NT + gridDim.x - 1u) / gridDim.x;
+    const uint32_t depth = share < kSlots ? (share ? share : 1u) : kSlots;
+    for (; issued < depth && !marks; ++issued) {
+      const uint32_t t = claim();
+      marks = t == kNone ? 1u : 0u;
+      issue(issued, t);
+    }
+    if (share <= 1u) {
+      static_assert(kLookbacks < kSlots, "one super-tile and the end marks");
+      for (; marks < kLookbacks; ++marks) issue(issued++, kNone);
+    }
+  }
+  {
+    const uint8_t* psrc = L <= (uint32_t)kInlineMax ? p.pat : p.pat_ext;
+    const uint8_t* rsrc = R <= (uint32_t)kInlineMax ? p.rep : p.rep_ext;
+    for (uint32_t i = tid; i < L; i += kRegionThreads) ps[i] = psrc[i];
+    for (uint32_t i = tid; i < R + 16; i += kRegionThreads) rs[i] = R ? rsrc[i % R] : (uint8_t)0;
+    if (R >= 1u && R <= 64u) {
+      uint8_t* t16 = smem + lay.tab16;
+      for (uint32_t i = tid; i < R * 16u; i += kRegionThreads) t16[i] = rsrc[((i >> 4) + (i & 15u)) % R];
+    }
+  }
+  if (NT == 0 && blockIdx.x == 0 && tid == 0) {  // nothing to emit: still report
+    if (p.len_out) *p.len_out = p.len_bias;
+    if (p.carry_out) *p.carry_out = carry0 > n ? carry0 - (uint32_t)n : 0u;
+    p.res->out_len = 0;
+    p.res->kept = 0;
+  }
+  __syncthreads();
+
+  const uint32_t tag = p.epoch & 0xFFFFFFu;
+  const bool use_rec = MODE == kModeFree || L <= 4u;
+  // kModeSmall: region q's entry for carry y in slot `slot` (kept count, carry-out << 16)
+  auto region_entry = [&](uint32_t slot, uint32_t q, uint32_t y) -> uint32_t {
+    const uint32_t k = s_kind[slot][q];
+    if (k == 0u) return 0u;
+    if (k == 2u) return dense_region_entry(y, L);
+    const uint8_t* const wt = smem + lay.wtab + slot * lay.wtab_set;
+    if (L <= 4u) return reinterpret_cast<const uint32_t*>(wt)[q * L + y];
+    const uint32_t v = reinterpret_cast<const uint16_t*>(wt)[q * L + y];
+    return (v >> 6) | ((v & 63u) << 16);
+  };
+  // last kept start and totals of super-tile t (one lane)
+  auto record = [&](uint32_t t, unsigned long long O, uint32_t len, uint32_t l1, uint32_t cin, unsigned long long kept) {
+    const unsigned long long tstart = (unsigned long long)t * S;
+    const long long lastt = l1 ? (long long)(tstart + l1 - 1u) : -1ll;
+    __stcg(p.tile_last + t, lastt);
+    if (lastt >= 0)
+      atomicMax(&p.res->last_tagged, ((unsigned long long)p.epoch << 40) | (unsigned long long)(lastt + 1));
+    if (t == NT - 1) {
+      p.res->out_len = O + len - p.len_bias;
+      p.res->kept = kept;
+      if (p.len_out) *p.len_out = O + len;
+      if (p.carry_out) {
+        // coverage past the output range n: by the last kept match, or by the carry into
+        // this super-tile when no match starts in it
+        unsigned long long e = tstart + cin;
+        if (lastt >= 0 && (unsigned long long)lastt + L > e) e = (unsigned long long)lastt + L;
+        *p.carry_out = e > n ? (unsigned int)(e - n) : 0u;
+      }
+    }
+  };
+
+  if (warp == kLoader) {
+    // ================================================================ loader warp
+    // A slot is loaded again once every worker has written its part of the super-tile in it.
+    issued = __shfl_sync(0xffffffffu, issued, 0);
+    marks = __shfl_sync(0xffffffffu, marks, 0);
+    bool ok = true;
+    uint32_t done = 0;  // super-tiles written
+    auto finish = [&]() {
+      const uint32_t slot = done % kSlots;
+      ok = pipe_wait(p, &s_bdone[slot], (done / kSlots) & 1u);
+      if (MODE == kModeSmall && ok && lane == 0) {
+        record(s_tile[slot], s_O[slot], s_total[slot] + s_cutlen[slot], s_last1[slot], s_cin[slot], s_kept[slot]);
+        s_last1[slot] = 0;
+        s_cutlen[slot] = 0;
+      }
+      __syncwarp();
+      ++done;
+    };
+#pragma unroll 1
+    while (marks < kLookbacks && ok) {
+      if (issued >= kSlots) finish();
+      if (!ok) break;
+      uint32_t t = kNone;
+      if (lane == 0) {
+        if (!marks) t = claim();
+        issue(issued % kSlots, t);
+      }
+      t = __shfl_sync(0xffffffffu, t, 0);
+      marks += t == kNone ? 1u : 0u;
+      ++issued;
+    }
+    while (MODE == kModeSmall && ok && done + marks < issued) finish();
+    // after a wait that gave up: the loads in flight end before this CTA does
+    for (uint32_t j = done; !ok && j < issued; ++j) (void)wait_tile(&s_full[j % kSlots], (j / kSlots) & 1u);
+    if (lane == 0) {
+      __threadfence();
+      const unsigned int d = atomicAdd(&p.res->done_ctas, 1u);
+      if (d == gridDim.x - 1) {
+        atomicExch(&p.res->tile_counter, 0u);
+        atomicExch(&p.res->done_ctas, 0u);
+        __threadfence();
+      }
+    }
+    return;
+  }
+
+  if (warp == kPublisher) {
+    // ================================================================ publisher warp
+    // The super-tile's function, from its regions', published as soon as pass A is done: whatever this
+    // CTA's look-back waits for, later super-tiles elsewhere never wait for it.
+#pragma unroll 1
+    for (uint32_t i = 0;; ++i) {
+      const uint32_t slot = i % kSlots, par = (i / kSlots) & 1u;
+      if (!pipe_wait(p, &s_full[slot], par)) break;
+      const uint32_t t = s_tile[slot];
+      if (t == kNone || !pipe_wait(p, &s_adone[slot], par)) break;
+      if (MODE == kModeFree) {
+        const uint32_t wc = lane < kWorkers ? s_wcnt[slot][lane] : 0u;
+        const uint32_t we = lane < kWorkers ? s_wend[slot][lane] : 0u;
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, wc), top = __reduce_max_sync(0xffffffffu, we);
+        const uint32_t lco = top > (uint32_t)S ? top - (uint32_t)S : 0u;  // reach past the super-tile
+        if (lane == 0) {
+          if (t > 0) rec_store(p.rec, t, rec_word(tag, kStAgg, sum), rec_word(tag, kStAgg, lco));
+          s_supc[slot][0] = sum;
+          s_supx[slot][0] = lco;
+        }
+      } else if (L <= 4u) {
+        uint32_t sup_cnt = 0, sup_carry = 0;
+        uint8_t* const wrec = smem + lay.wrec + slot * lay.wrec_set;
+        const uint32_t* const wt = reinterpret_cast<const uint32_t*>(smem + lay.wtab + slot * lay.wtab_set);
+        if (L == 2u)
+          fold_regions<2>(wt, s_kind[slot], wrec, kWorkers, &sup_cnt, &sup_carry);
+        else if (L == 3u)
+          fold_regions<3>(wt, s_kind[slot], wrec, kWorkers, &sup_cnt, &sup_carry);
+        else
+          fold_regions<4>(wt, s_kind[slot], wrec, kWorkers, &sup_cnt, &sup_carry);
+        const unsigned long long e = lane < L ? ((unsigned long long)sup_cnt | ((unsigned long long)sup_carry << 17)) : 0ull;
+        const unsigned long long e1 = __shfl_sync(0xffffffffu, e, 1), e2 = __shfl_sync(0xffffffffu, e, 2),
+                                 e3 = __shfl_sync(0xffffffffu, e, 3);
+        if (lane == 0 && t > 0)
+          rec_store(p.rec, t, rec_word(tag, kStAgg, e | (e1 << 19)), rec_word(tag, kStAgg, e2 | (e3 << 19)));
+        if (lane < L) {
+          s_supc[slot][lane] = sup_cnt;
+          s_supx[slot][lane] = sup_carry;
+        }
+      } else {
+        uint8_t* const wrec = smem + lay.wrec + slot * lay.wrec_set;
+        for (uint32_t c = lane; c < L; c += 32u) {
+          uint32_t y = c, kc = 0;
+#pragma unroll 1
+          for (uint32_t q = 0; q < kWorkers; ++q) {
+            wrec[q * L + c] = (uint8_t)y;
+            const uint32_t v = region_entry(slot, q, y);
+            kc += v & 0xFFFFu;
+            y = v >> 16;
+          }
+          s_supc[slot][c] = kc;
+          s_supx[slot][c] = y;
+          if (t > 0) __stcg(p.agg + (unsigned long long)t * L + c, (unsigned long long)kc | ((unsigned long long)y << 32));
+        }
+        __threadfence();
+        __syncwarp();
+        if (t > 0 && lane == 0) st_release_u32(p.status + t, (p.epoch << 2) | kStAgg);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_folded[slot]);
+    }
+    return;
+  }
+
+  if (warp >= kLookback) {
+    // ================================================================ look-back warps
+#pragma unroll 1
+    for (uint32_t i = warp - kLookback;; i += kLookbacks) {
+      const uint32_t slot = i % kSlots, par = (i / kSlots) & 1u;
+      if (!pipe_wait(p, &s_full[slot], par)) break;
+      const uint32_t t = s_tile[slot];
+      if (t == kNone) break;
+      const unsigned long long tstart = (unsigned long long)t * S;
+      // ---- what the super-tiles before leave: kept count and carry. It needs nothing of this one, so
+      // it runs while the workers search this super-tile.
+      unsigned long long K = 0;
+      uint32_t c = carry0;
+      bool ok = true;
+      if (t > 0) {
+        if (MODE == kModeFree)
+          ok = lookback_sum(p, t, &K, &c, carry0);
+        else if (L == 2u)
+          ok = lookback_small_rec<2>(p, t, &K, &c, carry0);
+        else if (L == 3u)
+          ok = lookback_small_rec<3>(p, t, &K, &c, carry0);
+        else if (L == 4u)
+          ok = lookback_small_rec<4>(p, t, &K, &c, carry0);
+        else if (L <= 32u)
+          ok = lookback_table<1>(p, t, L, &K, &c, carry0);
+        else
+          ok = lookback_table<2>(p, t, L, &K, &c, carry0);
+      }
+      if (!ok) K = c = 0;
+      if (!pipe_wait(p, &s_folded[slot], par)) break;
+      const unsigned long long Kin = K + s_supc[slot][MODE == kModeFree ? 0u : c];
+      const uint32_t cout = s_supx[slot][MODE == kModeFree ? 0u : c];
+      if (lane == 0) {
+        if (use_rec) rec_store(p.rec, t, rec_word(tag, kStInc, Kin), rec_word(tag, kStInc, cout));
+        __stcg(&p.incl[t].kept, Kin);
+        __stcg(&p.incl[t].carry, cout);
+        if (!use_rec) {
+          __threadfence();
+          st_release_u32(p.status + t, (p.epoch << 2) | kStInc);
+        }
+      }
+      // ---- place the regions' outputs (lane q: region q). The output range starts len_bias bytes into
+      // out[], and the carry0 leading bytes covered by a match kept before this buffer are not emitted here.
+      const unsigned long long O = p.len_bias + (unsigned long long)((long long)(tstart + c) - (long long)carry0 +
+                                                                     (long long)K * ((long long)R - (long long)L));
+      const uint32_t tvalid = n - tstart < S ? (uint32_t)(n - tstart) : (uint32_t)S;
+      const uint32_t qs = lane * kRegion;
+      const uint32_t vb = (lane < kWorkers && tvalid > qs) ? min(tvalid - qs, kRegion) : 0u;
+      uint32_t wc = 0, x0 = qs, olen = 0, last1 = 0;
+      bool cut = false;  // kModeSmall: a region cut at n whose last match may run past n (exact length later)
+      if (MODE == kModeFree) {
+        uint32_t we = 0;
+        if (lane < kWorkers) {
+          wc = s_wcnt[slot][lane];
+          we = s_wend[slot][lane];
+        }
+        uint32_t cov = we;  // furthest end of a match before the region
+        if (L > kRegion) {
+#pragma unroll
+          for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, cov, d);
+            if (lane >= (uint32_t)d) cov = o > cov ? o : cov;
+          }
+        }
+        cov = __shfl_up_sync(0xffffffffu, cov, 1);  // (otherwise only the region before reaches here)
+        if (lane == 0) cov = 0;
+        cov = cov > c ? cov : c;
+        x0 = cov > qs ? cov : qs;
+        const uint32_t over = (wc && we > qs + vb) ? we - (qs + vb) : 0u;
+        olen = vb - min(x0 - qs, vb) - wc * L + over + wc * R;
+        last1 = __reduce_max_sync(0xffffffffu, wc ? we - L + 1u : 0u);
+      } else if (vb) {
+        const uint32_t cw = (smem + lay.wrec + slot * lay.wrec_set)[lane * L + c];
+        const uint32_t e = region_entry(slot, lane, cw);
+        wc = e & 0xFFFFu;
+        x0 = qs + cw;
+        olen = vb - min(cw, vb) - wc * L + (e >> 16) + wc * R;
+        cut = vb < kRegion && p.hold != 0ull && wc != 0u;
+        if (cut) olen = 0;
+      }
+      const uint32_t incl = warp_incl_scan(olen, OpSum());
+      const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+      const bool fits = O <= p.out_cap && total <= p.out_cap - O;
+      const bool runs = R <= 64u && __all_sync(0xffffffffu, olen == wc * R && !cut);
+      const bool cuts = __any_sync(0xffffffffu, cut);  // at most one region of the launch
+      if (lane < kWorkers) s_reg[slot][lane] = make_uint4(incl - olen, olen, x0, wc);
+      if (lane == 0) {
+        s_O[slot] = O;
+        s_total[slot] = total;
+        s_flags[slot] = (fits && ok ? kWrite : 0u) | (runs ? kRuns : 0u) | (cuts ? kCut : 0u);
+        s_cin[slot] = c;
+        s_kept[slot] = Kin;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&s_ready[slot]);
+        if (!fits) atomicExch(&p.res->overflow_epoch, p.epoch);
+        if (MODE == kModeFree) record(t, O, total, last1, c, Kin);
+      }
+      __syncwarp();
+    }
+    return;
+  }
+
+  // ================================================================== worker warps
+  const unsigned long long lim = (n_all >= L) ? min(n_all - L + 1, n) : 0ull;  // candidates p < lim
+  const uint32_t rmag = mod_magic(R), step512 = R ? 512u % R : 0u;
+  // every pattern byte the same (kModeSmall: candidates are runs of one byte)
+  const bool same = MODE == kModeFree ? L == 1u : p.same != 0u;
+  uint32_t r[4];  // first pattern bytes, each in every byte
+#pragma unroll
+  for (int k = 0; k < 4; ++k) r[k] = ((p.p4 >> (8 * k)) & 0xFFu) * 0x01010101u;
+  uint8_t* const stg = smem + lay.scratch + warp * (lay.stage + 512u);
+  uint4* const gm = reinterpret_cast<uint4*>(stg + lay.stage);
+  const uint32_t qs = warp * kRegion;  // this warp's region of every super-tile
+  bool hot = false;                    // the last region searched had a candidate: no detection pass
+
+  // ---- pass A: candidates of the warp's region of super-tile t and what the control warp needs of it
+  auto pass_a = [&](const uint32_t t, const uint32_t slot) {
+    const unsigned long long rstart = (unsigned long long)t * S + qs;
+    const uint8_t* const tb = smem + lay.slots + slot * kSlot + qs;
+    uint64_t* const row = reinterpret_cast<uint64_t*>(smem + lay.masks) + (slot * kWorkers + warp) * 32u;
+    uint32_t cnt = 0, end = 0, kind = 0;
+    bool found = rstart < n;
+    // presence index: no candidate can start in a chunk that lacks the first byte
+    if (found && p.presence)
+      found = (p.presence[(rstart >> p.presence_shift) * 8ull + ((p.p4 & 0xFFu) >> 5)] >> (p.p4 & 31u)) & 1u;
+    if (found) {
+      const RegionWords w = load_region(tb);
+      uint2 m2 = make_uint2(0, 0);
+      uint64_t after = 0;  // same: which of the 64 bytes after the region are the byte
+      bool uniform = false;
+      if (same) {
+        uint32_t d = or_diff(0u, w.q0, r[0]);
+        uniform = __all_sync(0xffffffffu, d == 0u);  // (most text fails on the first row)
+        if (uniform) {
+          d = or_diff(d, w.q1, r[0]);
+          d = or_diff(d, w.q2, r[0]);
+          d = or_diff(d, w.q3, r[0]);
+          uniform = __all_sync(0xffffffffu, d == 0u);
+        }
+        const uint32_t nx[4] = {0, 0, 0, 0};
+        m2 = uniform ? make_uint2(~0u, ~0u) : mask_region<1>(w, nx, r);
+        if (MODE == kModeSmall) {
+          uint32_t hm = 0;
+          if (lane < 4u) hm = mask_chunk<1>(*reinterpret_cast<const uint4*>(tb + kRegion + 16u * lane), 0u, r);
+          const uint32_t h0 = __shfl_sync(0xffffffffu, hm, 0) | (__shfl_sync(0xffffffffu, hm, 1) << 16);
+          const uint32_t h1 = __shfl_sync(0xffffffffu, hm, 2) | (__shfl_sync(0xffffffffu, hm, 3) << 16);
+          after = ((uint64_t)h1 << 32) | h0;
+        }
+      } else {
+        uint32_t nx[4];
+        next_words(w, *reinterpret_cast<const uint32_t*>(tb + kRegion), nx);
+        if (L == 2u) {
+          if (hot || detect_region<2>(w, nx, r)) m2 = mask_region<2>(w, nx, r);
+        } else if (L == 3u) {
+          if (hot || detect_region<3>(w, nx, r)) m2 = mask_region<3>(w, nx, r);
+        } else {
+          if (hot || detect_region<3>(w, nx, r)) m2 = mask_region<4>(w, nx, r);
+        }
+      }
+      found = __any_sync(0xffffffffu, (m2.x | m2.y) != 0u);
+      hot = found;
+      if (found) {
+        // the lane's 64-byte segment of the mask, from the chunks' masks
+        uint64_t mask = ~0ull;
+        if (!uniform) {
+          uint16_t* const h = reinterpret_cast<uint16_t*>(row) + lane;
+          h[0] = (uint16_t)m2.x;
+          h[32] = (uint16_t)(m2.x >> 16);
+          h[64] = (uint16_t)m2.y;
+          h[96] = (uint16_t)(m2.y >> 16);
+          __syncwarp();
+          mask = row[lane];
+          __syncwarp();
+        }
+        if (MODE == kModeSmall && same) {
+          uint64_t hi = (uint64_t)__shfl_down_sync(0xffffffffu, (unsigned long long)mask, 1);
+          if (lane == 31u) hi = after;
+          mask = runs_of(mask, hi, L);
+        }
+        if (rstart < p.block_before || rstart + kRegion > lim) {
+          const unsigned long long gseg = rstart + lane * 64u;
+          uint32_t lo = 0, hi = 0;
+          if (p.block_before > gseg) {
+            const unsigned long long d = p.block_before - gseg;
+            lo = d < 64ull ? (uint32_t)d : 64u;
+          }
+          if (lim > gseg) {
+            const unsigned long long d = lim - gseg;
+            hi = d < 64ull ? (uint32_t)d : 64u;
+          }
+          mask &= low_bits(hi) & ~low_bits(lo);
+        }
+        if (!same && L > 4u)  // the rest of the pattern (a long one may run past what the slot holds)
+          mask = verify_tail(mask, L <= kHaloMax ? tb + 64u * lane : p.in + rstart + 64u * lane, ps, L);
+        row[lane] = mask;
+        if (MODE == kModeFree) {
+          cnt = __reduce_add_sync(0xffffffffu, (uint32_t)__popcll(mask));
+          end = __reduce_max_sync(0xffffffffu, mask ? lane * 64u + (63u - (uint32_t)__clzll((long long)mask)) + L : 0u);
+          if (end) end += qs;
+        } else {
+          __syncwarp();
+          const uint32_t some = __ballot_sync(0xffffffffu, mask != 0ull);
+          kind = some == 0u ? 0u : (__all_sync(0xffffffffu, mask == ~0ull) ? 2u : 1u);
+          if (kind == 1u) {
+            uint8_t* const wt = smem + lay.wtab + slot * lay.wtab_set;
+            if (L <= 4u) {
+              uint8_t* const sr = smem + lay.srec + slot * lay.srec_set + (warp * 32u + lane) * L;
+              uint32_t* const wt4 = reinterpret_cast<uint32_t*>(wt) + warp * L;
+              if (L == 2u)
+                ks_warp_tables<2>(mask, p.inv_l, p.stride_mask, sr, wt4);
+              else if (L == 3u)
+                ks_warp_tables<3>(mask, p.inv_l, p.stride_mask, sr, wt4);
+              else
+                ks_warp_tables<4>(mask, p.inv_l, p.stride_mask, sr, wt4);
+            } else {
+              // a lane per carry walks the segments that hold candidates
+              for (uint32_t c = lane; c < L; c += 32u) {
+                uint32_t x = c, kc = 0;
+                for (uint32_t sm = some; sm; sm &= sm - 1u) {
+                  const uint32_t s = (uint32_t)__ffs(sm) - 1u;
+                  x = walk_segment(x, s, row[s], L, &kc);
+                }
+                reinterpret_cast<uint16_t*>(wt)[warp * L + c] = (uint16_t)((kc << 6) | (x > kRegion ? x - kRegion : 0u));
+              }
+            }
+          }
+        }
+      }
+    }
+    if (lane == 0) {
+      if (MODE == kModeFree) {
+        s_wcnt[slot][warp] = cnt;
+        s_wend[slot][warp] = end;
+      } else {
+        s_kind[slot][warp] = (uint8_t)kind;
+      }
+    }
+  };
+
+  // A region as pieces: literal runs between replacements, one after the other by the whole warp.
+  // tb: the super-tile; x0, end: the region's literal range (relative to it); out[g0, g0 + total).
+  auto emit_pieces = [&](const uint8_t* tb, uint64_t kept, uint32_t x0, uint32_t end, unsigned long long g0, uint32_t total) {
+    uint32_t pos = x0, o = 0;
+#pragma unroll 1
+    for (uint32_t sm = __ballot_sync(0xffffffffu, kept != 0ull); sm; sm &= sm - 1u) {
+      const uint32_t s = (uint32_t)__ffs(sm) - 1u;
+#pragma unroll 1
+      for (uint64_t m = (uint64_t)__shfl_sync(0xffffffffu, (unsigned long long)kept, s); m; m &= m - 1ull) {
+        const uint32_t at = qs + 64u * s + (uint32_t)__ffsll((long long)m) - 1u;
+        const uint32_t l = at > pos ? at - pos : 0u;
+        if (o + l + R > total) {  // (ruled out by the arithmetic; nothing is written past the slot)
+          if (lane == 0) set_error(p);
+          return;
+        }
+        if (l) warp_emit_literal(p.out, tb, g0 + o, l, pos);
+        o += l;
+        for (uint32_t q = lane; q < R; q += 32u) p.out[g0 + o + q] = rs[q];
+        o += R;
+        pos = at + L;
+      }
+    }
+    const uint32_t l = end > pos ? end - pos : 0u;
+    if (o + l != total) {
+      if (lane == 0) set_error(p);
+    } else if (l) {
+      warp_emit_literal(p.out, tb, g0 + o, l, pos);
+    }
+  };
+
+  // A region that mixes literal bytes and replacements, scattered into the warp's staging area and
+  // copied out in rounds: kept starts `kept` of the lane's segment, x_in bytes of it covered by an
+  // earlier match, V valid bytes. With exact the output must be `total` bytes; otherwise its length
+  // goes to s_cutlen and is checked against the room here.
+  auto emit_scatter = [&](const uint8_t* src, uint64_t kept, uint32_t x_in, uint32_t V, unsigned long long g0, uint32_t total,
+                          bool exact, bool write, uint32_t slot) {
+    // literal bytes: valid, not covered by the carry-in or by a match of this segment
+    uint64_t C = kept;
+    {
+      const uint32_t Lc = L < 64u ? L : 64u;
+      uint32_t w = 1;
+      for (; 2u * w <= Lc; w *= 2u) C |= C << w;
+      if (w < Lc) C |= C << (Lc - w);
+      C = ~C & ~low_bits(x_in) & low_bits(V);
+    }
+    const uint32_t low = (uint32_t)__popc((uint32_t)C) + (uint32_t)__popc((uint32_t)kept) * R;
+    const uint32_t olen = low + (uint32_t)__popc((uint32_t)(C >> 32)) + (uint32_t)__popc((uint32_t)(kept >> 32)) * R;
+    const uint32_t end = warp_incl_scan(olen, OpSum()), start = end - olen;
+    const uint32_t len = __shfl_sync(0xffffffffu, end, 31);
+    if (exact) {
+      if (len != total) {  // (the arithmetic rules it out)
+        if (lane == 0) set_error(p);
+        return;
+      }
+    } else {
+      if (lane == 0) s_cutlen[slot] = len;
+      const bool room = g0 <= p.out_cap && len <= p.out_cap - g0;
+      if (!room && lane == 0) atomicExch(&p.res->overflow_epoch, p.epoch);
+      if (!room || !write) return;
+    }
+    gm[lane] = make_uint4((uint32_t)C, (uint32_t)kept, (uint32_t)(C >> 32), (uint32_t)(kept >> 32));
+    const bool one = __all_sync(0xffffffffu, L == 1u && V == 64u && x_in == 0u);
+#pragma unroll 1
+    for (uint32_t s0 = 0; s0 < 32u;) {  // rounds of as many segments as fit the staging area
+      const uint32_t from = __shfl_sync(0xffffffffu, start, s0);
+      const uint32_t over = __ballot_sync(0xffffffffu, lane >= s0 && end - from + 15u > lay.stage);
+      uint32_t s1 = over ? (uint32_t)__ffs(over) - 1u : 32u;
+      const bool direct = s1 == s0;  // one segment alone outgrows it: straight to global memory
+      if (direct) ++s1;
+      const uint32_t to = __shfl_sync(0xffffffffu, end, s1 - 1u);
+      const unsigned long long gr = g0 + from;
+      const uint32_t pk = ((uint32_t)(gr & 15ull) + start - from) | (low << 16);
+      __syncwarp();  // the masks are written, the last round's bytes read
+      scatter_any(direct ? p.out + (gr & ~15ull) : stg, src, gm, pk, s0, s1, R, rs, one);
+      __syncwarp();
+      if (to > from && !direct) warp_copy_staged(p.out, stg, gr, to - from);
+      s0 = s1;
+    }
+    __syncwarp();
+  };
+
+  // ---- pass B: the output of the warp's region of super-tile t
+  auto pass_b = [&](const uint32_t t, const uint32_t slot) {
+    const unsigned long long tstart = (unsigned long long)t * S;
+    uint8_t* const tb = smem + lay.slots + slot * kSlot;
+    const uint32_t flags = s_flags[slot];
+    const uint4 e = s_reg[slot][warp];  // output offset, length, first uncovered byte, kept count
+    const unsigned long long O = s_O[slot], g0 = O + e.x;
+    const bool write = (flags & kWrite) != 0u;
+    const uint4* const t16 = reinterpret_cast<const uint4*>(smem + lay.tab16);
+    uint32_t last1 = 0;  // kModeSmall: this region's last kept start + 1
+    const uint32_t tvalid = n - tstart < S ? (uint32_t)(n - tstart) : (uint32_t)S;
+    const uint32_t vb = tvalid > qs ? min(tvalid - qs, kRegion) : 0u;
+    const bool cut = MODE == kModeSmall && (flags & kCut) && vb != 0u && vb < kRegion;
+    if (flags & kRuns) {
+      // the whole super-tile is the replacement repeated (or nothing): slices cut at 16-byte boundaries
+      const uint32_t total = s_total[slot];
+      if (write && total) {
+        const unsigned long long end = O + total;
+        const unsigned long long s0 = warp == 0 ? O : (O + (unsigned long long)total * warp / kWorkers) & ~15ull;
+        const unsigned long long s1 = warp == kWorkers - 1u ? end : (O + (unsigned long long)total * (warp + 1u) / kWorkers) & ~15ull;
+        const unsigned long long a = s0 > O ? s0 : O, b = s1 < end ? s1 : end;
+        if (b > a) warp_emit_replace(p.out, t16, rs, R, step512, rmag, a, (uint32_t)(b - a), mod_small((uint32_t)(a - O), R, rmag));
+      }
+      if (MODE == kModeSmall && e.w) last1 = e.z + (e.w - 1u) * L + 1u;
+    } else if (e.w == 0u) {
+      if (write && e.y) warp_emit_literal(p.out, tb, g0, e.y, e.z);
+    } else if (!cut && R <= 64u && e.y == e.w * R) {  // nothing literal
+      if (write && e.y) warp_emit_replace(p.out, t16, rs, R, step512, rmag, g0, e.y);
+      if (MODE == kModeSmall) last1 = e.z + (e.w - 1u) * L + 1u;
+    } else {
+      const uint64_t* const row = reinterpret_cast<const uint64_t*>(smem + lay.masks) + (slot * kWorkers + warp) * 32u;
+      uint64_t kept = row[lane];
+      const uint32_t c0 = e.z - qs;  // bytes of the region covered by an earlier match
+      if (MODE == kModeSmall) {
+        // the greedy from the exact carry into the region
+        uint32_t xs = 0;  // carry into the lane's segment
+        if (s_kind[slot][warp] == 2u) {
+          xs = dense_seg_carry(c0, lane * 64u, L);
+        } else if (L <= 4u) {
+          xs = (smem + lay.srec + slot * lay.srec_set)[(warp * 32u + lane) * L + c0];
+        } else {
+          uint32_t x = c0, kc = 0;
+          for (uint32_t sm = __ballot_sync(0xffffffffu, kept != 0ull); sm; sm &= sm - 1u) {
+            const uint32_t s = (uint32_t)__ffs(sm) - 1u;
+            if (s == lane) xs = x > 64u * s ? x - 64u * s : 0u;
+            x = walk_segment(x, s, row[s], L, &kc);
+          }
+        }
+        kept = L <= 4u ? (xs < 64u ? seg_walk(kept, xs, L, p.inv_l, p.stride_mask).kept : 0ull) : walk_kept(xs, kept, L);
+        last1 = __reduce_max_sync(0xffffffffu, kept ? qs + lane * 64u + 64u - (uint32_t)__clzll((long long)kept) : 0u);
+      }
+      if (write || cut) {
+        // bytes of the lane's segment covered by an earlier match
+        uint32_t x_in;
+        if (L <= 64u) {  // only the previous segment's last match reaches here
+          const uint32_t ee = kept ? 63u - (uint32_t)__clzll((long long)kept) + L : 0u;
+          const uint32_t pe = __shfl_up_sync(0xffffffffu, ee, 1);
+          x_in = lane == 0 ? c0 : (pe > 64u ? pe - 64u : 0u);
+        } else {
+          uint32_t ee = kept ? lane * 64u + 63u - (uint32_t)__clzll((long long)kept) + L : 0u;
+#pragma unroll
+          for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, ee, d);
+            if (lane >= (uint32_t)d) ee = o > ee ? o : ee;
+          }
+          ee = __shfl_up_sync(0xffffffffu, ee, 1);
+          if (lane == 0) ee = 0;
+          ee = ee > c0 ? ee : c0;
+          x_in = ee > lane * 64u ? ee - lane * 64u : 0u;
+        }
+        const uint32_t V = vb > lane * 64u ? min(vb - lane * 64u, 64u) : 0u;
+        if (!cut && R == L && L <= kHaloMax) {
+          // equal lengths: written over the matches in shared memory, then copied (a match may run
+          // past the region: those bytes are its own)
+          uint8_t* const w = tb + qs + 64u * lane;
+          for (uint64_t km = kept; km; km &= km - 1ull) {
+            const uint32_t b = (uint32_t)(__ffsll((long long)km) - 1);
+            for (uint32_t q = 0; q < R; ++q) w[b + q] = rs[q];
+          }
+          fence_proxy_async_smem();  // the slot is loaded again by the async proxy
+          __syncwarp();
+          warp_emit_literal(p.out, tb, g0, e.y, e.z);
+        } else if (!cut && (R > 64u || e.w <= kRegionPieces)) {
+          emit_pieces(tb, kept, e.z, qs + vb, g0, e.y);
+        } else {
+          emit_scatter(tb + qs, kept, x_in, V, g0, e.y, !cut, write, slot);
+        }
+      }
+    }
+    if (MODE == kModeSmall && lane == 0 && last1) atomicMax(&s_last1[slot], last1);
+  };
+
+  // Pass A of the next super-tile as soon as it is loaded, else pass B of the oldest one placed: while
+  // slots are left, a look-back that waits elsewhere delays no function of this CTA.
+  uint32_t ia = 0, ib = 0;  // next super-tile to search, next to write
+  bool more = true;
+#pragma unroll 1
+  while (more || ib < ia) {
+    uint64_t* const full = &s_full[ia % kSlots];
+    uint64_t* const ready = &s_ready[ib % kSlots];
+    const uint32_t pa = (ia / kSlots) & 1u, pb = (ib / kSlots) & 1u;
+    uint32_t what = 0;  // 1: pass A, 2: pass B
+    unsigned long long t0 = 0;
+    for (;;) {
+      if (lane == 0) what = more && mbar_test(full, pa) ? 1u : (ib < ia && mbar_test(ready, pb) ? 2u : 0u);
+      what = __shfl_sync(0xffffffffu, what, 0);
+      if (what) break;
+      const unsigned long long now = global_ns();
+      if (t0 == 0)
+        t0 = now;
+      else if (now - t0 > kPipeLimitNs)
+        break;
+      __nanosleep(32);
+    }
+    if (!what) {
+      set_error(p);
+      break;
+    }
+    // (every lane observes the phase itself: the slot was written by the async proxy)
+    if (!pipe_wait(p, what == 1u ? full : ready, what == 1u ? pa : pb)) break;
+    const uint32_t slot = (what == 1u ? ia : ib) % kSlots;
+    const uint32_t t = s_tile[slot];
+    if (what == 1u) {
+      if (t == kNone) {
+        more = false;
+        continue;
+      }
+      pass_a(t, slot);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_adone[slot]);
+      ++ia;
+    } else {
+      pass_b(t, slot);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_bdone[slot]);
+      ++ib;
+    }
+  }
+}
+
 // One CTA answers query_prefix for a super-tile layout: kept starts before limit and the
 // last one, re-deriving the kept starts of the super-tile that holds limit from its exact
 // carry-in (the predecessor's inclusive prefix) and searching earlier super-tiles' records.
@@ -3685,51 +4826,79 @@ void prepare_pattern_fields(ReplaceParams& p, const uint8_t* pat, uint32_t L) {
   }
   p.stride_mask = stride;
   p.agg_entries = p.mode == kModeFree ? 1u : (L < (uint32_t)kTile ? L : (uint32_t)kTile);
+  p.same = 1;
+  for (uint32_t i = 1; i < L; ++i)
+    if (pat[i] != pat[0]) {
+      p.same = 0;
+      break;
+    }
 }
 
 uint32_t tile_kernel_smem_bytes(uint32_t mode, uint32_t L, uint32_t R) { return make_layout(mode, L, R).total; }
-// A single apply holds two super-tiles' tables at once (pass A of one overlaps the previous
-// one's look-back), so its super-tiles are 4 sub-tiles (64 KiB): three CTAs still fit an SM.
+// The super-tile kernel's super-tiles in a single apply and in a multi-pattern stage: 64 KiB.
 constexpr uint32_t kApplySub = 4;
+static_assert(kApplySub != kRegionSub, "nsub tells the kernel");
 
-uint32_t super_nsub(uint32_t mode, uint32_t L) {
-  if (mode == kModeFree) return kApplySub;
-  if (mode == kModeSmall && L >= 2 && L <= 32) {
-    const uint32_t by_rec = 128u / L;  // keep the per-segment carry records within 32 KiB
-    return by_rec < kApplySub ? (by_rec ? by_rec : 1u) : kApplySub;
-  }
+// Which kernel takes an input. The region kernel has the shorter path for one super-tile and more of
+// the chip at work on small inputs; its three slots hold a super-tile for its load, its
+// look-back and its output, so on large inputs the look-back bounds it, where the super-tile kernel
+// reads the input a second time from L2. Microseconds, super-tile kernel / region kernel:
+//                      1 MiB      16 MiB     32 MiB     64 MiB     128 MiB
+//   entity in text   21.4/14.2  26.2/21.6  36.8/32.2  56.9/52.9  89.4/94.5
+//   binary deletion  16.0/13.6  26.3/21.3  30.2/29.2  45.3/47.1  74.1/83.2
+//   blanks to %20    36.3/21.3  44.3/42.9  71.8/65.2   121/119    205/216
+//   a run, L = 1     15.6/13.2  21.9/24.0  35.0/37.4  57.8/61.9  96.1/112
+//   a run, L = 2     15.8/14.8  18.4/21.6  22.4/30.9  32.1/47.8  55.5/84.9
+// Bordered patterns of 5 to 64 bytes are always the region kernel's (64 MiB run of 6: 397 -> 122 us;
+// 32 MiB of rule lines, L = 40, which the tile kernel took before: 1020 -> 108 us).
+uint32_t super_nsub(uint32_t mode, uint32_t L, unsigned long long n) {
+  if (mode == kModeMulti) return kApplySub;
+  if (mode == kModeSmall && L > 4u) return kRegionSub;
+  const unsigned long long most = mode == kModeFree ? (L >= 2u ? 64ull << 20 : 32ull << 20) : 8ull << 20;
+  if (mode == kModeFree || (mode == kModeSmall && L >= 2u)) return n <= most ? kRegionSub : kApplySub;
   return 0;
 }
 
 namespace {
+// Shared-memory limits of the kernels of one apply, once per device.
 template <int MODE>
-cudaError_t launch_super_mode(const ReplaceParams& p, cudaStream_t st, int* grid_out) {
+cudaError_t super_attributes() {
   static std::mutex mu;
   static unsigned long long attr_dev_mask = 0;
-  const uint32_t smem = make_layout_s(MODE, p.L, p.R, p.nsub, 1u, 2u).total;  // two sets of tables
   int dev = 0;
   cudaGetDevice(&dev);
-  {
-    std::lock_guard<std::mutex> g(mu);
-    if (!(attr_dev_mask & (1ull << (dev & 63)))) {
-      cudaError_t e = cudaFuncSetAttribute(replace_super_kernel<MODE, false>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-      if (e != cudaSuccess) return e;
-      e = cudaFuncSetAttribute(query_super_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               200 * 1024);
-      if (e != cudaSuccess) return e;
-      attr_dev_mask |= 1ull << (dev & 63);
-    }
-  }
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, replace_super_kernel<MODE, false>,
-                                                                kThreads, smem);
+  std::lock_guard<std::mutex> g(mu);
+  if (attr_dev_mask & (1ull << (dev & 63))) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(replace_super_kernel<MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       220 * 1024);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(replace_region_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(query_super_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  if (e == cudaSuccess) attr_dev_mask |= 1ull << (dev & 63);
+  return e;
+}
+
+template <int MODE>
+cudaError_t launch_super_mode(const ReplaceParams& p, cudaStream_t st, int* grid_out) {
+  cudaError_t e = super_attributes<MODE>();
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
+  const bool region = p.nsub == kRegionSub;
+  const uint32_t smem = region ? make_layout_w(MODE, p.L, p.R).total
+                               : make_layout_s(MODE, p.L, p.R, p.nsub, 1u, 2u).total;  // two sets of tables
+  int per_sm = 1;  // (the region kernel: one persistent CTA per SM)
+  if (!region) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, replace_super_kernel<MODE, false>, kThreads, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) per_sm = 1;
+  }
   long long grid = (long long)per_sm * device_sm_count();
   if (grid > (long long)p.num_tiles) grid = p.num_tiles;
   if (grid < 1) grid = 1;
-  replace_super_kernel<MODE, false><<<(unsigned)grid, kThreads, smem, st>>>(p, SegLaunch{});
+  if (region)
+    replace_region_kernel<MODE><<<(unsigned)grid, kRegionThreads, smem, st>>>(p);
+  else
+    replace_super_kernel<MODE, false><<<(unsigned)grid, kThreads, smem, st>>>(p, SegLaunch{});
   if (grid_out) *grid_out = (int)grid;
   return cudaGetLastError();
 }
@@ -3834,7 +5003,7 @@ bool make_seg_pair(SegPair& q, const uint8_t* pat, uint32_t L, const uint8_t* re
   memset(&p, 0, sizeof(p));
   prepare_pattern_fields(p, pat, L);
   if (p.mode != kModeFree && p.mode != kModeSmall) return false;
-  if (p.mode == kModeSmall && super_nsub(p.mode, L) == 0) return false;
+  if (p.mode == kModeSmall && super_nsub(p.mode, L, 0) == 0) return false;
   memset(&q, 0, sizeof(q));
   q.stride_mask = p.stride_mask;
   q.L = L;

@@ -141,7 +141,7 @@ struct ReplaceParams {
   // pattern's first byte has no candidate and skips the search. nullptr: no index.
   const uint32_t* presence;
   unsigned int presence_shift;
-  unsigned int pad2;
+  unsigned int same;              // every pattern byte is the same
   uint8_t pat[kInlineMax];
   uint8_t rep[kInlineMax];
 };
@@ -203,8 +203,9 @@ void prepare_pattern_fields(ReplaceParams& p, const uint8_t* pat, uint32_t L);
 uint32_t tile_kernel_smem_bytes(uint32_t mode, uint32_t L, uint32_t R);
 // Launch one apply. grid_ctas_out receives the number of CTAs launched.
 cudaError_t launch_replace(const ReplaceParams& p, cudaStream_t st, int* grid_ctas_out);
-// Sub-tiles per super-tile for the super-tile kernel, or 0 when (mode, L) needs the tile kernel.
-uint32_t super_nsub(uint32_t mode, uint32_t L);
+// Sub-tiles per super-tile for an input of n bytes (3: the region kernel, else the super-tile kernel),
+// or 0 when (mode, L) needs the tile kernel.
+uint32_t super_nsub(uint32_t mode, uint32_t L, unsigned long long n);
 // Launch one apply with the super-tile kernel (p.nsub > 0, p.tile_last set).
 cudaError_t launch_replace_super(const ReplaceParams& p, cudaStream_t st, int* grid_ctas_out);
 // Query for an apply made by the super-tile kernel: p.query_limit64 = limit (< p.n).

@@ -303,8 +303,8 @@ int stream_setup(Stream& S, const uint8_t** pats, const int* pat_lens, const uin
     memset(&p, 0, sizeof(p));
     crb::prepare_pattern_fields(p, pats[k], (uint32_t)pl);
     p.R = (uint32_t)rl;
-    p.nsub = crb::super_nsub(p.mode, p.L);
-    if (!p.nsub) return kUnsupported;  // bordered pattern longer than the super-tile kernel takes
+    p.nsub = crb::super_nsub(p.mode, p.L, chunk);
+    if (!p.nsub || (p.mode == crb::kModeSmall && p.L > 32u)) return kUnsupported;  // long bordered pattern
     memcpy(p.pat, pats[k], (size_t)pl);
     if (rl) memcpy(p.rep, reps[k], (size_t)rl);
     S.st[(size_t)k].P = (uint32_t)pl - 1;
@@ -397,7 +397,7 @@ int stream_replace(const uint8_t* src, size_t n, const uint8_t** pats, const int
       ReplaceParams q;
       memset(&q, 0, sizeof(q));
       crb::prepare_pattern_fields(q, pats[k], (uint32_t)pat_lens[k]);
-      if (!crb::super_nsub(q.mode, q.L)) return kUnsupported;
+      if (!crb::super_nsub(q.mode, q.L, 0) || (q.mode == crb::kModeSmall && q.L > 32u)) return kUnsupported;
     }
     return 0;
   }
