@@ -2139,6 +2139,25 @@ __device__ __forceinline__ void warp_emit_replace(uint8_t* out, const uint4* t16
   if (ok) out[b] = rs[mod_small((uint32_t)(b - g0) + ph0, R, rmag)];
 }
 
+// Shared-memory reads of scatter_any only: its sources do not change while it runs, so the compiler may
+// move them across its stores.
+__device__ __forceinline__ uint32_t lds8(uint32_t a) {
+  uint32_t v;
+  asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts8(uint32_t a, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+
 // Staging bytes of segments [s0, s1) of a warp's region. gm[s]: segment s's literal bytes (x: low 32,
 // z: high 32) and kept starts (y, w); pk (lane s): staging position of its first byte in bits 0-15 and
 // the output length of its first 32 bytes in bits 16-31. A lane takes one byte of each 32: a
@@ -2149,51 +2168,87 @@ __device__ __forceinline__ void warp_emit_replace(uint8_t* out, const uint4* t16
 // blank replaced by three bytes, 340 -> 115 us; line ends made CRLF, 149 -> 97 us.
 // ONE: L = 1 and every byte valid (literal = not kept). RC: R, or 5 for any R > 4.
 template <bool ONE, int RC>
-__device__ __forceinline__ void scatter_segments(uint8_t* stg, const uint8_t* src, const uint4* gm, uint32_t pk,
-                                                 uint32_t s0, uint32_t s1, uint32_t R, const uint8_t* rs) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t bit = 1u << lane, below = bit - 1u;
-  const uint32_t r4 = *reinterpret_cast<const uint32_t*>(rs);
-#pragma unroll 1
-  for (uint32_t s = s0; s < s1; ++s) {
-    const uint4 q = gm[s];
-    const uint32_t b = __shfl_sync(0xffffffffu, pk, s);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t C = h ? q.z : q.x, K = h ? q.w : q.y;
-      const uint32_t base = h ? (b & 0xFFFFu) + (b >> 16) : (b & 0xFFFFu);
-      const uint32_t kb = (uint32_t)__popc(K & below);
-      uint8_t* d = stg + base + (ONE ? lane - kb : (uint32_t)__popc(C & below)) +
-                   (RC == 5 ? kb * R : kb * (uint32_t)RC);
-      const uint8_t v = src[64u * s + 32u * (uint32_t)h + lane];
-      const bool mat = (K & bit) != 0u, lit = ONE ? !mat : (C & bit) != 0u;
-      if (RC == 0) {
-        if (lit) *d = v;
-      } else {
-        if (lit || mat) *d = mat ? (uint8_t)r4 : v;
-        if (RC >= 2 && mat) {
-          d[1] = (uint8_t)(r4 >> 8);
-          if (RC >= 3) d[2] = (uint8_t)(r4 >> 16);
-          if (RC >= 4) d[3] = (uint8_t)(r4 >> 24);
-          if (RC >= 5)
-            for (uint32_t r = 4; r < R; ++r) d[r] = rs[r];
-        }
-      }
+__device__ __forceinline__ void scatter_half(uint32_t stg, uint32_t base, uint32_t v, uint32_t C, uint32_t K, uint32_t below,
+                                             uint32_t R, uint32_t rep4, uint32_t rs) {
+  const uint32_t bit = below + 1u;
+  // bytes emitted before this lane's
+  uint32_t d = stg + base;
+  if (RC == 1) {
+    d += (uint32_t)__popc((C | K) & below);  // a literal and a match each emit one
+  } else if (RC == 0) {
+    d += ONE ? (uint32_t)__popc(~K & below) : (uint32_t)__popc(C & below);
+  } else {
+    const uint32_t kb = (uint32_t)__popc(K & below);
+    d += (ONE ? (threadIdx.x & 31u) - kb : (uint32_t)__popc(C & below)) + (RC == 5 ? kb * R : kb * (uint32_t)RC);
+  }
+  const bool mat = (K & bit) != 0u, lit = ONE ? !mat : (C & bit) != 0u;
+  if (RC == 0) {
+    if (lit) sts8(d, v);
+  } else {
+    if (lit || mat) sts8(d, mat ? rep4 : v);
+    if (RC >= 2 && mat) {
+      sts8(d + 1u, rep4 >> 8);
+      if (RC >= 3) sts8(d + 2u, rep4 >> 16);
+      if (RC >= 4) sts8(d + 3u, rep4 >> 24);
+      if (RC >= 5)
+        for (uint32_t r = 4; r < R; ++r) sts8(d + r, lds8(rs + r));
     }
   }
 }
-
-template <bool ONE>
-__device__ __forceinline__ void scatter_by_length(uint8_t* stg, const uint8_t* src, const uint4* gm, uint32_t pk,
-                                                  uint32_t s0, uint32_t s1, uint32_t R, const uint8_t* rs) {
-  switch (R) {  // the same in every lane
-    case 0: scatter_segments<ONE, 0>(stg, src, gm, pk, s0, s1, R, rs); break;
-    case 1: scatter_segments<ONE, 1>(stg, src, gm, pk, s0, s1, R, rs); break;
-    case 2: scatter_segments<ONE, 2>(stg, src, gm, pk, s0, s1, R, rs); break;
-    case 3: scatter_segments<ONE, 3>(stg, src, gm, pk, s0, s1, R, rs); break;
-    case 4: scatter_segments<ONE, 4>(stg, src, gm, pk, s0, s1, R, rs); break;
-    default: scatter_segments<ONE, 5>(stg, src, gm, pk, s0, s1, R, rs); break;
+template <bool ONE, int RC>
+__device__ __forceinline__ void scatter_segments(uint32_t stg, uint32_t src, uint32_t gm, uint32_t pk, uint32_t s0,
+                                                 uint32_t s1, uint32_t R, uint32_t rs) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t below = (1u << lane) - 1u;
+  const uint32_t rep4 = lds32(rs);
+  src += 64u * s0 + lane;
+  gm += 16u * s0;
+#pragma unroll 2
+  for (uint32_t s = s0; s < s1; ++s, src += 64u, gm += 16u) {
+    const uint4 q = lds128(gm);
+    const uint32_t b = __shfl_sync(0xffffffffu, pk, s);
+    scatter_half<ONE, RC>(stg, b & 0xFFFFu, lds8(src), q.x, q.y, below, R, rep4, rs);
+    scatter_half<ONE, RC>(stg, (b & 0xFFFFu) + (b >> 16), lds8(src + 32u), q.z, q.w, below, R, rep4, rs);
   }
+}
+
+// One segment straight to global memory (its output alone outgrows the staging area): as
+// scatter_segments, with the staging position 0 at `out`.
+__device__ __noinline__ void scatter_direct(uint8_t* out, const uint8_t* src, const uint4* gm, uint32_t pk, uint32_t s,
+                                            uint32_t R, const uint8_t* rs) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t bit = 1u << lane, below = bit - 1u;
+  const uint4 q = gm[s];
+  const uint32_t b = __shfl_sync(0xffffffffu, pk, s);
+  for (uint32_t h = 0; h < 2u; ++h) {
+    const uint32_t C = h ? q.z : q.x, K = h ? q.w : q.y;
+    uint8_t* d = out + (b & 0xFFFFu) + (h ? b >> 16 : 0u) + __popc(C & below) + (uint32_t)__popc(K & below) * R;
+    if (C & bit) *d = src[64u * s + 32u * h + lane];
+    if (K & bit)
+      for (uint32_t r = 0; r < R; ++r) d[r] = rs[r];
+  }
+}
+
+// scatter_segments by R and shape, kept out of line: its twelve loops would crowd the kernel's instruction
+// cache (inlined, sparse inputs measured 3-4% slower). Shared-memory addresses, 32 bits each.
+__device__ __noinline__ void scatter_any(uint32_t stg, uint32_t src, uint32_t gm, uint32_t pk, uint32_t s0, uint32_t s1,
+                                         uint32_t R, uint32_t rs, bool one) {
+#define CRB_SCATTER(RC)                                                 \
+  case RC:                                                              \
+    if (one)                                                            \
+      scatter_segments<true, RC>(stg, src, gm, pk, s0, s1, R, rs);      \
+    else                                                                \
+      scatter_segments<false, RC>(stg, src, gm, pk, s0, s1, R, rs);     \
+    break;
+  switch (R < 5u ? R : 5u) {  // the same in every lane
+    CRB_SCATTER(0)
+    CRB_SCATTER(1)
+    CRB_SCATTER(2)
+    CRB_SCATTER(3)
+    CRB_SCATTER(4)
+    CRB_SCATTER(5)
+  }
+#undef CRB_SCATTER
 }
 
 // A warp's staged bytes to out[g0, g0 + len): staging byte (g0 & 15) + i holds output byte i. Whole
@@ -2216,6 +2271,79 @@ __device__ __forceinline__ void warp_copy_staged(uint8_t* out, const uint8_t* st
     ok = b < gend;
   }
   if (ok) out[b] = stg[(uint32_t)(b - ga)];
+}
+
+// Output of a warp region with few matches (at most kGatherMax, output at most kGatherBytes; R <= 64):
+// every 16-byte chunk of the output is taken by one lane, which copies it as if it began a literal
+// run (right up to the chunk's first match); the bytes from each match's replacement to the end of its
+// last chunk are then written over it one per lane. A chunk's source follows from the number of matches
+// that end before it: counted per chunk, then a scan. kept: the lane's kept starts in its segment of the
+// region at tb + qs; literal bytes [x0, end) (relative to tb); out[g0, g0 + total). scr: kGatherScratch
+// bytes of the warp's own. Returns false, writing nothing, when the lengths do not add up.
+// Bound by instruction issue: its cost grows with the matches, the scatter's does not. 24 MiB of random
+// bytes with 8 / 16 / 20 / 25 planted matches per region: 33.9 / 38.9 / 39.4 / 42.6 us, scattered 35.9
+// (more than 12 scattered) / 40.3 / 40.3 / 41.4 us; 32 MiB of rule lines 107 -> 83 us (pieces before).
+constexpr uint32_t kGatherMax = 20, kGatherBytes = 4064, kGatherScratch = 1024 + 2 * kGatherMax;
+__device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32_t* scr, uint64_t kept, uint32_t qs,
+                                         uint32_t x0, uint32_t end, unsigned long long g0, uint32_t total, uint32_t L,
+                                         uint32_t R, const uint8_t* rs) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const int grow = (int)R - (int)L;
+  uint16_t* const os = reinterpret_cast<uint16_t*>(scr + 256);  // output offset of every replacement
+  const uint32_t a0 = (uint32_t)g0 & 15u, nch = (total + a0 + 15u) >> 4;  // chunks touched, the first at g0 - a0
+  for (uint32_t c = lane; c < nch; c += 32u) scr[c] = 0;
+  const uint32_t cnt = (uint32_t)__popcll(kept);
+  const uint32_t incl = warp_incl_scan(cnt, OpSum());
+  const uint32_t M = __shfl_sync(0xffffffffu, incl, 31);
+  __syncwarp();
+  uint32_t k = incl - cnt;
+  for (uint64_t km = kept; km; km &= km - 1ull, ++k) {
+    const uint32_t o = (uint32_t)((int)(qs + 64u * lane + (uint32_t)__ffsll((long long)km) - 1u - x0) + (int)k * grow);
+    os[k] = (uint16_t)o;
+    const uint32_t ce = (o + R + a0 + 15u) >> 4;  // the first chunk that starts at or after its end
+    if (ce < nch) atomicAdd(scr + ce, 1u);
+  }
+  __syncwarp();
+  {
+    const uint32_t lo = os[M - 1u], last = (uint32_t)((int)(lo + x0) - (int)(M - 1u) * grow) + L;  // end of the last match
+    if (lo + R + (end > last ? end - last : 0u) != total) return false;
+  }
+  uint8_t* const og = out + g0;
+  uint32_t j = 0, jb = 0;
+#pragma unroll 1
+  for (uint32_t c0 = 0; c0 < nch; c0 += 32u) {
+    const uint32_t c = c0 + lane;
+    j = jb + warp_incl_scan(c < nch ? scr[c] : 0u, OpSum());
+    jb = __shfl_sync(0xffffffffu, j, 31);
+    if (16u * c >= a0 && 16u * c + 16u <= total + a0) {
+      const uint32_t src = (uint32_t)((int)(x0 + 16u * c - a0) - (int)j * grow);
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(tb + (src & ~3u));
+      const uint32_t sh = (src & 3u) * 8u;
+      const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
+      st_out16(og + (16u * c - a0), make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh),
+                                               __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh)));
+    }
+  }
+  {
+    // the partial chunks at both ends, one byte per lane: before the first whole chunk on lanes 0-15
+    // (no match ends before it), the last chunk's on lanes 16-31
+    const uint32_t jt = __shfl_sync(0xffffffffu, j, (nch - 1u) & 31u);
+    const uint32_t head = (16u - a0) & 15u, tail0 = 16u * (nch - 1u) - a0;  // (tail0 wraps for a lone first chunk)
+    const bool tail = (nch > 1u || a0 == 0u) && tail0 + 16u > total;
+    const uint32_t b = lane < 16u ? lane : tail0 + (lane - 16u);
+    const bool ok = lane < 16u ? (lane < head && lane < total) : (tail && b < total);
+    if (ok) og[b] = tb[(uint32_t)((int)(x0 + b) - (lane < 16u ? 0 : (int)jt * grow))];
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (uint32_t i = 0; i < M; ++i) {
+    const uint32_t o = os[i], nx = i + 1u < M ? os[i + 1u] : total;
+    const uint32_t fe = ((o + R + a0 + 15u) & ~15u) - a0, to = fe < nx ? fe : nx;
+    for (uint32_t b = o + lane; b < to; b += 32u)
+      og[b] = b < o + R ? rs[b - o] : tb[(uint32_t)((int)(x0 + b) - (int)(i + 1u) * grow)];
+  }
+  __syncwarp();
+  return true;
 }
 
 // Input length, output range and super-tile count of the job described by p.
@@ -2757,7 +2885,16 @@ __global__ void __launch_bounds__(kThreads, 3)
       warp_emit_literal(p.out, tb, g0, wtot, warp * 2048u + x0r);
       return;
     }
-    if (emit_pieces(tb, kept, gseg, x0r, __reduce_add_sync(0xffffffffu, V), g0, wtot)) return;
+    const uint32_t vend = __reduce_add_sync(0xffffffffu, V);
+    if (emit_pieces(tb, kept, gseg, x0r, vend, g0, wtot)) return;
+    if (R <= 64u && wtot <= kGatherBytes && __reduce_add_sync(0xffffffffu, (uint32_t)__popcll(kept)) <= kGatherMax) {
+      const uint32_t q0 = warp * 2048u;
+      if (!emit_gather(p.out, tb, reinterpret_cast<uint32_t*>(ob) + (size_t)warp * lay.wstage_words, kept, q0, q0 + x0r,
+                       q0 + vend, g0, wtot, L, R, rs) &&
+          lane == 0)
+        set_error(p);  // (the arithmetic rules it out)
+      return;
+    }
     // literal bytes: valid, not covered by the carry-in or by a match of this segment
     uint64_t C = kept;
     {
@@ -2791,11 +2928,9 @@ __global__ void __launch_bounds__(kThreads, 3)
       const uint32_t pk = ((uint32_t)(gr & 15ull) + start - from) | (low << 16);
       __syncwarp();  // the masks (and the last round's copies) are done
       if (direct)
-        scatter_segments<false, 5>(p.out + (gr & ~15ull), src, gm, pk, s0, s1, R, rs);
-      else if (one)
-        scatter_by_length<true>(stg, src, gm, pk, s0, s1, R, rs);
+        scatter_direct(p.out + (gr & ~15ull), src, gm, pk, s0, R, rs);
       else
-        scatter_by_length<false>(stg, src, gm, pk, s0, s1, R, rs);
+        scatter_any(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs), one);
       __syncwarp();
       if (to > from && !direct) warp_copy_staged(p.out, stg, gr, to - from);
       s0 = s1;
@@ -3506,9 +3641,10 @@ constexpr uint32_t kRegionSub = kWorkers * kRegion / kTile;  // nsub of the regi
 constexpr uint32_t kHaloMax = 272;                       // bytes after a super-tile held with it
 constexpr uint32_t kSlot = kWorkers * kRegion + kHaloMax + 48;
 constexpr uint32_t kSlots = 3;
-constexpr uint32_t kRegionPieces = 4;                    // regions with up to this many matches: pieces
+constexpr uint32_t kRegionPieces = 1;                    // regions with up to this many matches: pieces
 constexpr unsigned long long kPipeLimitNs = 6000000000ull;  // bounded wait inside a CTA (a look-back may take 2 s)
 static_assert(kRegionSub * kTile == kWorkers * kRegion, "super-tiles are whole sub-tiles (query kernel)");
+static_assert(kGatherScratch <= 1040u + 512u, "emit_gather works in the staging area and the masks behind it");
 
 struct LayoutW {
   uint32_t slots, masks, scratch, pat, rep, tab16, srec, wtab, wrec, total;
@@ -3905,16 +4041,6 @@ __device__ __forceinline__ void fold_regions(const uint32_t* wt, const uint8_t* 
       *sup_carry = e >> 24;
     }
   }
-}
-
-// The scatter of scatter_segments by R and shape; kept out of line: its twelve loops would crowd the
-// kernel's instruction cache (inlined, sparse inputs measured 3-4% slower).
-__device__ __noinline__ void scatter_any(uint8_t* stg, const uint8_t* src, const uint4* gm, uint32_t pk, uint32_t s0,
-                                         uint32_t s1, uint32_t R, const uint8_t* rs, bool one) {
-  if (one)
-    scatter_by_length<true>(stg, src, gm, pk, s0, s1, R, rs);
-  else
-    scatter_by_length<false>(stg, src, gm, pk, s0, s1, R, rs);
 }
 
 }  // namespace
@@ -4468,7 +4594,10 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       const unsigned long long gr = g0 + from;
       const uint32_t pk = ((uint32_t)(gr & 15ull) + start - from) | (low << 16);
       __syncwarp();  // the masks are written, the last round's bytes read
-      scatter_any(direct ? p.out + (gr & ~15ull) : stg, src, gm, pk, s0, s1, R, rs, one);
+      if (direct)
+        scatter_direct(p.out + (gr & ~15ull), src, gm, pk, s0, R, rs);
+      else
+        scatter_any(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs), one);
       __syncwarp();
       if (to > from && !direct) warp_copy_staged(p.out, stg, gr, to - from);
       s0 = s1;
@@ -4560,6 +4689,10 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
           warp_emit_literal(p.out, tb, g0, e.y, e.z);
         } else if (!cut && (R > 64u || e.w <= kRegionPieces)) {
           emit_pieces(tb, kept, e.z, qs + vb, g0, e.y);
+        } else if (!cut && e.w <= kGatherMax && e.y <= kGatherBytes) {
+          if (!emit_gather(p.out, tb, reinterpret_cast<uint32_t*>(stg), kept, qs, e.z, qs + vb, g0, e.y, L, R, rs) &&
+              lane == 0)
+            set_error(p);  // (the arithmetic rules it out)
         } else {
           emit_scatter(tb + qs, kept, x_in, V, g0, e.y, !cut, write, slot);
         }
