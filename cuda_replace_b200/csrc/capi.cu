@@ -489,7 +489,7 @@ int apply_one(Session* s, const uint8_t* pat, int pat_len, const uint8_t* rep, i
   crb::prepare_pattern_fields(p, pat, L);
   p.R = R;
   p.nsub = crb::super_nsub(p.mode, L, n);
-  const size_t tile_bytes = (size_t)crb::kTile * (p.nsub ? p.nsub : 1u);
+  const size_t tile_bytes = p.nsub ? crb::super_tile(p) : (size_t)crb::kTile;
   const size_t tiles = (n + tile_bytes - 1) / tile_bytes;
   if (tiles > 0xFFFFFFF0ull) return (int)cudaErrorInvalidValue;
   p.num_tiles = (uint32_t)tiles;
@@ -613,7 +613,7 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
       if (rl) memcpy(p.rep, reps[k], (size_t)rl);
       bnext = output_bound(b, p.L, p.R);
     }
-    const size_t tb = (size_t)crb::kTile * p.nsub;
+    const size_t tb = crb::super_tile(p);
     const size_t tiles = (b + tb - 1) / tb;
     p.num_tiles = (uint32_t)(tiles ? tiles : 1);
     tiles_max = std::max(tiles_max, (size_t)p.num_tiles);
@@ -1026,7 +1026,7 @@ CR_EXPORT int cuda_replace_apply_device_async(void* h, const uint8_t* d_in, size
   crb::prepare_pattern_fields(p, pat, L);
   p.R = R;
   p.nsub = crb::super_nsub(p.mode, L, n);
-  const size_t tile_bytes = (size_t)crb::kTile * (p.nsub ? p.nsub : 1u);
+  const size_t tile_bytes = p.nsub ? crb::super_tile(p) : (size_t)crb::kTile;
   const size_t tiles = (n + tile_bytes - 1) / tile_bytes;
   if (tiles > 0xFFFFFFF0ull) return (int)cudaErrorInvalidValue;
   p.num_tiles = (uint32_t)tiles;
@@ -1133,7 +1133,7 @@ int unified_chunked(Session* s, const uint8_t* src, size_t n, const uint8_t* pat
   while (nchunks > 1 && (nchunks - 1) * chunk + P >= n) --nchunks;
   if (nchunks > (size_t)kUnifiedChunks) return kFallback;
   auto bnd = [&](size_t k) -> size_t { return k == 0 ? 0 : (k >= nchunks ? n : k * chunk + P); };
-  const size_t tile_bytes = (size_t)crb::kTile * proto.nsub;
+  const size_t tile_bytes = crb::super_tile(proto);
 
   cudaError_t e = cudaSuccess;
   if (!s->up) e = cudaStreamCreateWithFlags(&s->up, cudaStreamNonBlocking);

@@ -3616,14 +3616,14 @@ __global__ void __launch_bounds__(kThreads, 3)
 }
 
 // ============================================================================ region kernel
-// One apply in one launch, warp-specialised: a persistent CTA per SM of 24 worker warps and three
-// control warps. A super-tile is 48 KiB (nsub = 3), a 2 KiB region per worker warp, and stays in shared
-// memory from its single load until its output is written. The loader fills three slots by 1-D TMA bulk
-// copies, a whole super-tile ahead. For super-tile i a worker finds its region's candidates (pass A,
-// chunks in registers); the publisher folds the regions and publishes the super-tile's function; the
-// look-back warp resolves what the super-tiles before leave and places the regions' outputs, while
-// the workers write super-tile i - 1 (pass B, from shared memory) and search i + 1. Nobody but the
-// look-back warp waits for another CTA, and warps meet only at mbarriers, never at a block barrier.
+// One apply in one launch, warp-specialised: a persistent CTA per SM of 24 worker warps and four
+// control warps. A super-tile's regions of 2 KiB, one per worker warp, stay in shared memory from their
+// single load until their output is written. The loader keeps every free slot filling by 1-D TMA bulk
+// copies. For each super-tile a worker finds its region's candidates (pass A, chunks in registers); the
+// publisher folds the regions and publishes the super-tile's function; a look-back warp resolves what
+// the super-tiles before leave and places the regions' outputs; the workers write them (pass B, from
+// shared memory). Nobody but the look-back warps waits for another CTA, and warps meet only at mbarriers,
+// never at a block barrier.
 //
 // Why: with the input read twice (for the search and, after the look-back, for the output) the
 // second read came from L2 only while every CTA's super-tiles in flight fitted it (64 KiB super-tiles
@@ -3632,18 +3632,24 @@ __global__ void __launch_bounds__(kThreads, 3)
 namespace {
 
 constexpr uint32_t kRegion = 2048;
-constexpr uint32_t kWorkers = 24;                        // worker warps = regions of a super-tile
+constexpr uint32_t kWorkers = 24;  // worker warps
 // control warps (the look-backs of successive super-tiles alternate between two warps: one takes
-// 3500 cycles, most of it the round trip to the records, a super-tile at DRAM speed 4400)
+// most of the 4400 cycles that two super-tiles take at DRAM speed, nearly all of it the round trip to the
+// records)
 constexpr uint32_t kLoader = kWorkers, kPublisher = kWorkers + 1, kLookback = kWorkers + 2, kLookbacks = 2;
 constexpr uint32_t kRegionThreads = (kWorkers + 2 + kLookbacks) * 32;
-constexpr uint32_t kRegionSub = kWorkers * kRegion / kTile;  // nsub of the region kernel
-constexpr uint32_t kHaloMax = 272;                       // bytes after a super-tile held with it
-constexpr uint32_t kSlot = kWorkers * kRegion + kHaloMax + 48;
-constexpr uint32_t kSlots = 3;
-constexpr uint32_t kRegionPieces = 1;                    // regions with up to this many matches: pieces
+constexpr uint32_t kRegionSub = 1;   // nsub of an apply that takes the region kernel (its super-tiles: region_tile)
+constexpr uint32_t kHaloMax = 272;   // bytes after a super-tile held with it
+constexpr uint32_t kRegionPieces = 1;  // regions with up to this many matches are written as pieces
 constexpr unsigned long long kPipeLimitNs = 6000000000ull;  // bounded wait inside a CTA (a look-back may take 2 s)
-static_assert(kRegionSub * kTile == kWorkers * kRegion, "super-tiles are whole sub-tiles (query kernel)");
+// Regions of a super-tile (a worker warp each; 24 workers are one or two teams) and slots. A slot is
+// held from its load's start to its output's end, some 10,000 cycles of which the look-back and the load are
+// most, so many small super-tiles in flight keep DRAM busier than few large ones; the functions of
+// bordered patterns cost the control warps more per super-tile, so theirs are the larger ones.
+__host__ __device__ constexpr uint32_t region_count(uint32_t mode) { return mode == kModeFree ? 12u : 24u; }
+__host__ __device__ constexpr uint32_t region_slots(uint32_t mode) { return mode == kModeFree ? 6u : 3u; }
+__host__ __device__ constexpr uint32_t region_tile(uint32_t mode) { return region_count(mode) * kRegion; }
+__host__ __device__ constexpr uint32_t region_slot(uint32_t mode) { return region_tile(mode) + kHaloMax + 48u; }
 static_assert(kGatherScratch <= 1040u + 512u, "emit_gather works in the staging area and the masks behind it");
 
 struct LayoutW {
@@ -3655,10 +3661,11 @@ struct LayoutW {
 __host__ __device__ __forceinline__ LayoutW make_layout_w(uint32_t mode, uint32_t L, uint32_t R) {
   LayoutW s{};
   uint32_t off = 0;
+  const uint32_t NS = region_slots(mode), NR = region_count(mode);
   s.slots = off;
-  off += kSlots * kSlot;
+  off += NS * region_slot(mode);
   s.masks = off;
-  off += kSlots * kWorkers * 256u;
+  off += NS * NR * 256u;
   s.scratch = off;
   s.stage = (mode == kModeFree && L <= 256u && R <= 256u) ? 1552u : 1040u;
   off += kWorkers * (s.stage + 512u);  // and the segments' masks
@@ -3671,15 +3678,15 @@ __host__ __device__ __forceinline__ LayoutW make_layout_w(uint32_t mode, uint32_
   if (mode == kModeSmall) {
     if (L <= 4u) {
       s.srec = off;
-      s.srec_set = kWorkers * 32u * L;
-      off += kSlots * s.srec_set;
+      s.srec_set = NR * 32u * L;
+      off += NS * s.srec_set;
     }
     s.wtab = off;  // per region and carry: kept count (low half), carry-out
-    s.wtab_set = kWorkers * L * (L <= 4u ? 4u : 2u);
-    off += align_up_u32(kSlots * s.wtab_set, 16);
+    s.wtab_set = NR * L * (L <= 4u ? 4u : 2u);
+    off += align_up_u32(NS * s.wtab_set, 16);
     s.wrec = off;
-    s.wrec_set = kWorkers * L;
-    off += align_up_u32(kSlots * s.wrec_set, 16);
+    s.wrec_set = NR * L;
+    off += align_up_u32(NS * s.wrec_set, 16);
   }
   s.total = off;
   return s;
@@ -3820,91 +3827,80 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Look-back of kModeFree in the region kernel. Its carry-in is the reach recorded by the super-tile
-// before (no pattern is as long as a super-tile, so no older carry passes through one); its prefix is the
-// sum of the counts back to the nearest inclusive record. A window is 160 predecessors (with a
-// CTA per SM at most 148 super-tiles are between claim and record), five words per lane in one
-// round trip: windows of 32 took up to five round trips, which bounded the whole pipeline.
-struct SumWindow {
-  static constexpr int kPer = 5;
-  unsigned long long w[kPer];  // first record words of super-tiles base - lane - 32k
-  unsigned long long carry;    // lane 0, first window: the second word of the nearest record
+// Look-back of kModeFree in the region kernel: a running sum. The carry into super-tile t is the reach
+// recorded by t - 1 (no pattern is as long as a super-tile, so no older carry passes through one), and a
+// warp's next super-tile lies only some hundreds of records after its last, so it adds up the counts
+// between the two: nobody publishes inclusive prefixes and nobody waits for another's. A window is
+// 320 records, ten first words per lane in one round trip (1.2 us under load, which windows of 32 back to the
+// nearest inclusive record paid up to five times).
+struct RunningSum {
+  static constexpr int kPer = 10;
+  unsigned long long sum;                // kept in super-tiles [0, pos)
+  unsigned long long w[kPer], n0, n1;    // a window's first words; lane 0: the record of t - 1, both words
+  uint32_t pos;
 
-  __device__ __forceinline__ void load(const ReplaceParams& p, long long base, bool first) {
+  __device__ __forceinline__ void init() {
+    sum = 0;
+    pos = 0;
+  }
+  // Start reading the window at pos on the way to super-tile t.
+  __device__ __forceinline__ void load(const ReplaceParams& p, uint32_t t) {
     const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-      const long long j = base - (long long)lane - 32 * k;
+      const uint32_t j = pos + lane + 32u * (uint32_t)k;
       w[k] = 0;
-      if (j < 0) continue;
-      if (k == 0 && first && lane == 0)
-        rec_load(p.rec, (uint32_t)j, &w[0], &carry);
-      else
-        asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(w[k]) : "l"(p.rec + 2ull * (unsigned long long)j) : "memory");
+      if (j < t)
+        asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(w[k]) : "l"(p.rec + 2ull * j) : "memory");
+    }
+    n0 = n1 = 0;
+    if (t - pos <= 32u * kPer && lane == 0) rec_load(p.rec, t - 1u, &n0, &n1);
+  }
+  // The kept count before super-tile t >= pos and the carry into it, after load; false when the wait
+  // gave up.
+  __device__ __forceinline__ bool reach(const ReplaceParams& p, uint32_t t, unsigned long long* K_out, uint32_t* c_out) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned long long tag = (unsigned long long)(p.epoch & 0xFFFFFFu);
+    unsigned long long t0 = 0;
+    uint32_t ns = 32;
+    for (;;) {
+      const bool lastw = t - pos <= 32u * kPer;
+      uint32_t part = 0;
+      bool ready = true;
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const uint32_t j = pos + lane + 32u * (uint32_t)k;
+        if (j < t) {
+          ready = ready && (w[k] >> 40) == tag && ((w[k] >> 38) & 3ull) != 0ull;
+          part += (uint32_t)rec_data(w[k]);
+        }
+      }
+      if (lastw && lane == 0)
+        ready = ready && (n0 >> 40) == tag && (n1 >> 40) == tag && ((n0 >> 38) & 3ull) != 0ull && ((n1 >> 38) & 3ull) != 0ull;
+      if (__all_sync(0xffffffffu, ready)) {
+        sum += __reduce_add_sync(0xffffffffu, part);
+        pos = lastw ? t : pos + 32u * kPer;
+        if (lastw) {
+          *K_out = sum;
+          *c_out = __shfl_sync(0xffffffffu, (uint32_t)rec_data(n1), 0);
+          return true;
+        }
+      } else {
+        if (aborted(p)) return false;
+        const unsigned long long now = global_ns();
+        if (t0 == 0) {
+          t0 = now;
+        } else if (now - t0 > kSpinLimitNs) {
+          if (lane == 0) set_error(p);
+          return false;
+        }
+        __nanosleep(ns);
+        if (ns < 128) ns <<= 1;
+      }
+      load(p, t);
     }
   }
 };
-__device__ __forceinline__ bool lookback_sum(const ReplaceParams& p, uint32_t t, unsigned long long* K_out,
-                                             uint32_t* c_out, uint32_t carry0) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const unsigned long long tag = p.epoch & 0xFFFFFFu;
-  unsigned long long acc = 0, t0 = 0;
-  long long base = (long long)t - 1;
-  bool first = true;
-  uint32_t ns = 32;
-  SumWindow W;
-  W.load(p, base, true);
-  for (;;) {
-    uint32_t D = 32u * SumWindow::kPer;  // distance of the nearest inclusive record
-    bool ready = true;
-    uint32_t part = 0;
-    unsigned long long Kd = 0;
-#pragma unroll
-    for (int k = 0; k < SumWindow::kPer; ++k) {
-      const long long j = base - (long long)lane - 32 * k;
-      const unsigned long long v = W.w[k];
-      uint32_t st = (v >> 40) == tag ? (uint32_t)(v >> 38) & 3u : 0u;
-      if (k == 0 && first && lane == 0 && ((W.carry >> 40) != tag || ((uint32_t)(W.carry >> 38) & 3u) != st)) st = 0;
-      if (j < 0) st = kStInc;  // the virtual super-tile before the first: nothing kept
-      const uint32_t okm = __ballot_sync(0xffffffffu, st != 0u), inc = __ballot_sync(0xffffffffu, st == (uint32_t)kStInc);
-      if (D == 32u * SumWindow::kPer) {  // (the same in every lane)
-        const uint32_t pl = inc ? (uint32_t)__ffs(inc) - 1u : 32u;
-        const uint32_t need = pl >= 31u ? 0xffffffffu : ((2u << pl) - 1u);
-        ready = ready && (okm & need) == need;
-        if (lane < pl) part += (uint32_t)rec_data(v);
-        if (inc) {
-          D = 32u * (uint32_t)k + pl;
-          Kd = __shfl_sync(0xffffffffu, j < 0 ? 0ull : rec_data(v), pl);
-        }
-      }
-    }
-    if (ready) {
-      if (first) {
-        const uint32_t c = base < 0 ? carry0 : (uint32_t)rec_data(W.carry);
-        *c_out = __shfl_sync(0xffffffffu, c, 0);
-        first = false;
-      }
-      acc += __reduce_add_sync(0xffffffffu, part);
-      if (D < 32u * SumWindow::kPer) {
-        *K_out = acc + Kd;
-        return true;
-      }
-      base -= 32 * SumWindow::kPer;
-    } else {
-      if (aborted(p)) return false;
-      const unsigned long long now = global_ns();
-      if (t0 == 0) {
-        t0 = now;
-      } else if (now - t0 > kSpinLimitNs) {
-        if (lane == 0) set_error(p);
-        return false;
-      }
-      __nanosleep(ns);
-      if (ns < 128) ns <<= 1;
-    }
-    W.load(p, base, first);
-  }
-}
 
 // Look-back for patterns of 5..64 bytes with a border: super-tile functions are tables over
 // carries in global memory; lane c holds entries c and (NE = 2) c + 32. 32 / NE predecessors per
@@ -4047,22 +4043,23 @@ __device__ __forceinline__ void fold_regions(const uint32_t* wt, const uint8_t* 
 
 template <int MODE>
 __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const __grid_constant__ ReplaceParams p) {
+  constexpr uint32_t NR = region_count(MODE), NS = region_slots(MODE), kTeams = kWorkers / NR;
+  constexpr uint32_t kNone = 0xFFFFFFFFu;
   extern __shared__ __align__(128) uint8_t smem[];
   // per slot: its load has landed; every worker's pass A is done; its function is known; its outputs
   // are placed; every worker's pass B is done
-  __shared__ __align__(8) uint64_t s_full[kSlots], s_adone[kSlots], s_folded[kSlots], s_ready[kSlots], s_bdone[kSlots];
-  __shared__ uint32_t s_tile[kSlots];
-  __shared__ uint32_t s_wcnt[kSlots][kWorkers], s_wend[kSlots][kWorkers];  // kModeFree: kept count, end of the last match
-  __shared__ uint8_t s_kind[kSlots][kWorkers];  // kModeSmall: 0 no candidate, 1 mixed, 2 all candidates
+  __shared__ __align__(8) uint64_t s_full[NS], s_adone[NS], s_folded[NS], s_ready[NS], s_bdone[NS];
+  __shared__ uint32_t s_tile[NS];
+  __shared__ uint32_t s_wcnt[NS][NR], s_wend[NS][NR];  // kModeFree: kept count, end of the last match
+  __shared__ uint8_t s_kind[NS][NR];  // kModeSmall: 0 no candidate, 1 mixed, 2 all candidates
   // per region: output offset in the super-tile's, length, first byte not covered by an earlier
   // match (relative to the super-tile), kept count
-  __shared__ uint4 s_reg[kSlots][kWorkers];
-  __shared__ unsigned long long s_O[kSlots];  // where the super-tile's output starts
-  __shared__ uint32_t s_total[kSlots], s_flags[kSlots], s_cin[kSlots];
-  __shared__ unsigned long long s_kept[kSlots];  // kept through the super-tile
-  __shared__ uint32_t s_supc[kSlots][64], s_supx[kSlots][64];  // its function: kept count, carry-out (kModeFree: entry 0)
-  __shared__ uint32_t s_last1[kSlots], s_cutlen[kSlots];  // kModeSmall: last kept start + 1; cut region's length
-  constexpr uint32_t kNone = 0xFFFFFFFFu;
+  __shared__ uint4 s_reg[NS][NR];
+  __shared__ unsigned long long s_O[NS];  // where the super-tile's output starts
+  __shared__ uint32_t s_total[NS], s_flags[NS], s_cin[NS];
+  __shared__ unsigned long long s_kept[NS];  // kept through the super-tile
+  __shared__ uint32_t s_supc[NS][64], s_supx[NS][64];  // its function: kept count, carry-out (kModeFree: entry 0)
+  __shared__ uint32_t s_last1[NS], s_cutlen[NS];  // kModeSmall: last kept start + 1; cut region's length
   constexpr uint32_t kWrite = 1u, kRuns = 2u, kCut = 4u;  // s_flags: write; all replacements; the region at n is cut
 
   const uint32_t L = p.L, R = p.R;
@@ -4070,7 +4067,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
   uint8_t* const ps = smem + lay.pat;
   uint8_t* const rs = smem + lay.rep;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  constexpr unsigned long long S = (unsigned long long)kWorkers * kRegion;
+  constexpr unsigned long long S = region_tile(MODE);
   const JobDims dims = job_dims(p, S);
   const unsigned long long n_all = dims.n_all, n = dims.n, n16 = dims.n16;
   const uint32_t NT = dims.NT, carry0 = dims.carry0;
@@ -4086,7 +4083,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     const unsigned long long a = (unsigned long long)t * S;
     const uint32_t bytes = (uint32_t)min(S + halo, n16 - a);
     mbar_arrive_expect_tx(&s_full[slot], bytes);
-    bulk_load_hint(smem + lay.slots + slot * kSlot, p.in + a, bytes, &s_full[slot], l2_policy_evict_first());
+    bulk_load_hint(smem + lay.slots + slot * region_slot(MODE), p.in + a, bytes, &s_full[slot], l2_policy_evict_first());
   };
   auto claim = [&]() -> uint32_t {
     const uint32_t c = atomicAdd(&p.res->tile_counter, 1u);
@@ -4095,12 +4092,12 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
   uint32_t issued = 0;  // loader: super-tiles and end marks issued
   uint32_t marks = 0;   // ... end marks among them (one for each look-back warp)
   if (tid == kLoader * 32u) {
-    for (uint32_t s = 0; s < kSlots; ++s) {
+    for (uint32_t s = 0; s < NS; ++s) {
       mbar_init(&s_full[s], 1);
-      mbar_init(&s_adone[s], kWorkers);
+      mbar_init(&s_adone[s], NR);
       mbar_init(&s_folded[s], 1);
       mbar_init(&s_ready[s], 1);
-      mbar_init(&s_bdone[s], kWorkers);
+      mbar_init(&s_bdone[s], NR);
       s_last1[s] = 0;
       s_cutlen[s] = 0;
     }
@@ -4108,14 +4105,14 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     // one super-tile when every CTA gets at most one (none is taken from a CTA that starts late),
     // else up to three ahead
     const uint32_t share = (NT + gridDim.x - 1u) / gridDim.x;
-    const uint32_t depth = share < kSlots ? (share ? share : 1u) : kSlots;
+    const uint32_t depth = share < NS ? (share ? share : 1u) : NS;
     for (; issued < depth && !marks; ++issued) {
       const uint32_t t = claim();
       marks = t == kNone ? 1u : 0u;
       issue(issued, t);
     }
     if (share <= 1u) {
-      static_assert(kLookbacks < kSlots, "one super-tile and the end marks");
+      static_assert(kLookbacks < NS, "one super-tile and the end marks");
       for (; marks < kLookbacks; ++marks) issue(issued++, kNone);
     }
   }
@@ -4178,8 +4175,8 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     bool ok = true;
     uint32_t done = 0;  // super-tiles written
     auto finish = [&]() {
-      const uint32_t slot = done % kSlots;
-      ok = pipe_wait(p, &s_bdone[slot], (done / kSlots) & 1u);
+      const uint32_t slot = done % NS;
+      ok = pipe_wait(p, &s_bdone[slot], (done / NS) & 1u);
       if (MODE == kModeSmall && ok && lane == 0) {
         record(s_tile[slot], s_O[slot], s_total[slot] + s_cutlen[slot], s_last1[slot], s_cin[slot], s_kept[slot]);
         s_last1[slot] = 0;
@@ -4190,12 +4187,12 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     };
 #pragma unroll 1
     while (marks < kLookbacks && ok) {
-      if (issued >= kSlots) finish();
+      if (issued >= NS) finish();
       if (!ok) break;
       uint32_t t = kNone;
       if (lane == 0) {
         if (!marks) t = claim();
-        issue(issued % kSlots, t);
+        issue(issued % NS, t);
       }
       t = __shfl_sync(0xffffffffu, t, 0);
       marks += t == kNone ? 1u : 0u;
@@ -4203,7 +4200,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     }
     while (MODE == kModeSmall && ok && done + marks < issued) finish();
     // after a wait that gave up: the loads in flight end before this CTA does
-    for (uint32_t j = done; !ok && j < issued; ++j) (void)wait_tile(&s_full[j % kSlots], (j / kSlots) & 1u);
+    for (uint32_t j = done; !ok && j < issued; ++j) (void)wait_tile(&s_full[j % NS], (j / NS) & 1u);
     if (lane == 0) {
       __threadfence();
       const unsigned int d = atomicAdd(&p.res->done_ctas, 1u);
@@ -4222,17 +4219,17 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     // CTA's look-back waits for, later super-tiles elsewhere never wait for it.
 #pragma unroll 1
     for (uint32_t i = 0;; ++i) {
-      const uint32_t slot = i % kSlots, par = (i / kSlots) & 1u;
+      const uint32_t slot = i % NS, par = (i / NS) & 1u;
       if (!pipe_wait(p, &s_full[slot], par)) break;
       const uint32_t t = s_tile[slot];
       if (t == kNone || !pipe_wait(p, &s_adone[slot], par)) break;
       if (MODE == kModeFree) {
-        const uint32_t wc = lane < kWorkers ? s_wcnt[slot][lane] : 0u;
-        const uint32_t we = lane < kWorkers ? s_wend[slot][lane] : 0u;
+        const uint32_t wc = lane < NR ? s_wcnt[slot][lane] : 0u;
+        const uint32_t we = lane < NR ? s_wend[slot][lane] : 0u;
         const uint32_t sum = __reduce_add_sync(0xffffffffu, wc), top = __reduce_max_sync(0xffffffffu, we);
         const uint32_t lco = top > (uint32_t)S ? top - (uint32_t)S : 0u;  // reach past the super-tile
         if (lane == 0) {
-          if (t > 0) rec_store(p.rec, t, rec_word(tag, kStAgg, sum), rec_word(tag, kStAgg, lco));
+          rec_store(p.rec, t, rec_word(tag, kStAgg, sum), rec_word(tag, kStAgg, lco));
           s_supc[slot][0] = sum;
           s_supx[slot][0] = lco;
         }
@@ -4241,11 +4238,11 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
         uint8_t* const wrec = smem + lay.wrec + slot * lay.wrec_set;
         const uint32_t* const wt = reinterpret_cast<const uint32_t*>(smem + lay.wtab + slot * lay.wtab_set);
         if (L == 2u)
-          fold_regions<2>(wt, s_kind[slot], wrec, kWorkers, &sup_cnt, &sup_carry);
+          fold_regions<2>(wt, s_kind[slot], wrec, NR, &sup_cnt, &sup_carry);
         else if (L == 3u)
-          fold_regions<3>(wt, s_kind[slot], wrec, kWorkers, &sup_cnt, &sup_carry);
+          fold_regions<3>(wt, s_kind[slot], wrec, NR, &sup_cnt, &sup_carry);
         else
-          fold_regions<4>(wt, s_kind[slot], wrec, kWorkers, &sup_cnt, &sup_carry);
+          fold_regions<4>(wt, s_kind[slot], wrec, NR, &sup_cnt, &sup_carry);
         const unsigned long long e = lane < L ? ((unsigned long long)sup_cnt | ((unsigned long long)sup_carry << 17)) : 0ull;
         const unsigned long long e1 = __shfl_sync(0xffffffffu, e, 1), e2 = __shfl_sync(0xffffffffu, e, 2),
                                  e3 = __shfl_sync(0xffffffffu, e, 3);
@@ -4260,7 +4257,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
         for (uint32_t c = lane; c < L; c += 32u) {
           uint32_t y = c, kc = 0;
 #pragma unroll 1
-          for (uint32_t q = 0; q < kWorkers; ++q) {
+          for (uint32_t q = 0; q < NR; ++q) {
             wrec[q * L + c] = (uint8_t)y;
             const uint32_t v = region_entry(slot, q, y);
             kc += v & 0xFFFFu;
@@ -4282,90 +4279,105 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
 
   if (warp >= kLookback) {
     // ================================================================ look-back warps
+    RunningSum run;  // kModeFree
+    run.init();
 #pragma unroll 1
     for (uint32_t i = warp - kLookback;; i += kLookbacks) {
-      const uint32_t slot = i % kSlots, par = (i / kSlots) & 1u;
+      const uint32_t slot = i % NS, par = (i / NS) & 1u;
       if (!pipe_wait(p, &s_full[slot], par)) break;
       const uint32_t t = s_tile[slot];
       if (t == kNone) break;
       const unsigned long long tstart = (unsigned long long)t * S;
-      // ---- what the super-tiles before leave: kept count and carry. It needs nothing of this one, so
-      // it runs while the workers search this super-tile.
+      uint32_t total = 0, last1 = 0;
+      bool runs = false, cuts = false;
+      // The regions' outputs (lane q: region q) from the carry c into the super-tile.
+      auto place = [&](uint32_t c) {
+        const uint32_t tvalid = n - tstart < S ? (uint32_t)(n - tstart) : (uint32_t)S;
+        const uint32_t qs = lane * kRegion;
+        const uint32_t vb = (lane < NR && tvalid > qs) ? min(tvalid - qs, kRegion) : 0u;
+        uint32_t wc = 0, x0 = qs, olen = 0;
+        bool cut = false;  // kModeSmall: a region cut at n whose last match may run past n (exact length later)
+        if (MODE == kModeFree) {
+          uint32_t we = 0;
+          if (lane < NR) {
+            wc = s_wcnt[slot][lane];
+            we = s_wend[slot][lane];
+          }
+          uint32_t cov = we;  // furthest end of a match before the region
+          if (L > kRegion) {
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+              const uint32_t o = __shfl_up_sync(0xffffffffu, cov, d);
+              if (lane >= (uint32_t)d) cov = o > cov ? o : cov;
+            }
+          }
+          cov = __shfl_up_sync(0xffffffffu, cov, 1);  // (otherwise only the region before reaches here)
+          if (lane == 0) cov = 0;
+          cov = cov > c ? cov : c;
+          x0 = cov > qs ? cov : qs;
+          const uint32_t over = (wc && we > qs + vb) ? we - (qs + vb) : 0u;
+          olen = vb - min(x0 - qs, vb) - wc * L + over + wc * R;
+          last1 = __reduce_max_sync(0xffffffffu, wc ? we - L + 1u : 0u);
+        } else if (vb) {
+          const uint32_t cw = (smem + lay.wrec + slot * lay.wrec_set)[lane * L + c];
+          const uint32_t e = region_entry(slot, lane, cw);
+          wc = e & 0xFFFFu;
+          x0 = qs + cw;
+          olen = vb - min(cw, vb) - wc * L + (e >> 16) + wc * R;
+          cut = vb < kRegion && p.hold != 0ull && wc != 0u;
+          if (cut) olen = 0;
+        }
+        const uint32_t incl = warp_incl_scan(olen, OpSum());
+        total = __shfl_sync(0xffffffffu, incl, 31);
+        runs = R <= 64u && __all_sync(0xffffffffu, olen == wc * R && !cut);
+        cuts = __any_sync(0xffffffffu, cut);  // at most one region of the launch
+        if (lane < NR) s_reg[slot][lane] = make_uint4(incl - olen, olen, x0, wc);
+      };
+      // ---- what the super-tiles before leave: kept count and carry. Its first window is on its way while
+      // the workers search this super-tile and (kModeFree) its regions are placed as if no match
+      // reached into it, which is right for nearly all.
       unsigned long long K = 0;
       uint32_t c = carry0;
       bool ok = true;
-      if (t > 0) {
-        if (MODE == kModeFree)
-          ok = lookback_sum(p, t, &K, &c, carry0);
-        else if (L == 2u)
-          ok = lookback_small_rec<2>(p, t, &K, &c, carry0);
-        else if (L == 3u)
-          ok = lookback_small_rec<3>(p, t, &K, &c, carry0);
-        else if (L == 4u)
-          ok = lookback_small_rec<4>(p, t, &K, &c, carry0);
-        else if (L <= 32u)
-          ok = lookback_table<1>(p, t, L, &K, &c, carry0);
-        else
-          ok = lookback_table<2>(p, t, L, &K, &c, carry0);
+      if (MODE == kModeFree) {
+        if (t > 0) run.load(p, t);
+        if (!pipe_wait(p, &s_folded[slot], par)) break;
+        place(0u);
+        if (t > 0) ok = run.reach(p, t, &K, &c);
+      } else {
+        if (t > 0) {
+          if (L == 2u)
+            ok = lookback_small_rec<2>(p, t, &K, &c, carry0);
+          else if (L == 3u)
+            ok = lookback_small_rec<3>(p, t, &K, &c, carry0);
+          else if (L == 4u)
+            ok = lookback_small_rec<4>(p, t, &K, &c, carry0);
+          else if (L <= 32u)
+            ok = lookback_table<1>(p, t, L, &K, &c, carry0);
+          else
+            ok = lookback_table<2>(p, t, L, &K, &c, carry0);
+        }
+        if (!pipe_wait(p, &s_folded[slot], par)) break;
       }
       if (!ok) K = c = 0;
-      if (!pipe_wait(p, &s_folded[slot], par)) break;
       const unsigned long long Kin = K + s_supc[slot][MODE == kModeFree ? 0u : c];
       const uint32_t cout = s_supx[slot][MODE == kModeFree ? 0u : c];
-      if (lane == 0) {
-        if (use_rec) rec_store(p.rec, t, rec_word(tag, kStInc, Kin), rec_word(tag, kStInc, cout));
-        __stcg(&p.incl[t].kept, Kin);
-        __stcg(&p.incl[t].carry, cout);
-        if (!use_rec) {
+      if (MODE == kModeSmall && lane == 0) {  // the inclusive prefix, for later super-tiles
+        if (use_rec) {
+          rec_store(p.rec, t, rec_word(tag, kStInc, Kin), rec_word(tag, kStInc, cout));
+        } else {
+          __stcg(&p.incl[t].kept, Kin);
+          __stcg(&p.incl[t].carry, cout);
           __threadfence();
           st_release_u32(p.status + t, (p.epoch << 2) | kStInc);
         }
       }
-      // ---- place the regions' outputs (lane q: region q). The output range starts len_bias bytes into
-      // out[], and the carry0 leading bytes covered by a match kept before this buffer are not emitted here.
+      if (MODE == kModeSmall || c != 0u) place(c);
+      // The output range starts len_bias bytes into out[], and the carry0 leading bytes covered by a match
+      // kept before this buffer are not emitted here.
       const unsigned long long O = p.len_bias + (unsigned long long)((long long)(tstart + c) - (long long)carry0 +
                                                                      (long long)K * ((long long)R - (long long)L));
-      const uint32_t tvalid = n - tstart < S ? (uint32_t)(n - tstart) : (uint32_t)S;
-      const uint32_t qs = lane * kRegion;
-      const uint32_t vb = (lane < kWorkers && tvalid > qs) ? min(tvalid - qs, kRegion) : 0u;
-      uint32_t wc = 0, x0 = qs, olen = 0, last1 = 0;
-      bool cut = false;  // kModeSmall: a region cut at n whose last match may run past n (exact length later)
-      if (MODE == kModeFree) {
-        uint32_t we = 0;
-        if (lane < kWorkers) {
-          wc = s_wcnt[slot][lane];
-          we = s_wend[slot][lane];
-        }
-        uint32_t cov = we;  // furthest end of a match before the region
-        if (L > kRegion) {
-#pragma unroll
-          for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xffffffffu, cov, d);
-            if (lane >= (uint32_t)d) cov = o > cov ? o : cov;
-          }
-        }
-        cov = __shfl_up_sync(0xffffffffu, cov, 1);  // (otherwise only the region before reaches here)
-        if (lane == 0) cov = 0;
-        cov = cov > c ? cov : c;
-        x0 = cov > qs ? cov : qs;
-        const uint32_t over = (wc && we > qs + vb) ? we - (qs + vb) : 0u;
-        olen = vb - min(x0 - qs, vb) - wc * L + over + wc * R;
-        last1 = __reduce_max_sync(0xffffffffu, wc ? we - L + 1u : 0u);
-      } else if (vb) {
-        const uint32_t cw = (smem + lay.wrec + slot * lay.wrec_set)[lane * L + c];
-        const uint32_t e = region_entry(slot, lane, cw);
-        wc = e & 0xFFFFu;
-        x0 = qs + cw;
-        olen = vb - min(cw, vb) - wc * L + (e >> 16) + wc * R;
-        cut = vb < kRegion && p.hold != 0ull && wc != 0u;
-        if (cut) olen = 0;
-      }
-      const uint32_t incl = warp_incl_scan(olen, OpSum());
-      const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
       const bool fits = O <= p.out_cap && total <= p.out_cap - O;
-      const bool runs = R <= 64u && __all_sync(0xffffffffu, olen == wc * R && !cut);
-      const bool cuts = __any_sync(0xffffffffu, cut);  // at most one region of the launch
-      if (lane < kWorkers) s_reg[slot][lane] = make_uint4(incl - olen, olen, x0, wc);
       if (lane == 0) {
         s_O[slot] = O;
         s_total[slot] = total;
@@ -4377,6 +4389,10 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       if (lane == 0) {
         mbar_arrive(&s_ready[slot]);
         if (!fits) atomicExch(&p.res->overflow_epoch, p.epoch);
+        if (MODE == kModeFree || use_rec) {  // (query_prefix reads these)
+          __stcg(&p.incl[t].kept, Kin);
+          __stcg(&p.incl[t].carry, cout);
+        }
         if (MODE == kModeFree) record(t, O, total, last1, c, Kin);
       }
       __syncwarp();
@@ -4394,14 +4410,14 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
   for (int k = 0; k < 4; ++k) r[k] = ((p.p4 >> (8 * k)) & 0xFFu) * 0x01010101u;
   uint8_t* const stg = smem + lay.scratch + warp * (lay.stage + 512u);
   uint4* const gm = reinterpret_cast<uint4*>(stg + lay.stage);
-  const uint32_t qs = warp * kRegion;  // this warp's region of every super-tile
+  const uint32_t wq = warp % NR, qs = wq * kRegion;  // this warp's region of its team's super-tiles
   bool hot = false;                    // the last region searched had a candidate: no detection pass
 
   // ---- pass A: candidates of the warp's region of super-tile t and what the control warp needs of it
   auto pass_a = [&](const uint32_t t, const uint32_t slot) {
     const unsigned long long rstart = (unsigned long long)t * S + qs;
-    const uint8_t* const tb = smem + lay.slots + slot * kSlot + qs;
-    uint64_t* const row = reinterpret_cast<uint64_t*>(smem + lay.masks) + (slot * kWorkers + warp) * 32u;
+    const uint8_t* const tb = smem + lay.slots + slot * region_slot(MODE) + qs;
+    uint64_t* const row = reinterpret_cast<uint64_t*>(smem + lay.masks) + (slot * NR + wq) * 32u;
     uint32_t cnt = 0, end = 0, kind = 0;
     bool found = rstart < n;
     // presence index: no candidate can start in a chunk that lacks the first byte
@@ -4488,8 +4504,8 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
           if (kind == 1u) {
             uint8_t* const wt = smem + lay.wtab + slot * lay.wtab_set;
             if (L <= 4u) {
-              uint8_t* const sr = smem + lay.srec + slot * lay.srec_set + (warp * 32u + lane) * L;
-              uint32_t* const wt4 = reinterpret_cast<uint32_t*>(wt) + warp * L;
+              uint8_t* const sr = smem + lay.srec + slot * lay.srec_set + (wq * 32u + lane) * L;
+              uint32_t* const wt4 = reinterpret_cast<uint32_t*>(wt) + wq * L;
               if (L == 2u)
                 ks_warp_tables<2>(mask, p.inv_l, p.stride_mask, sr, wt4);
               else if (L == 3u)
@@ -4504,7 +4520,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
                   const uint32_t s = (uint32_t)__ffs(sm) - 1u;
                   x = walk_segment(x, s, row[s], L, &kc);
                 }
-                reinterpret_cast<uint16_t*>(wt)[warp * L + c] = (uint16_t)((kc << 6) | (x > kRegion ? x - kRegion : 0u));
+                reinterpret_cast<uint16_t*>(wt)[wq * L + c] = (uint16_t)((kc << 6) | (x > kRegion ? x - kRegion : 0u));
               }
             }
           }
@@ -4513,10 +4529,10 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     }
     if (lane == 0) {
       if (MODE == kModeFree) {
-        s_wcnt[slot][warp] = cnt;
-        s_wend[slot][warp] = end;
+        s_wcnt[slot][wq] = cnt;
+        s_wend[slot][wq] = end;
       } else {
-        s_kind[slot][warp] = (uint8_t)kind;
+        s_kind[slot][wq] = (uint8_t)kind;
       }
     }
   };
@@ -4608,9 +4624,9 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
   // ---- pass B: the output of the warp's region of super-tile t
   auto pass_b = [&](const uint32_t t, const uint32_t slot) {
     const unsigned long long tstart = (unsigned long long)t * S;
-    uint8_t* const tb = smem + lay.slots + slot * kSlot;
+    uint8_t* const tb = smem + lay.slots + slot * region_slot(MODE);
     const uint32_t flags = s_flags[slot];
-    const uint4 e = s_reg[slot][warp];  // output offset, length, first uncovered byte, kept count
+    const uint4 e = s_reg[slot][wq];  // output offset, length, first uncovered byte, kept count
     const unsigned long long O = s_O[slot], g0 = O + e.x;
     const bool write = (flags & kWrite) != 0u;
     const uint4* const t16 = reinterpret_cast<const uint4*>(smem + lay.tab16);
@@ -4623,8 +4639,8 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       const uint32_t total = s_total[slot];
       if (write && total) {
         const unsigned long long end = O + total;
-        const unsigned long long s0 = warp == 0 ? O : (O + (unsigned long long)total * warp / kWorkers) & ~15ull;
-        const unsigned long long s1 = warp == kWorkers - 1u ? end : (O + (unsigned long long)total * (warp + 1u) / kWorkers) & ~15ull;
+        const unsigned long long s0 = wq == 0 ? O : (O + (unsigned long long)total * wq / NR) & ~15ull;
+        const unsigned long long s1 = wq == NR - 1u ? end : (O + (unsigned long long)total * (wq + 1u) / NR) & ~15ull;
         const unsigned long long a = s0 > O ? s0 : O, b = s1 < end ? s1 : end;
         if (b > a) warp_emit_replace(p.out, t16, rs, R, step512, rmag, a, (uint32_t)(b - a), mod_small((uint32_t)(a - O), R, rmag));
       }
@@ -4635,16 +4651,16 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       if (write && e.y) warp_emit_replace(p.out, t16, rs, R, step512, rmag, g0, e.y);
       if (MODE == kModeSmall) last1 = e.z + (e.w - 1u) * L + 1u;
     } else {
-      const uint64_t* const row = reinterpret_cast<const uint64_t*>(smem + lay.masks) + (slot * kWorkers + warp) * 32u;
+      const uint64_t* const row = reinterpret_cast<const uint64_t*>(smem + lay.masks) + (slot * NR + wq) * 32u;
       uint64_t kept = row[lane];
       const uint32_t c0 = e.z - qs;  // bytes of the region covered by an earlier match
       if (MODE == kModeSmall) {
         // the greedy from the exact carry into the region
         uint32_t xs = 0;  // carry into the lane's segment
-        if (s_kind[slot][warp] == 2u) {
+        if (s_kind[slot][wq] == 2u) {
           xs = dense_seg_carry(c0, lane * 64u, L);
         } else if (L <= 4u) {
-          xs = (smem + lay.srec + slot * lay.srec_set)[(warp * 32u + lane) * L + c0];
+          xs = (smem + lay.srec + slot * lay.srec_set)[(wq * 32u + lane) * L + c0];
         } else {
           uint32_t x = c0, kc = 0;
           for (uint32_t sm = __ballot_sync(0xffffffffu, kept != 0ull); sm; sm &= sm - 1u) {
@@ -4703,13 +4719,13 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
 
   // Pass A of the next super-tile as soon as it is loaded, else pass B of the oldest one placed: while
   // slots are left, a look-back that waits elsewhere delays no function of this CTA.
-  uint32_t ia = 0, ib = 0;  // next super-tile to search, next to write
+  uint32_t ia = warp / NR, ib = ia;  // the team's next super-tile to search, next to write
   bool more = true;
 #pragma unroll 1
   while (more || ib < ia) {
-    uint64_t* const full = &s_full[ia % kSlots];
-    uint64_t* const ready = &s_ready[ib % kSlots];
-    const uint32_t pa = (ia / kSlots) & 1u, pb = (ib / kSlots) & 1u;
+    uint64_t* const full = &s_full[ia % NS];
+    uint64_t* const ready = &s_ready[ib % NS];
+    const uint32_t pa = (ia / NS) & 1u, pb = (ib / NS) & 1u;
     uint32_t what = 0;  // 1: pass A, 2: pass B
     unsigned long long t0 = 0;
     for (;;) {
@@ -4729,7 +4745,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     }
     // (every lane observes the phase itself: the slot was written by the async proxy)
     if (!pipe_wait(p, what == 1u ? full : ready, what == 1u ? pa : pb)) break;
-    const uint32_t slot = (what == 1u ? ia : ib) % kSlots;
+    const uint32_t slot = (what == 1u ? ia : ib) % NS;
     const uint32_t t = s_tile[slot];
     if (what == 1u) {
       if (t == kNone) {
@@ -4739,14 +4755,18 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       pass_a(t, slot);
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_adone[slot]);
-      ++ia;
+      ia += kTeams;
     } else {
       pass_b(t, slot);
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_bdone[slot]);
-      ++ib;
+      ib += kTeams;
     }
   }
+}
+
+__host__ __device__ __forceinline__ uint32_t super_tile_bytes(const ReplaceParams& p) {
+  return p.nsub == kRegionSub ? region_tile(p.mode) : p.nsub * (uint32_t)kTile;
 }
 
 // One CTA answers query_prefix for a super-tile layout: kept starts before limit and the
@@ -4768,7 +4788,7 @@ __global__ void __launch_bounds__(kThreads) query_super_kernel(const __grid_cons
   uint64_t* masks = reinterpret_cast<uint64_t*>(smem + lay.masks);
   const uint32_t tid = threadIdx.x, sb = tid * kSeg;
   const unsigned long long n = p.n, n16 = (n + 15ull) & ~15ull;
-  const unsigned long long S = (unsigned long long)p.nsub * kTile;
+  const unsigned long long S = super_tile_bytes(p);
   const unsigned long long limit = p.query_limit64;
   const uint32_t t = (uint32_t)(limit / S);
   const unsigned long long rel = limit - (unsigned long long)t * S;
@@ -4973,21 +4993,24 @@ constexpr uint32_t kApplySub = 4;
 static_assert(kApplySub != kRegionSub, "nsub tells the kernel");
 
 // Which kernel takes an input. The region kernel has the shorter path for one super-tile and more of
-// the chip at work on small inputs; its three slots hold a super-tile for its load, its
-// look-back and its output, so on large inputs the look-back bounds it, where the super-tile kernel
-// reads the input a second time from L2. Microseconds, super-tile kernel / region kernel:
-//                      1 MiB      16 MiB     32 MiB     64 MiB     128 MiB
-//   entity in text   21.4/14.2  26.2/21.6  36.8/32.2  56.9/52.9  89.4/94.5
-//   binary deletion  16.0/13.6  26.3/21.3  30.2/29.2  45.3/47.1  74.1/83.2
-//   blanks to %20    36.3/21.3  44.3/42.9  71.8/65.2   121/119    205/216
-//   a run, L = 1     15.6/13.2  21.9/24.0  35.0/37.4  57.8/61.9  96.1/112
-//   a run, L = 2     15.8/14.8  18.4/21.6  22.4/30.9  32.1/47.8  55.5/84.9
+// the chip at work on small inputs; its slots hold a super-tile for its load, its look-back and its
+// output, so on large inputs the look-back bounds it, where the super-tile kernel reads the input a second
+// time from L2. Microseconds, super-tile kernel / region kernel:
+//                      1 MiB      16 MiB     64 MiB     128 MiB
+//   entity in text   21.4/13.2  26.2/20.3  56.9/55.5  89.4/102
+//   binary deletion  16.0/12.7  26.3/17.5  45.3/41.0  74.1/73.6
+//   ACGT -> N        34.2/13.6  45.1/28.1   129/77.5   219/145 (150 with the gather)
+//   line ends, CRLF  32.4/14.3  39.9/33.2   101/88.7   178/159
+//   a run, L = 1     15.6/12.4  21.9/21.7  57.8/54.7  96.1/98.5
+//   a run, L = 2     15.8/14.8  18.4/21.6  32.1/47.8  55.5/84.9 (overlapping itself: up to 8 MiB)
 // Bordered patterns of 5 to 64 bytes are always the region kernel's (64 MiB run of 6: 397 -> 122 us;
-// 32 MiB of rule lines, L = 40, which the tile kernel took before: 1020 -> 108 us).
+// 32 MiB of rule lines, L = 40, which the tile kernel took before: 1020 -> 83 us).
+uint32_t super_tile(const ReplaceParams& p) { return super_tile_bytes(p); }
+
 uint32_t super_nsub(uint32_t mode, uint32_t L, unsigned long long n) {
   if (mode == kModeMulti) return kApplySub;
   if (mode == kModeSmall && L > 4u) return kRegionSub;
-  const unsigned long long most = mode == kModeFree ? (L >= 2u ? 64ull << 20 : 32ull << 20) : 8ull << 20;
+  const unsigned long long most = mode == kModeFree ? 64ull << 20 : 8ull << 20;
   if (mode == kModeFree || (mode == kModeSmall && L >= 2u)) return n <= most ? kRegionSub : kApplySub;
   return 0;
 }
@@ -5005,7 +5028,7 @@ cudaError_t super_attributes() {
   cudaError_t e = cudaFuncSetAttribute(replace_super_kernel<MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        220 * 1024);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(replace_region_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 223 * 1024);
+    e = cudaFuncSetAttribute(replace_region_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 221 * 1024);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(query_super_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e == cudaSuccess) attr_dev_mask |= 1ull << (dev & 63);

@@ -203,10 +203,12 @@ void prepare_pattern_fields(ReplaceParams& p, const uint8_t* pat, uint32_t L);
 uint32_t tile_kernel_smem_bytes(uint32_t mode, uint32_t L, uint32_t R);
 // Launch one apply. grid_ctas_out receives the number of CTAs launched.
 cudaError_t launch_replace(const ReplaceParams& p, cudaStream_t st, int* grid_ctas_out);
-// Sub-tiles per super-tile for an input of n bytes (3: the region kernel, else the super-tile kernel),
-// or 0 when (mode, L) needs the tile kernel.
+// Which kernel takes an input of n bytes: 1 the region kernel, more the super-tile kernel (its sub-tiles
+// per super-tile), 0 the tile kernel (mode, L).
 uint32_t super_nsub(uint32_t mode, uint32_t L, unsigned long long n);
-// Launch one apply with the super-tile kernel (p.nsub > 0, p.tile_last set).
+// Bytes of a super-tile of the kernel that p.nsub > 0 names.
+uint32_t super_tile(const ReplaceParams& p);
+// Launch one apply with that kernel (p.nsub > 0, p.tile_last set).
 cudaError_t launch_replace_super(const ReplaceParams& p, cudaStream_t st, int* grid_ctas_out);
 // Query for an apply made by the super-tile kernel: p.query_limit64 = limit (< p.n).
 cudaError_t launch_query_super(const ReplaceParams& p, cudaStream_t st);

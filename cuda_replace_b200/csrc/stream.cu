@@ -120,7 +120,7 @@ struct Stream {
     if (d2h) cudaStreamDestroy(d2h);
   }
 
-  size_t tile_bytes(int k) const { return (size_t)crb::kTile * st[(size_t)k].proto.nsub; }
+  size_t tile_bytes(int k) const { return crb::super_tile(st[(size_t)k].proto); }
 
   // Output capacity planned for stage k with input capacity in_cap: a quarter over the
   // chunk, scaled by the stage's growth factor, never above the worst case of the pair.

@@ -1,5 +1,5 @@
 """The region kernel and the line between it and the super-tile kernel: sizes around its 2 KiB regions
-and 48 KiB super-tiles, patterns of every carry class, uniform and periodic texts, query_prefix."""
+and its super-tiles (24 KiB, 48 KiB for patterns that overlap themselves), patterns of every carry class, uniform and periodic texts, query_prefix."""
 import numpy as np
 import pytest
 
@@ -8,7 +8,8 @@ from cuda_replace_b200.cuda_replace_wrapper import Session
 pytestmark = pytest.mark.gpu
 
 T = 49152
-SIZES = [1, 63, 64, 65, 2047, 2048, 2049, T - 1, T, T + 1, T + 2048, 2 * T + 2049, 7 * T + 31, 200 * T + 777]
+SIZES = [1, 63, 64, 65, 2047, 2048, 2049, T // 2 - 1, T // 2, T // 2 + 1, T - 1, T, T + 1, T + 2048, 2 * T + 2049,
+         7 * T + 31, 200 * T + 777]
 PATTERNS = [b"a", b"aa", b"aaa", b"aaaa", b"aaaaa", b"a" * 31, b"a" * 32, b"a" * 33, b"a" * 40, b"a" * 63, b"a" * 64,
             b"ab", b"aba", b"abab", b"ababa", b"abaababaab", b"ab" * 16, b"ab" * 20 + b"a", b"abc" * 21,
             b"ba", b"baaa", b"b" + b"a" * 63, b"ab" + b"c" * 62 + b"ab"]
@@ -41,7 +42,7 @@ def test_sizes_and_carries(cr_lib, pat):
                         assert s.query_prefix(limit) == (kept, last), (n, i, limit)
 
 
-@pytest.mark.parametrize("pat,edge", [(b"q", 32 << 20), (b"qz", 64 << 20), (b"qq", 8 << 20)])
+@pytest.mark.parametrize("pat,edge", [(b"q", 64 << 20), (b"qz", 64 << 20), (b"qq", 8 << 20)])
 def test_either_side_of_the_kernel_choice(cr_lib, pat, edge):
     rng = np.random.default_rng(len(pat))
     base = rng.integers(0, 256, size=edge + 1, dtype=np.uint8)
