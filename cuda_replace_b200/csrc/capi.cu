@@ -157,6 +157,7 @@ struct Session {
   cudaStream_t async_stream = nullptr;  // stream of the last cuda_replace_apply_device_async
   uint32_t async_epoch = 0;
   bool async_copy = false;          // the last async call copied its input (n < pattern length)
+  bool async_mirror = false;        // ... its launch writes res_host itself
   unsigned long long async_n = 0;   // ... and this many bytes
   cudaEvent_t ev_order = nullptr;   // orders the session stream and a caller stream
 
@@ -180,6 +181,8 @@ cudaError_t dev_grow(uint8_t** ptr, size_t* cap, size_t need, bool keep, size_t 
   uint8_t* p = nullptr;
   cudaError_t e = cudaMalloc(&p, new_cap);
   if (e != cudaSuccess) {
+    cudaGetLastError();
+    crb::dev_blocks_trim();
     // retry without headroom before giving up
     const size_t tight = round_up(need + 4096, 4096);
     e = cudaMalloc(&p, tight);
@@ -341,45 +344,87 @@ bool host_is_pinned(const void* p) {
   return a.type == cudaMemoryTypeHost;
 }
 
-// Host -> device copy of len bytes. A large pageable source is staged through two page-locked
-// 32 MiB buffers filled by several host threads, so the copy runs near the host link's speed
-// (a pageable cudaMemcpy goes through the driver's single-threaded staging).
-cudaError_t upload_host(uint8_t* dst, const uint8_t* src, size_t len, cudaStream_t st) {
-  const size_t kChunk = 32u << 20;
-  if (len < (8u << 20) || host_is_pinned(src)) return cudaMemcpyAsync(dst, src, len, cudaMemcpyHostToDevice, st);
+// Pieces of a pageable transfer staged through page-locked memory: large enough to copy on all host
+// threads, small enough that the copy of one hides behind the link's work on the one before.
+size_t stage_piece(size_t len) {
+  return std::min<size_t>((size_t)32 << 20, std::max<size_t>((size_t)1 << 20, round_up(len / 16, (size_t)1 << 18)));
+}
+
+// Host -> device copy of len bytes. A large pageable source is staged piece by piece through three
+// page-locked slots filled by the host threads (a pageable cudaMemcpy goes through the driver's
+// single-threaded staging; in pieces of 32 MiB the first copy hid behind nothing: 12 MiB took 2.1 ms,
+// now 0.5, 64 MiB 4.0 ms, now 2.5; the copies and the link share the host's memory bandwidth).
+cudaError_t upload_host(Session* s, uint8_t* dst, const uint8_t* src, size_t len, cudaStream_t st) {
+  if (len < (3u << 20) || host_is_pinned(src)) return cudaMemcpyAsync(dst, src, len, cudaMemcpyHostToDevice, st);
+  const size_t piece = stage_piece(len);
   cudaError_t e = cudaSuccess;
-  uint8_t* stage[2] = {nullptr, nullptr};
-  cudaEvent_t ev[2] = {nullptr, nullptr};
-  for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
-    stage[b] = static_cast<uint8_t*>(pinned_pool().get(kChunk, &e));
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming);
-  }
-  for (size_t off = 0, i = 0; off < len && e == cudaSuccess; off += kChunk, ++i) {
-    const int b = (int)(i & 1);
-    const size_t m = std::min(kChunk, len - off);
-    if (i >= 2) e = cudaEventSynchronize(ev[b]);  // stage[b] has reached the device
+  uint8_t* stage = static_cast<uint8_t*>(pinned_pool().get(3 * piece, &e));
+  if (!stage) return e;
+  for (int b = 0; b < 3 && e == cudaSuccess; ++b)
+    if (!s->ev_stage[b]) e = cudaEventCreateWithFlags(&s->ev_stage[b], cudaEventDisableTiming);
+  for (size_t off = 0, i = 0; off < len && e == cudaSuccess; off += piece, ++i) {
+    const int b = (int)(i % 3);
+    const size_t m = std::min(piece, len - off);
+    if (i >= 3) e = cudaEventSynchronize(s->ev_stage[b]);  // the slot has reached the device
     if (e != cudaSuccess) break;
-    crb::parallel_memcpy(stage[b], src + off, m);
-    e = cudaMemcpyAsync(dst + off, stage[b], m, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaEventRecord(ev[b], st);
+    crb::parallel_memcpy(stage + b * piece, src + off, m);
+    e = cudaMemcpyAsync(dst + off, stage + b * piece, m, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaEventRecord(s->ev_stage[b], st);
   }
   const cudaError_t se = cudaStreamSynchronize(st);  // the staging goes back to the pool
-  for (int b = 0; b < 2; ++b) {
-    if (ev[b]) cudaEventDestroy(ev[b]);
-    if (stage[b]) pinned_pool().put(stage[b]);
-  }
+  pinned_pool().put(stage);
   return e != cudaSuccess ? e : se;
 }
 
-int session_load(Session* s, const uint8_t* src, size_t len) {
+// The session buffer to caller memory dst[0, s->len): a large pageable dst by way of a pooled page-locked
+// block. Up to 32 MiB each piece is copied into dst on the host threads as soon as it lands while the next
+// ones download (12 MiB into a fresh bytes object 0.73 -> 0.38 ms); above, one copy after the download
+// is the faster (64 MiB: 3.3 ms against 5.0 ms in pieces, whose first touches of dst's pages collide with
+// the downloads).
+cudaError_t download_host(Session* s, uint8_t* dst) {
+  cudaError_t e = cudaSuccess;
+  if (s->len < (3u << 20) || host_is_pinned(dst)) {
+    e = cudaMemcpyAsync(dst, s->buf, s->len, cudaMemcpyDeviceToHost, s->stream);
+    const cudaError_t se = cudaStreamSynchronize(s->stream);
+    return e != cudaSuccess ? e : se;
+  }
+  uint8_t* host = static_cast<uint8_t*>(pinned_pool().get(s->len, &e));
+  if (!host) return e;
+  if (s->len > ((size_t)32 << 20)) {
+    e = cudaMemcpyAsync(host, s->buf, s->len, cudaMemcpyDeviceToHost, s->stream);
+    const cudaError_t se = cudaStreamSynchronize(s->stream);
+    if (e == cudaSuccess) e = se;
+    if (e == cudaSuccess) crb::parallel_memcpy(dst, host, s->len);
+    pinned_pool().put(host);
+    return e;
+  }
+  // (a piece per event, at most kUnifiedChunks)
+  const size_t piece = std::max<size_t>((size_t)1 << 20, round_up((s->len + kUnifiedChunks - 1) / kUnifiedChunks, (size_t)1 << 18));
+  CopyOut copyout;
+  copyout.open(s->device);
+  for (size_t off = 0, k = 0; e == cudaSuccess && off < s->len; off += piece, ++k) {
+    const size_t m = std::min(piece, s->len - off);
+    if (!s->ev_dl[k]) e = cudaEventCreateWithFlags(&s->ev_dl[k], cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(host + off, s->buf + off, m, cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = cudaEventRecord(s->ev_dl[k], s->stream);
+    if (e == cudaSuccess) copyout.push(dst + off, host + off, m, s->ev_dl[k]);
+  }
+  const cudaError_t e0 = copyout.finish();
+  const cudaError_t e1 = cudaStreamSynchronize(s->stream);
+  pinned_pool().put(host);
+  return e != cudaSuccess ? e : (e0 != cudaSuccess ? e0 : e1);
+}
+
+// wait: the source may be released when this returns; without it, once the stream is done.
+int session_load(Session* s, const uint8_t* src, size_t len, bool wait = true) {
   if (len && !src) return -1;
   cudaError_t e = dev_grow(&s->buf, &s->buf_cap, len ? len : 1, false, 0, s->stream);
   if (e != cudaSuccess) return (int)e;
   if (len) {
-    e = upload_host(s->buf, src, len, s->stream);
+    e = upload_host(s, s->buf, src, len, s->stream);
     if (e != cudaSuccess) return (int)e;
   }
-  e = cudaStreamSynchronize(s->stream);
+  if (wait) e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) return (int)e;
   s->len = len;
   ++s->buf_version;
@@ -529,10 +574,11 @@ int apply_one(Session* s, const uint8_t* pat, int pat_len, const uint8_t* rep, i
     p.out = s->alt;
     p.out_cap = s->alt_cap;
     p.epoch = next_epoch(s);
+    if (p.nsub) p.res_mirror = s->res_host;
     e = p.nsub ? crb::launch_replace_super(p, s->stream, nullptr) : crb::launch_replace(p, s->stream, nullptr);
     if (e != cudaSuccess) return (int)e;
     ++s->launches;
-    e = cudaMemcpyAsync(s->res_host, s->res, sizeof(ApplyResult), cudaMemcpyDeviceToHost, s->stream);
+    if (!p.nsub) e = cudaMemcpyAsync(s->res_host, s->res, sizeof(ApplyResult), cudaMemcpyDeviceToHost, s->stream);
     if (e != cudaSuccess) return (int)e;
     e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return (int)e;
@@ -691,6 +737,7 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
         p.presence_shift = s->pres_shift;
       }
     }
+    if (k == nst - 1) p.res_mirror = s->res_host;  // (epochs of earlier launches stay in the block)
     if (tab_of[(size_t)k] >= 0) {
       p.multi = s->mtab + tab_of[(size_t)k];
       e = crb::launch_replace_multi(p, s->stream, nullptr);
@@ -702,8 +749,6 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
   }
   e = cudaMemcpyAsync(s->lens_host, s->lens, ((size_t)nst + 1) * sizeof(unsigned long long),
                       cudaMemcpyDeviceToHost, s->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(s->res_host, s->res, sizeof(ApplyResult), cudaMemcpyDeviceToHost, s->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) return (int)e;
   const ApplyResult r = *s->res_host;
@@ -976,9 +1021,7 @@ CR_EXPORT int cuda_replace_result_into(void* h, uint8_t* dst, size_t cap, size_t
   if (s->len == 0) return 0;
   if (!dst) return -1;
   if (cap < s->len) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaMemcpyAsync(dst, s->buf, s->len, cudaMemcpyDeviceToHost, s->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-  return (int)e;
+  return (int)download_host(s, dst);
 }
 
 CR_EXPORT int cuda_replace_length(void* h, size_t* len) {
@@ -1045,6 +1088,7 @@ CR_EXPORT int cuda_replace_apply_device_async(void* h, const uint8_t* d_in, size
   p.agg = s->agg;
   p.res = s->res;
   p.epoch = next_epoch(s);
+  if (p.nsub) p.res_mirror = s->res_host;
   if (st != s->stream) {
     // ensure_scratch and next_epoch clear look-back scratch on the session stream: the kernel
     // on the caller's stream must not start before those clears have landed.
@@ -1064,6 +1108,7 @@ CR_EXPORT int cuda_replace_apply_device_async(void* h, const uint8_t* d_in, size
   s->async_stream = st;
   s->async_epoch = p.epoch;
   s->async_copy = false;
+  s->async_mirror = p.nsub != 0u;
   s->q_kind = 0;
   return 0;
 }
@@ -1079,7 +1124,7 @@ CR_EXPORT int cuda_replace_device_result(void* h, size_t* out_len, unsigned long
     if (kept) *kept = 0;
     return 0;
   }
-  e = cudaMemcpy(s->res_host, s->res, sizeof(ApplyResult), cudaMemcpyDeviceToHost);
+  if (!s->async_mirror) e = cudaMemcpy(s->res_host, s->res, sizeof(ApplyResult), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return (int)e;
   const ApplyResult r = *s->res_host;
   if (r.error_epoch == s->async_epoch || r.overflow_epoch == s->async_epoch) return kErrUnknown;
@@ -1238,12 +1283,10 @@ int unified_chunked(Session* s, const uint8_t* src, size_t n, const uint8_t* pat
     p.tile_last = s->tile_last;
     p.rec = s->rec;
     p.epoch = next_epoch(s);
+    p.res_mirror = s->res_host;
     e = cudaStreamWaitEvent(s->stream, s->ev_up[k], 0);
     if (e == cudaSuccess) e = crb::launch_replace_super(p, s->stream, nullptr);
-    if (e == cudaSuccess) {
-      ++s->launches;
-      e = cudaMemcpyAsync(s->res_host, s->res, sizeof(ApplyResult), cudaMemcpyDeviceToHost, s->stream);
-    }
+    if (e == cudaSuccess) ++s->launches;
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) {
       rc = (int)e;
@@ -1325,7 +1368,7 @@ CR_EXPORT int cuda_replace_unified(const uint8_t* src, size_t src_len, const uin
     }
     rc = 0;
   }
-  rc = session_load(s, src, src_len);
+  rc = session_load(s, src, src_len, false);  // (the apply or the download below waits for the stream)
   if (rc == 0) rc = apply_one(s, pat, pat_len, rep, rep_len, 0, nullptr, nullptr);
   if (rc == 0) rc = result_to_pinned(s, out_host, out_len);
   if (rc == 0) {
@@ -1375,37 +1418,17 @@ CR_EXPORT int cuda_replace_unified_into(const uint8_t* src, size_t src_len, cons
     }
     rc = 0;
   }
-  rc = session_load(s, src, src_len);
+  rc = session_load(s, src, src_len, false);  // (the apply or the download below waits for the stream)
   if (rc == 0) rc = apply_one(s, pat, pat_len, rep, rep_len, 0, nullptr, nullptr);
   bool too_small = false;
   if (rc == 0) {
     *out_len = s->len;
     if (s->len > dst_cap) {
       too_small = true;
+      cudaStreamSynchronize(s->stream);  // (no apply ran when n < pat_len: src may still be read)
       rc = (int)cudaErrorInvalidValue;  // *out_len tells the length needed
-    } else if (s->len >= ((size_t)32 << 20)) {
-      // downloaded in up to kUnifiedChunks pieces into a pooled page-locked block, each piece
-      // copied into dst as soon as it lands while the next ones download
-      uint8_t* host = static_cast<uint8_t*>(pinned_pool().get(s->len, &e));
-      const size_t piece = round_up((s->len + kUnifiedChunks - 1) / kUnifiedChunks, (size_t)1 << 20);
-      CopyOut copyout;
-      if (host) copyout.open(s->device);
-      for (size_t off = 0, k = 0; host && e == cudaSuccess && off < s->len; off += piece, ++k) {
-        const size_t m = std::min(piece, s->len - off);
-        if (!s->ev_dl[k]) e = cudaEventCreateWithFlags(&s->ev_dl[k], cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(host + off, s->buf + off, m, cudaMemcpyDeviceToHost, s->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(s->ev_dl[k], s->stream);
-        if (e == cudaSuccess) copyout.push(dst + off, host + off, m, s->ev_dl[k]);
-      }
-      const cudaError_t e0 = copyout.finish();
-      const cudaError_t e1 = cudaStreamSynchronize(s->stream);
-      if (e == cudaSuccess) e = e0 != cudaSuccess ? e0 : e1;
-      if (host) pinned_pool().put(host);
-      rc = (int)e;
     } else if (s->len) {
-      e = cudaMemcpyAsync(dst, s->buf, s->len, cudaMemcpyDeviceToHost, s->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-      rc = (int)e;
+      rc = (int)download_host(s, dst);
     }
   }
   if (rc == 0 || too_small) {

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <chrono>
 #include <cstddef>
 #include <cstdint>
 #include <condition_variable>
@@ -93,39 +95,44 @@ class PinnedPool {
 // The process-wide pool (never destroyed: CUDA may be torn down first at exit).
 PinnedPool& host_pinned_pool();
 
-// A few persistent host threads for large memcpys (pageable <-> page-locked staging, result
-// copies): spawning threads per copy would cost more than the copy of a 32 MiB chunk.
+// A few persistent host threads for memcpys from 1 MiB (pageable <-> page-locked staging, result
+// copies): spawning threads per copy would cost more than the copy of a staging piece. The parts are
+// taken one by one, by the calling thread too, and a worker looks out for the next copy for a moment
+// before it sleeps, so the pieces of a pipelined transfer follow each other without a wake-up each.
 class CopyWorkers {
  public:
+  static constexpr size_t kMin = 1u << 20, kPart = 256u << 10;
   static CopyWorkers& get() {
     static CopyWorkers* w = new CopyWorkers();  // never destroyed (threads parked at exit)
     return *w;
   }
   // dst[0, n) = src[0, n), split across the workers and the calling thread
   void copy(void* dst, const void* src, size_t n) {
-    const size_t kMin = 8u << 20;
-    const unsigned parts = nthreads_ + 1;
     if (n < kMin || nthreads_ == 0) {
       memcpy(dst, src, n);
       return;
     }
-    const size_t part = pool_round_up((n + parts - 1) / parts, 4096);
     std::unique_lock<std::mutex> lk(mu_);
-    caller_.wait(lk, [&] { return !busy_; });  // one parallel copy at a time
+    if (busy_) {  // one parallel copy at a time; a small one is quicker by itself than in the queue
+      if (n < 8 * kMin) {
+        lk.unlock();
+        memcpy(dst, src, n);
+        return;
+      }
+      caller_.wait(lk, [&] { return !busy_; });
+    }
     busy_ = true;
     dst_ = static_cast<char*>(dst);
     src_ = static_cast<const char*>(src);
     n_ = n;
-    part_ = part;
-    next_ = 1;  // part 0 is the caller's
-    pending_ = 0;
-    for (unsigned i = 1; i < parts; ++i)
-      if (part * i < n) ++pending_;
-    ++gen_;
-    work_.notify_all();
-    lk.unlock();
-    memcpy(dst, src, part < n ? part : n);
-    lk.lock();
+    const size_t most = n / kPart;
+    parts_ = most < nthreads_ + 1u ? most : nthreads_ + 1u;
+    part_ = pool_round_up((n + parts_ - 1) / parts_, 4096);
+    next_ = 0;
+    pending_ = parts_;
+    gen_.store(gen_.load(std::memory_order_relaxed) + 1, std::memory_order_release);
+    if (asleep_) work_.notify_all();
+    take_parts(lk);
     done_.wait(lk, [&] { return pending_ == 0; });
     busy_ = false;
     caller_.notify_one();
@@ -137,30 +144,40 @@ class CopyWorkers {
     nthreads_ = hw > 1 ? (hw - 1 < 15u ? hw - 1 : 15u) : 0u;
     for (unsigned i = 0; i < nthreads_; ++i) std::thread([this] { loop(); }).detach();
   }
-  void loop() {
-    unsigned long long seen = 0;
-    std::unique_lock<std::mutex> lk(mu_);
-    for (;;) {
-      work_.wait(lk, [&] { return gen_ != seen && busy_ && next_ * part_ < n_; });
-      const size_t i = next_++;
-      if (next_ * part_ >= n_ || next_ > nthreads_) seen = gen_;
+  // parts of the current copy until none is left (lk held on entry and exit, not while copying)
+  void take_parts(std::unique_lock<std::mutex>& lk) {
+    while (next_ < parts_) {
+      const size_t a = part_ * next_++;
       char* d = dst_;
-      const char* s = src_;
-      const size_t a = i * part_, len = part_ < n_ - a ? part_ : n_ - a;
+      const char* f = src_;
+      const size_t len = a < n_ ? (part_ < n_ - a ? part_ : n_ - a) : 0;
       lk.unlock();
-      memcpy(d + a, s + a, len);
+      if (len) memcpy(d + a, f + a, len);
       lk.lock();
       if (--pending_ == 0) done_.notify_all();
     }
   }
+  void loop() {
+    unsigned long long seen = 0;
+    for (;;) {
+      const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(60);
+      while (gen_.load(std::memory_order_acquire) == seen && std::chrono::steady_clock::now() < until) std::this_thread::yield();
+      std::unique_lock<std::mutex> lk(mu_);
+      ++asleep_;
+      work_.wait(lk, [&] { return gen_.load(std::memory_order_relaxed) != seen; });
+      --asleep_;
+      seen = gen_.load(std::memory_order_relaxed);
+      take_parts(lk);
+    }
+  }
   std::mutex mu_;
   std::condition_variable work_, done_, caller_;
-  unsigned nthreads_ = 0;
+  unsigned nthreads_ = 0, asleep_ = 0;
   bool busy_ = false;
   char* dst_ = nullptr;
   const char* src_ = nullptr;
-  size_t n_ = 0, part_ = 0, next_ = 0, pending_ = 0;
-  unsigned long long gen_ = 0;
+  size_t n_ = 0, part_ = 0, parts_ = 0, next_ = 0, pending_ = 0;
+  std::atomic<unsigned long long> gen_{0};
 };
 
 // memcpy split over the copy workers when it is large.
@@ -307,6 +324,8 @@ class HostArena {
 void host_arena_register(HostArena* a);
 // The owner closes its area: freed now, or when its last block is released.
 void host_arena_close(HostArena* a);
+// Give the idle device blocks of finished streams back to the driver (stream.cu).
+void dev_blocks_trim();
 // Release a block handed to a caller: into its host area, else into the pool.
 void host_free(void* p);
 

@@ -25,6 +25,7 @@
 #include "replace_kernels.h"
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstring>
 #include <mutex>
@@ -2346,6 +2347,21 @@ __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32
   return true;
 }
 
+// The launch's results to the host's page-locked copy, by the thread that knows every CTA has written
+// its own (the caller then only waits for the stream: no copy to enqueue and wait for).
+__device__ __forceinline__ void mirror_result(const ReplaceParams& p) {
+  if (!p.res_mirror) return;
+  __threadfence();
+  const volatile ApplyResult* r = p.res;
+  volatile ApplyResult* m = p.res_mirror;
+  m->out_len = r->out_len;
+  m->kept = r->kept;
+  m->last_kept = r->last_kept;
+  m->error_epoch = r->error_epoch;
+  m->overflow_epoch = r->overflow_epoch;
+  m->last_tagged = r->last_tagged;
+}
+
 // Input length, output range and super-tile count of the job described by p.
 struct JobDims {
   unsigned long long n_all, n, n16;
@@ -2411,6 +2427,7 @@ __device__ __forceinline__ uint32_t seg_claim(const SegLaunch& sl, ReplaceParams
     sj.rep_ext = Q.rep;
     sj.multi = nullptr;
     sj.presence = nullptr;
+    sj.res_mirror = nullptr;
   }
   return g - base;
 }
@@ -3610,6 +3627,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     if (d == gridDim.x - 1) {
       atomicExch(sched, 0u);
       atomicExch(sched + 1, 0u);
+      if (!SEG) mirror_result(p);
       __threadfence();
     }
   }
@@ -4198,7 +4216,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       marks += t == kNone ? 1u : 0u;
       ++issued;
     }
-    while (MODE == kModeSmall && ok && done + marks < issued) finish();
+    while (ok && done + marks < issued) finish();
     // after a wait that gave up: the loads in flight end before this CTA does
     for (uint32_t j = done; !ok && j < issued; ++j) (void)wait_tile(&s_full[j % NS], (j / NS) & 1u);
     if (lane == 0) {
@@ -4207,7 +4225,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       if (d == gridDim.x - 1) {
         atomicExch(&p.res->tile_counter, 0u);
         atomicExch(&p.res->done_ctas, 0u);
-        __threadfence();
+        mirror_result(p);
       }
     }
     return;
@@ -4387,13 +4405,13 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       }
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(&s_ready[slot]);
         if (!fits) atomicExch(&p.res->overflow_epoch, p.epoch);
+        if (MODE == kModeFree) record(t, O, total, last1, c, Kin);
+        mbar_arrive(&s_ready[slot]);
         if (MODE == kModeFree || use_rec) {  // (query_prefix reads these)
           __stcg(&p.incl[t].kept, Kin);
           __stcg(&p.incl[t].carry, cout);
         }
-        if (MODE == kModeFree) record(t, O, total, last1, c, Kin);
       }
       __syncwarp();
     }
@@ -4920,10 +4938,15 @@ struct KernelCache {
 };
 
 int device_sm_count() {
+  static std::atomic<int> counts[64];  // per device; 0: not asked yet
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
+  std::atomic<int>& known = counts[dev & 63];
+  if (dev < 64 && (sms = known.load(std::memory_order_relaxed)) > 0) return sms;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms > 0 ? sms : 1;
+  if (sms < 1) sms = 1;
+  if (dev < 64) known.store(sms, std::memory_order_relaxed);
+  return sms;
 }
 
 template <int MODE>

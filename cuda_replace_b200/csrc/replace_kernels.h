@@ -142,6 +142,9 @@ struct ReplaceParams {
   const uint32_t* presence;
   unsigned int presence_shift;
   unsigned int same;              // every pattern byte is the same
+  // Page-locked host memory that receives the results when the launch ends (region and super-tile
+  // kernel; q_* and the scheduler's words are not written). nullptr: none.
+  ApplyResult* res_mirror;
   uint8_t pat[kInlineMax];
   uint8_t rep[kInlineMax];
 };

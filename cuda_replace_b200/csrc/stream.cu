@@ -27,7 +27,9 @@
 #include <cerrno>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "cuda_replace.h"
@@ -58,6 +60,106 @@ bool is_pinned(const void* p) {
   }
   return a.type == cudaMemoryTypeHost;
 }
+
+// Device blocks of finished streams, kept for the next one: allocating and freeing some thirty of them
+// took 5 ms of every call. At most kMaxIdle bytes are kept, the blocks idle the longest go first; a
+// block is put here only when no stream uses it any more, and all of them go back to the driver when an
+// allocation of this library fails (dev_blocks_trim).
+class DevBlocks {
+ public:
+  cudaError_t get(void** p, size_t n) {
+    n = rup(n ? n : 1, n < (1u << 20) ? 512 : (1u << 20));
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      size_t best = idle_.size();
+      for (size_t i = 0; i < idle_.size(); ++i)
+        if (idle_[i].dev == dev && idle_[i].size >= n && idle_[i].size <= n + n / 4 &&
+            (best == idle_.size() || idle_[i].size < idle_[best].size))
+          best = i;
+      if (best < idle_.size()) {
+        live_[*p = idle_[best].ptr] = idle_[best];
+        idle_bytes_ -= idle_[best].size;
+        idle_.erase(idle_.begin() + (long)best);
+        return cudaSuccess;
+      }
+    }
+    *p = nullptr;
+    e = cudaMalloc(p, n);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      trim();
+      e = cudaMalloc(p, n);
+    }
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> g(mu_);
+    live_[*p] = Block{*p, n, dev};
+    return cudaSuccess;
+  }
+  void put(void* p) {
+    if (!p) return;
+    std::vector<Block> out;
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      auto it = live_.find(p);
+      if (it == live_.end()) return;
+      idle_.push_back(it->second);
+      idle_bytes_ += it->second.size;
+      live_.erase(it);
+      while (idle_bytes_ > kMaxIdle || idle_.size() > kMaxBlocks) {
+        idle_bytes_ -= idle_.front().size;
+        out.push_back(idle_.front());
+        idle_.erase(idle_.begin());
+      }
+    }
+    release(out);
+  }
+  void trim() {
+    std::vector<Block> out;
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      out.swap(idle_);
+      idle_bytes_ = 0;
+    }
+    release(out);
+  }
+
+ private:
+  static constexpr size_t kMaxIdle = 1ull << 30, kMaxBlocks = 256;
+  struct Block {
+    void* ptr;
+    size_t size;
+    int dev;
+  };
+  static void release(const std::vector<Block>& out) {
+    if (out.empty()) return;
+    int cur = 0;
+    cudaGetDevice(&cur);
+    for (const Block& b : out) {
+      cudaSetDevice(b.dev);
+      cudaFree(b.ptr);
+    }
+    cudaSetDevice(cur);
+  }
+  std::mutex mu_;
+  std::vector<Block> idle_;  // the oldest first
+  std::unordered_map<void*, Block> live_;
+  size_t idle_bytes_ = 0;
+};
+DevBlocks& blocks() {
+  static DevBlocks* b = new DevBlocks();  // never destroyed: CUDA may be torn down first at exit
+  return *b;
+}
+
+}  // namespace
+
+namespace crb {
+void dev_blocks_trim() { blocks().trim(); }
+}  // namespace crb
+
+namespace {
 
 struct Stage {
   ReplaceParams proto;                    // pattern fields for every launch of this stage
@@ -100,11 +202,11 @@ struct Stream {
     if (d2h) cudaStreamSynchronize(d2h);
     for (auto& s : st)
       for (int b = 0; b < 2; ++b)
-        if (s.pend[b]) cudaFree(s.pend[b]);
+        blocks().put(s.pend[b]);
     for (int b = 0; b < 2; ++b) {
-      if (in0[b]) cudaFree(in0[b]);
-      if (x[b]) cudaFree(x[b]);
-      if (out[b]) cudaFree(out[b]);
+      blocks().put(in0[b]);
+      blocks().put(x[b]);
+      blocks().put(out[b]);
       if (hin[b]) crb::host_pinned_pool().put(hin[b]);
       if (ev_h2d[b]) cudaEventDestroy(ev_h2d[b]);
       if (ev_stage0[b]) cudaEventDestroy(ev_stage0[b]);
@@ -112,9 +214,9 @@ struct Stream {
     }
     for (void* q : {(void*)lens, (void*)outlen, (void*)carry, (void*)status, (void*)incl, (void*)tile_last,
                     (void*)rec, (void*)agg, (void*)res})
-      if (q) cudaFree(q);
-    if (res_host) cudaFreeHost(res_host);
-    if (meta_host) cudaFreeHost(meta_host);
+      blocks().put(q);
+    crb::host_pinned_pool().put(res_host);
+    crb::host_pinned_pool().put(meta_host);
     if (comp) cudaStreamDestroy(comp);
     if (h2d) cudaStreamDestroy(h2d);
     if (d2h) cudaStreamDestroy(d2h);
@@ -132,12 +234,21 @@ struct Stream {
     return std::max<size_t>(16, est >= (double)worst ? worst : (size_t)est);
   }
 
-  static cudaError_t regrow(uint8_t** p, size_t* cap, size_t want) {
+  // Hand a block back while the stream goes on: whatever still uses it ends first.
+  void give_back(void* q) {
+    if (!q) return;
+    cudaStreamSynchronize(comp);
+    cudaStreamSynchronize(h2d);
+    cudaStreamSynchronize(d2h);
+    blocks().put(q);
+  }
+
+  cudaError_t regrow(uint8_t** p, size_t* cap, size_t want) {
     if (want <= *cap && *p) return cudaSuccess;
-    if (*p) cudaFree(*p);
+    give_back(*p);
     *p = nullptr;
     const size_t c = rup(want, 1u << 20);
-    const cudaError_t e = cudaMalloc(p, c + 64);  // + 64: reads rounded up to 16 bytes stay inside
+    const cudaError_t e = blocks().get((void**)p, c + 64);  // + 64: reads rounded up to 16 bytes stay inside
     if (e == cudaSuccess) *cap = c;
     return e;
   }
@@ -174,25 +285,25 @@ struct Stream {
     }
     if (need_tiles > tiles_cap) {
       for (void* q : {(void*)status, (void*)incl, (void*)tile_last, (void*)rec})
-        if (q) cudaFree(q);
+        give_back(q);
       status = nullptr;
       incl = nullptr;
       tile_last = nullptr;
       rec = nullptr;
       const size_t cap = need_tiles + 64;
-      e = cudaMalloc(&status, cap * sizeof(uint32_t));
-      if (e == cudaSuccess) e = cudaMalloc(&incl, cap * sizeof(TileIncl));
-      if (e == cudaSuccess) e = cudaMalloc(&tile_last, cap * sizeof(long long));
-      if (e == cudaSuccess) e = cudaMalloc(&rec, cap * 2 * sizeof(unsigned long long));
+      e = blocks().get((void**)&status, cap * sizeof(uint32_t));
+      if (e == cudaSuccess) e = blocks().get((void**)&incl, cap * sizeof(TileIncl));
+      if (e == cudaSuccess) e = blocks().get((void**)&tile_last, cap * sizeof(long long));
+      if (e == cudaSuccess) e = blocks().get((void**)&rec, cap * 2 * sizeof(unsigned long long));
       if (e == cudaSuccess) e = cudaMemsetAsync(status, 0, cap * sizeof(uint32_t), comp);
       if (e == cudaSuccess) e = cudaMemsetAsync(rec, 0, cap * 2 * sizeof(unsigned long long), comp);
       if (e != cudaSuccess) return e;
       tiles_cap = cap;
     }
     if (need_agg > agg_cap) {
-      if (agg) cudaFree(agg);
+      give_back(agg);
       agg = nullptr;
-      e = cudaMalloc(&agg, (need_agg + 1024) * sizeof(unsigned long long));
+      e = blocks().get((void**)&agg, (need_agg + 1024) * sizeof(unsigned long long));
       if (e != cudaSuccess) return e;
       agg_cap = need_agg + 1024;
     }
@@ -320,22 +431,23 @@ int stream_setup(Stream& S, const uint8_t** pats, const int* pat_lens, const uin
   }
   S.in0_cap = S.st[0].P + S.chunk;
   for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
-    e = cudaMalloc(&S.in0[b], rup(S.in0_cap, 1u << 20) + 64);
+    e = blocks().get((void**)&S.in0[b], rup(S.in0_cap, 1u << 20) + 64);
     if (e == cudaSuccess && staging) S.hin[b] = static_cast<uint8_t*>(pool.get(S.chunk, &e));
   }
   for (int k = 0; k < count && e == cudaSuccess; ++k)
     for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
-      e = cudaMalloc(&S.st[(size_t)k].pend[b], 256);
+      e = blocks().get((void**)&S.st[(size_t)k].pend[b], 256);
       if (e == cudaSuccess) e = cudaMemsetAsync(S.st[(size_t)k].pend[b], 0, 256, S.comp);
     }
-  if (e == cudaSuccess) e = cudaMalloc(&S.lens, (size_t)(count + 1) * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = blocks().get((void**)&S.lens, (size_t)(count + 1) * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMemsetAsync(S.lens, 0, (size_t)(count + 1) * sizeof(unsigned long long), S.comp);
-  if (e == cudaSuccess) e = cudaMalloc(&S.outlen, 2 * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMalloc(&S.carry, (size_t)2 * count * sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMalloc(&S.res, sizeof(ApplyResult));
+  if (e == cudaSuccess) e = blocks().get((void**)&S.outlen, 2 * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = blocks().get((void**)&S.carry, (size_t)2 * count * sizeof(unsigned int));
+  if (e == cudaSuccess) e = blocks().get((void**)&S.res, sizeof(ApplyResult));
   if (e == cudaSuccess) e = cudaMemsetAsync(S.res, 0, sizeof(ApplyResult), S.comp);
-  if (e == cudaSuccess) e = cudaMallocHost(&S.res_host, sizeof(ApplyResult));
-  if (e == cudaSuccess) e = cudaMallocHost(&S.meta_host, (size_t)(count + 2) * sizeof(unsigned long long));
+  if (e == cudaSuccess) S.res_host = static_cast<ApplyResult*>(pool.get(sizeof(ApplyResult), &e));
+  if (e == cudaSuccess)
+    S.meta_host = static_cast<unsigned long long*>(pool.get((size_t)(count + 2) * sizeof(unsigned long long), &e));
   if (e == cudaSuccess) e = S.size_buffers();
   if (e != cudaSuccess) return (int)e;
   // every stage starts with its P held bytes covered: at the first chunk they do not exist

@@ -117,6 +117,15 @@ def _advise_huge(addr: int, n: int) -> None:
         _madvise(c_void_p(a), c_size_t(e - a), C.c_int(_MADV_HUGEPAGE))
 
 
+def _need_bytes(pat, rep) -> None:
+    if not isinstance(pat, bytes) or not isinstance(rep, bytes):
+        raise TypeError("pattern and replacement must be bytes")
+
+
+class _Outgrown(Exception):
+    """The session's buffer grew (in another thread) between its length and its download."""
+
+
 def _src_pointer(src):
     """(keep-alive object, pointer, length) of a bytes-like input without copying bytes objects."""
     if isinstance(src, bytes):
@@ -232,6 +241,25 @@ class CudaReplaceLib:
               [c_uint8_p, c_size_t, c_uint8_pp, c_int_p, c_uint8_pp, c_int_p, C.c_int, c_size_t,
                C.POINTER(c_uint8_p), c_size_t_p], C.c_int, optional=True)
 
+        # The per-call entry points once more with the pattern and the replacement as char pointers:
+        # ctypes passes a bytes object's own memory, with no copy and no cast (which cost more than the
+        # call itself on small buffers). c_char_p refuses what create_string_buffer refused.
+        s, i = C.c_char_p, C.c_int
+        self._apply = self._again("cuda_replace_apply", [c_void_p, s, i, s, i, c_size_t_p])
+        self._unified = self._again("cuda_replace_unified",
+                                    [c_uint8_p, c_size_t, s, i, s, i, C.POINTER(c_uint8_p), c_size_t_p])
+        self._async = self._again("cuda_replace_apply_device_async",
+                                  [c_void_p, c_void_p, c_size_t, s, i, s, i, c_void_p, c_size_t, c_void_p])
+
+    def _again(self, name: str, argtypes):
+        try:
+            fn = self.lib[name]  # (indexing makes a new function object)
+        except AttributeError:
+            return None
+        fn.argtypes = argtypes
+        fn.restype = C.c_int
+        return fn
+
     def version(self) -> str:
         return self.lib.cuda_replace_version().decode()
 
@@ -240,10 +268,10 @@ class CudaReplaceLib:
         returned bytes object (cuda_replace_unified_into): its copy out of page-locked memory
         overlaps the transfers instead of following them."""
         keep, src_p, n = _src_pointer(src)
-        pat_buf = C.create_string_buffer(pat, len(pat) or 1)
-        rep_buf = C.create_string_buffer(rep, len(rep) or 1)
         into = getattr(self.lib, "cuda_replace_unified_into", None)
         if into is not None and pat and n >= _PARALLEL_COPY_MIN:
+            pat_buf = C.create_string_buffer(pat, len(pat) or 1)
+            rep_buf = C.create_string_buffer(rep, len(rep) or 1)
             bound = c_size_t()
             self.lib.cuda_replace_output_bound(c_size_t(n), C.c_int(len(pat)), C.c_int(len(rep)), C.byref(bound))
             if bound.value <= 4 * n + (64 << 20):
@@ -261,11 +289,8 @@ class CudaReplaceLib:
                     del keep
         out_ptr = c_uint8_p()
         out_len = c_size_t()
-        rc = self.lib.cuda_replace_unified(
-            src_p, c_size_t(n),
-            C.cast(pat_buf, c_uint8_p), C.c_int(len(pat)),
-            C.cast(rep_buf, c_uint8_p), C.c_int(len(rep)),
-            C.byref(out_ptr), C.byref(out_len))
+        _need_bytes(pat, rep)
+        rc = self._unified(src_p, n, pat, len(pat), rep, len(rep), C.byref(out_ptr), C.byref(out_len))
         del keep
         if rc != 0:
             raise RuntimeError(f"cuda_replace_unified failed rc={rc}")
@@ -306,11 +331,9 @@ class Session:
             raise RuntimeError(f"cuda_replace_build_index failed rc={rc}")
 
     def apply(self, pat: bytes, rep: bytes) -> int:
-        pb = C.create_string_buffer(pat, len(pat) or 1)
-        rb = C.create_string_buffer(rep, len(rep) or 1)
+        _need_bytes(pat, rep)
         new_len = c_size_t()
-        rc = self.lib.lib.cuda_replace_apply(self.h, C.cast(pb, c_uint8_p), C.c_int(len(pat)),
-                                             C.cast(rb, c_uint8_p), C.c_int(len(rep)), C.byref(new_len))
+        rc = self.lib._apply(self.h, pat, len(pat), rep, len(rep), C.byref(new_len))
         if rc != 0:
             raise RuntimeError(f"cuda_replace_apply failed rc={rc}")
         return int(new_len.value)
@@ -363,6 +386,20 @@ class Session:
         return int(kept.value), int(last.value)
 
     def result(self) -> bytes:
+        n = self.length()
+        if n >= _PARALLEL_COPY_MIN:  # straight into the bytes object, the copies behind the download
+            def fill(addr, cap):
+                got = c_size_t()
+                rc = self.lib.lib.cuda_replace_result_into(self.h, c_void_p(addr), c_size_t(cap), C.byref(got))
+                if rc == 1 and got.value > cap:
+                    raise _Outgrown
+                if rc != 0:
+                    raise RuntimeError(f"cuda_replace_result failed rc={rc}")
+                return got.value
+            try:
+                return _bytes_filled(n, fill)
+            except _Outgrown:
+                pass
         out_ptr = c_uint8_p()
         out_len = c_size_t()
         rc = self.lib.lib.cuda_replace_result(self.h, C.byref(out_ptr), C.byref(out_len))
@@ -390,11 +427,8 @@ class Session:
     def apply_device_async(self, d_in: int, n: int, pat: bytes, rep: bytes, d_out: int, out_cap: int,
                            stream: int = 0) -> None:
         """Enqueue a replace of device memory d_in[0, n) into d_out on a CUDA stream handle."""
-        pb = C.create_string_buffer(pat, len(pat) or 1)
-        rb = C.create_string_buffer(rep, len(rep) or 1)
-        rc = self.lib.lib.cuda_replace_apply_device_async(
-            self.h, c_void_p(d_in), c_size_t(n), C.cast(pb, c_uint8_p), C.c_int(len(pat)),
-            C.cast(rb, c_uint8_p), C.c_int(len(rep)), c_void_p(d_out), c_size_t(out_cap), c_void_p(stream))
+        _need_bytes(pat, rep)
+        rc = self.lib._async(self.h, d_in, n, pat, len(pat), rep, len(rep), d_out, out_cap, stream)
         if rc != 0:
             raise RuntimeError(f"cuda_replace_apply_device_async failed rc={rc}")
 
