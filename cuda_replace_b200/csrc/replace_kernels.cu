@@ -2056,40 +2056,29 @@ __device__ __forceinline__ void literal_chunks(uint8_t* dst, const uint8_t* src,
 // One warp's output when it is a copy of its input: wtot bytes from tile byte srcw, written at
 // out[g0, g0 + wtot) with aligned 16-byte stores (funnel-shifted from shared memory); the
 // partial 16-byte chunks at both ends one byte per lane (the neighbouring regions own their
-// other bytes).
+// other bytes). Positions are 32-bit, relative to g0: a region's copy is 50 instructions of loop and
+// was 100 of 64-bit address arithmetic around it.
 __device__ __forceinline__ void warp_emit_literal(uint8_t* out, const uint8_t* tb, unsigned long long g0,
                                                   uint32_t wtot, uint32_t srcw) {
   const uint32_t lane = threadIdx.x & 31u;
-  const unsigned long long ga = g0 & ~15ull;
-  const unsigned long long gend = g0 + wtot;
-  const uint32_t c0 = (uint32_t)((g0 - ga + 15ull) >> 4);  // first whole 16-byte chunk
-  const uint32_t c1 = (uint32_t)((gend - ga) >> 4);        // end of the whole chunks
-  const uint32_t off0 = srcw + (uint32_t)(ga + ((unsigned long long)c0 << 4) - g0);
-  const uint32_t r = off0 & 15u, q = r >> 2, sh = (r & 3u) * 8u;
-  {
-    const uint32_t c = c0 + lane;
-    if (c < c1) {
-      const uint32_t k = (c1 - c + 31u) >> 5;  // this lane's chunks c, c + 32, ...
-      const uint8_t* src = tb + (off0 - r + ((c - c0) << 4));
-      uint8_t* dst = out + ga + ((unsigned long long)c << 4);
-      switch (q) {  // the same in every lane
-        case 0: literal_chunks<0>(dst, src, k, sh); break;
-        case 1: literal_chunks<1>(dst, src, k, sh); break;
-        case 2: literal_chunks<2>(dst, src, k, sh); break;
-        default: literal_chunks<3>(dst, src, k, sh); break;
-      }
+  uint8_t* const og = out + g0;
+  const uint32_t head = (0u - (uint32_t)g0) & 15u;              // bytes before the first whole chunk
+  const uint32_t nc = wtot > head ? (wtot - head) >> 4 : 0u;    // whole chunks
+  if (lane < nc) {
+    const uint32_t k = (nc - lane + 31u) >> 5;  // this lane's chunks lane, lane + 32, ...
+    const uint32_t off = srcw + head, r = off & 15u, sh = (r & 3u) * 8u;
+    const uint8_t* src = tb + (off - r + 16u * lane);
+    uint8_t* dst = og + (head + 16u * lane);
+    switch (r >> 2) {  // the same in every lane
+      case 0: literal_chunks<0>(dst, src, k, sh); break;
+      case 1: literal_chunks<1>(dst, src, k, sh); break;
+      case 2: literal_chunks<2>(dst, src, k, sh); break;
+      default: literal_chunks<3>(dst, src, k, sh); break;
     }
   }
-  unsigned long long b;
-  bool ok;
-  if (c0 < c1) {
-    b = lane < 16u ? g0 + lane : ga + ((unsigned long long)c1 << 4) + (lane - 16u);
-    ok = lane < 16u ? (b < ga + ((unsigned long long)c0 << 4)) : (b < gend);
-  } else {
-    b = g0 + lane;
-    ok = b < gend;
-  }
-  if (ok) out[b] = tb[srcw + (uint32_t)(b - g0)];
+  // head bytes on lanes 0-15, tail bytes on lanes 16-31; with no whole chunk, fewer than 32 bytes in all
+  const uint32_t b = (lane < 16u || nc == 0u) ? lane : head + 16u * nc + (lane - 16u);
+  if (b < ((lane < 16u && nc != 0u) ? head : wtot)) og[b] = tb[srcw + b];
 }
 
 // x mod R for x < 2^26 and 1 <= R <= 64, with rmag = ceil(2^32 / R) (0 for R = 1): the
@@ -2272,6 +2261,39 @@ __device__ __forceinline__ void warp_copy_staged(uint8_t* out, const uint8_t* st
     ok = b < gend;
   }
   if (ok) out[b] = stg[(uint32_t)(b - ga)];
+}
+
+// Output of a warp region as pieces: literal runs between replacements, one after the other by the whole
+// warp. kept: the lane's kept starts in its segment of the region at tb + qs; literal bytes [x0, end)
+// (relative to tb); out[g0, g0 + total). Returns false when the lengths do not add up (nothing is
+// written past the slot).
+__device__ __noinline__ bool warp_emit_pieces(uint8_t* out, const uint8_t* tb, uint64_t kept, uint32_t qs, uint32_t x0,
+                                              uint32_t end, unsigned long long g0, uint32_t total, uint32_t L, uint32_t R,
+                                              const uint8_t* rs) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t pos = x0, o = 0;
+  uint32_t sm = __ballot_sync(0xffffffffu, kept != 0ull);
+  uint64_t m = 0;
+  uint32_t s = 0;
+#pragma unroll 1
+  for (;;) {  // (one copy of the literal loops for the runs before matches and for the last)
+    if (!m && sm) {
+      s = (uint32_t)__ffs(sm) - 1u;
+      sm &= sm - 1u;
+      m = (uint64_t)__shfl_sync(0xffffffffu, (unsigned long long)kept, s);
+    }
+    const bool match = m != 0ull;
+    const uint32_t at = match ? qs + 64u * s + (uint32_t)__ffsll((long long)m) - 1u : end;
+    m &= m - 1ull;
+    const uint32_t l = at > pos ? at - pos : 0u;
+    if (match ? o + l + R > total : o + l != total) return false;
+    if (l) warp_emit_literal(out, tb, g0 + o, l, pos);
+    if (!match) return true;
+    o += l;
+    for (uint32_t q = lane; q < R; q += 32u) out[g0 + o + q] = rs[q];
+    o += R;
+    pos = at + L;
+  }
 }
 
 // Output of a warp region with few matches (at most kGatherMax, output at most kGatherBytes; R <= 64):
@@ -2817,7 +2839,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     ring.issue(p, smem, lay, s_bar, S, n16, want_a, n, nsub);
   };
 
-  // Output of one warp region with at most 16 matches (kFreeLike): literal runs between its
+  // Output of one warp region with at most 16 matches (kModeMulti): literal runs between its
   // replacements. Each run is copied by the whole warp (aligned 16-byte stores, like a
   // copy-only region), each replacement by as many lanes as it has bytes; no staging of the
   // whole output. kept: this thread's kept starts in its 64-byte segment of the sub-tile at tb
@@ -2829,14 +2851,13 @@ __global__ void __launch_bounds__(kThreads, 3)
                          unsigned long long g0, uint32_t wtot) -> bool {
     const uint32_t cnt = (uint32_t)__popcll(kept);
     const uint32_t M = __reduce_add_sync(0xffffffffu, cnt);
-    if (M > (MODE == kModeMulti ? 16u : kPieceMax)) return false;
+    if (M > 16u) return false;
     uint32_t* desc = reinterpret_cast<uint32_t*>(ob) + (size_t)warp * lay.wstage_words;
     const uint32_t mb = warp_incl_scan(cnt, OpSum()) - cnt;  // this lane's first match index
     uint32_t i = 0;
     for (uint64_t km = kept; km; km &= km - 1ull, ++i) {
       const uint32_t b = (uint32_t)(__ffsll((long long)km) - 1);
-      int k = 0;  // the match's pair (kModeMulti)
-      if constexpr (MODE == kModeMulti) k = multi_identify(MT, tb + sb + b, n_all - (gseg + b));
+      const int k = multi_identify(MT, tb + sb + b, n_all - (gseg + b));  // the match's pair
       desc[2 * (mb + i)] = lane * 64u + b;  // start within the region
       desc[2 * (mb + i) + 1] = (uint32_t)(k < 0 ? 0 : k);
     }
@@ -2847,14 +2868,14 @@ __global__ void __launch_bounds__(kThreads, 3)
       uint32_t st0 = x0r;
       if (lane > 0) {
         const uint32_t pk = desc[2 * (lane - 1) + 1];
-        st0 = desc[2 * (lane - 1)] + (MODE == kModeMulti ? (uint32_t)MT.L[pk] : L);
+        st0 = desc[2 * (lane - 1)] + (uint32_t)MT.L[pk];
       }
       const uint32_t en = lane < M ? desc[2 * lane] : vend;
       lstart = st0;
       llen = en > st0 ? en - st0 : 0u;
       if (lane < M) {
         pid = desc[2 * lane + 1];
-        rlen = MODE == kModeMulti ? (uint32_t)MT.R[pid] : R;
+        rlen = (uint32_t)MT.R[pid];
       }
     }
     const uint32_t piece = llen + rlen;
@@ -2872,7 +2893,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       if (jp < M) {
         const uint32_t rl = __shfl_sync(0xffffffffu, rlen, jp);
         const uint32_t pk = __shfl_sync(0xffffffffu, pid, jp);
-        const uint8_t* rb = MODE == kModeMulti ? MT.rep[pk] : rs;  // rs: the replacement (and more)
+        const uint8_t* rb = MT.rep[pk];
         for (uint32_t q = lane; q < rl; q += 32u) p.out[g0 + po + ll + q] = rb[q];
       }
     }
@@ -2903,9 +2924,13 @@ __global__ void __launch_bounds__(kThreads, 3)
       return;
     }
     const uint32_t vend = __reduce_add_sync(0xffffffffu, V);
-    if (emit_pieces(tb, kept, gseg, x0r, vend, g0, wtot)) return;
-    if (R <= 64u && wtot <= kGatherBytes && __reduce_add_sync(0xffffffffu, (uint32_t)__popcll(kept)) <= kGatherMax) {
-      const uint32_t q0 = warp * 2048u;
+    const uint32_t M = __reduce_add_sync(0xffffffffu, (uint32_t)__popcll(kept)), q0 = warp * 2048u;
+    if (M <= kPieceMax) {
+      if (!warp_emit_pieces(p.out, tb, kept, q0, q0 + x0r, q0 + vend, g0, wtot, L, R, rs) && lane == 0)
+        set_error(p);  // (the arithmetic rules it out)
+      return;
+    }
+    if (R <= 64u && wtot <= kGatherBytes && M <= kGatherMax) {
       if (!emit_gather(p.out, tb, reinterpret_cast<uint32_t*>(ob) + (size_t)warp * lay.wstage_words, kept, q0, q0 + x0r,
                        q0 + vend, g0, wtot, L, R, rs) &&
           lane == 0)
@@ -4555,36 +4580,6 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     }
   };
 
-  // A region as pieces: literal runs between replacements, one after the other by the whole warp.
-  // tb: the super-tile; x0, end: the region's literal range (relative to it); out[g0, g0 + total).
-  auto emit_pieces = [&](const uint8_t* tb, uint64_t kept, uint32_t x0, uint32_t end, unsigned long long g0, uint32_t total) {
-    uint32_t pos = x0, o = 0;
-#pragma unroll 1
-    for (uint32_t sm = __ballot_sync(0xffffffffu, kept != 0ull); sm; sm &= sm - 1u) {
-      const uint32_t s = (uint32_t)__ffs(sm) - 1u;
-#pragma unroll 1
-      for (uint64_t m = (uint64_t)__shfl_sync(0xffffffffu, (unsigned long long)kept, s); m; m &= m - 1ull) {
-        const uint32_t at = qs + 64u * s + (uint32_t)__ffsll((long long)m) - 1u;
-        const uint32_t l = at > pos ? at - pos : 0u;
-        if (o + l + R > total) {  // (ruled out by the arithmetic; nothing is written past the slot)
-          if (lane == 0) set_error(p);
-          return;
-        }
-        if (l) warp_emit_literal(p.out, tb, g0 + o, l, pos);
-        o += l;
-        for (uint32_t q = lane; q < R; q += 32u) p.out[g0 + o + q] = rs[q];
-        o += R;
-        pos = at + L;
-      }
-    }
-    const uint32_t l = end > pos ? end - pos : 0u;
-    if (o + l != total) {
-      if (lane == 0) set_error(p);
-    } else if (l) {
-      warp_emit_literal(p.out, tb, g0 + o, l, pos);
-    }
-  };
-
   // A region that mixes literal bytes and replacements, scattered into the warp's staging area and
   // copied out in rounds: kept starts `kept` of the lane's segment, x_in bytes of it covered by an
   // earlier match, V valid bytes. With exact the output must be `total` bytes; otherwise its length
@@ -4722,7 +4717,8 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
           __syncwarp();
           warp_emit_literal(p.out, tb, g0, e.y, e.z);
         } else if (!cut && (R > 64u || e.w <= kRegionPieces)) {
-          emit_pieces(tb, kept, e.z, qs + vb, g0, e.y);
+          if (!warp_emit_pieces(p.out, tb, kept, qs, e.z, qs + vb, g0, e.y, L, R, rs) && lane == 0)
+            set_error(p);  // (the arithmetic rules it out)
         } else if (!cut && e.w <= kGatherMax && e.y <= kGatherBytes) {
           if (!emit_gather(p.out, tb, reinterpret_cast<uint32_t*>(stg), kept, qs, e.z, qs + vb, g0, e.y, L, R, rs) &&
               lane == 0)
