@@ -3843,6 +3843,25 @@ __device__ __forceinline__ uint64_t walk_kept(uint32_t y, uint64_t mask, uint32_
   return kept;
 }
 
+// Whether a region's candidates (64 per lane) are one run of consecutive positions [*a, *b) (relative to the
+// region): inside a long run, at its ends, or a single rule line. Its greedy has a closed form.
+__device__ __forceinline__ bool single_run(uint64_t mask, uint32_t* a, uint32_t* b) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t prev = __shfl_up_sync(0xffffffffu, (uint32_t)(mask >> 63), 1);
+  if (lane == 0) prev = 0;
+  const uint32_t starts = (uint32_t)__popcll(mask & ~((mask << 1) | prev));
+  if (__reduce_add_sync(0xffffffffu, starts) != 1u) return false;
+  *a = __reduce_min_sync(0xffffffffu, mask ? 64u * lane + (uint32_t)__ffsll((long long)mask) - 1u : ~0u);
+  *b = __reduce_max_sync(0xffffffffu, mask ? 64u * lane + 64u - (uint32_t)__clzll((long long)mask) : 0u);
+  return true;
+}
+// The lane's kept starts of that run when the first is x.
+__device__ __forceinline__ uint64_t run_kept(uint64_t mask, uint32_t x, uint32_t L, uint64_t stride) {
+  const uint32_t off = 64u * (threadIdx.x & 31u);
+  const uint32_t first = off <= x ? x - off : dense_seg_carry(x, off, L);
+  return first < 64u ? (stride << first) & mask : 0ull;
+}
+
 // Bounded wait inside the CTA.
 __device__ __forceinline__ bool pipe_wait(const ReplaceParams& p, uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;
@@ -3937,13 +3956,18 @@ struct RunningSum {
           if (lane == 0) set_error(p);
           return false;
         }
-        __nanosleep(ns);
+        if (ns > 32u) __nanosleep(ns >> 1);  // (the first window was read early: again at once)
         if (ns < 128) ns <<= 1;
       }
       load(p, t);
     }
   }
 };
+
+// Record flags of a super-tile of kModeSmall with L > 4 (second word, beside its carry-out; the first holds its
+// kept count from carry 0): the carry-out is the same for every carry; the kept count too; every position
+// is a candidate.
+constexpr uint32_t kRecSame = 0x100u, kRecFixed = 0x200u, kRecDense = 0x400u;
 
 // Look-back for patterns of 5..64 bytes with a border: super-tile functions are tables over
 // carries in global memory; lane c holds entries c and (NE = 2) c + 32. 32 / NE predecessors per
@@ -4047,6 +4071,110 @@ __device__ __forceinline__ bool lookback_table(const ReplaceParams& p, uint32_t 
   }
 }
 
+// Look-back for patterns of 5..64 bytes with a border: RunningSum with a carry. A super-tile's carry-out is
+// the same for every carry-in (nearly always), or it holds nothing but candidates (inside a long run)
+// and its function has a closed form; then each one's carry-in follows from the last of the first kind before
+// it, and its count is the recorded one, the closed form, or (rarely: the carry reaches a candidate) an
+// entry of its table. With any other super-tile on the way the tables are composed back to the nearest
+// inclusive prefix. 32 MiB of rule lines, L = 40: composing tables alone took 83 us, now 62.
+struct RunningCarry {
+  static constexpr int kPer = 5;
+  unsigned long long sum;  // kept in super-tiles [0, pos)
+  uint32_t pos, carry;     // ... and the carry into pos
+
+  __device__ __forceinline__ void init(uint32_t carry0) {
+    sum = 0;
+    pos = 0;
+    carry = carry0;
+  }
+  __device__ __forceinline__ bool reach(const ReplaceParams& p, uint32_t t, uint32_t L, unsigned long long* K_out,
+                                        uint32_t* c_out, uint32_t carry0) {
+    constexpr uint32_t S = region_tile(kModeSmall);
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned long long tag = (unsigned long long)(p.epoch & 0xFFFFFFu);
+    unsigned long long t0 = 0;
+    uint32_t ns = 32;
+    for (;;) {
+      unsigned long long w0[kPer], w1[kPer];
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const uint32_t j = pos + lane + 32u * (uint32_t)k;
+        w0[k] = w1[k] = 0;
+        if (j < t) rec_load(p.rec, j, &w0[k], &w1[k]);
+      }
+      bool ready = true, same = true, dense = false;
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const uint32_t j = pos + lane + 32u * (uint32_t)k;
+        if (j < t) {
+          ready = ready && (w0[k] >> 40) == tag && (w1[k] >> 40) == tag && ((w0[k] >> 38) & 3ull) != 0ull &&
+                  ((w1[k] >> 38) & 3ull) != 0ull;
+          same = same && (w1[k] & (kRecSame | kRecDense)) != 0ull;
+          dense = dense || (w1[k] & kRecDense) != 0ull;
+        }
+      }
+      if (__all_sync(0xffffffffu, ready)) {
+        if (!__all_sync(0xffffffffu, same)) {
+          unsigned long long K;
+          uint32_t c;
+          if (!(L <= 32u ? lookback_table<1>(p, t, L, &K, &c, carry0) : lookback_table<2>(p, t, L, &K, &c, carry0))) return false;
+          sum = K;
+          carry = c;
+          pos = t;
+        } else {
+          uint32_t part = 0, c0 = carry, at = pos;  // carry c0 into super-tile `at`; all candidates from there on
+          const bool any_dense = __any_sync(0xffffffffu, dense);
+#pragma unroll
+          for (int k = 0; k < kPer; ++k) {
+            const uint32_t row = pos + 32u * (uint32_t)k, j = row + lane;
+            const uint32_t out = (uint32_t)w1[k] & 0xFFu;
+            const uint32_t sm = __ballot_sync(0xffffffffu, j < t && (w1[k] & kRecSame) != 0ull);
+            const uint32_t below = sm & ((1u << lane) - 1u), l = below ? 31u - (uint32_t)__clz((int)below) : 0u;
+            const uint32_t prev = __shfl_sync(0xffffffffu, out, l);
+            if (j < t) {
+              uint32_t c = below ? prev : c0;
+              if (any_dense) c = dense_seg_carry(c, (below ? lane - l - 1u : j - at) * S, L);
+              uint32_t cnt = (uint32_t)rec_data(w0[k]);
+              if (w1[k] & kRecDense) {
+                cnt = (S - c + L - 1u) / L;
+              } else if (c != 0u && !(w1[k] & kRecFixed)) {
+                __threadfence();  // the table was written before the record
+                cnt = (uint32_t)__ldcg(p.agg + (unsigned long long)j * L + c);
+              }
+              part += cnt;
+            }
+            if (sm) {
+              const uint32_t h = 31u - (uint32_t)__clz((int)sm);
+              c0 = __shfl_sync(0xffffffffu, out, h);
+              at = row + h + 1u;
+            }
+          }
+          pos = min(t, pos + 32u * kPer);
+          const uint32_t last = any_dense ? dense_seg_carry(c0, (pos - at) * S, L) : c0;
+          sum += __reduce_add_sync(0xffffffffu, part);
+          carry = last;
+        }
+        if (pos == t) {
+          *K_out = sum;
+          *c_out = carry;
+          return true;
+        }
+      } else {
+        if (aborted(p)) return false;
+        const unsigned long long now = global_ns();
+        if (t0 == 0) {
+          t0 = now;
+        } else if (now - t0 > kSpinLimitNs) {
+          if (lane == 0) set_error(p);
+          return false;
+        }
+        if (ns > 32u) __nanosleep(ns >> 1);
+        if (ns < 128) ns <<= 1;
+      }
+    }
+  }
+};
+
 // Fold of up to 32 regions for patterns of LL <= 4 bytes (one warp): lane r holds region r's function
 // (the identity beyond nreg). A scan over the lanes gives the carry into every region for each
 // carry into the super-tile (wrec) and the super-tile's function (entry `lane`).
@@ -4094,7 +4222,13 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
   __shared__ __align__(8) uint64_t s_full[NS], s_adone[NS], s_folded[NS], s_ready[NS], s_bdone[NS];
   __shared__ uint32_t s_tile[NS];
   __shared__ uint32_t s_wcnt[NS][NR], s_wend[NS][NR];  // kModeFree: kept count, end of the last match
-  __shared__ uint8_t s_kind[NS][NR];  // kModeSmall: 0 no candidate, 1 mixed, 2 all candidates
+  // kModeSmall: 0 no candidate; 1 a table over carries; 2 all candidates. With L > 4 also 3: no candidate in
+  // its first L bytes, so its kept starts are the same for every carry (kept count and carry-out in
+  // s_wcnt and s_wend); 4: a table whose carry-out is the same for every carry (in s_wend)
+  __shared__ uint8_t s_kind[NS][NR];
+  // L > 4: how the carry into a region follows from the super-tile's: 1: regions 1.. have the carries s_cw
+  // whatever it is; 2: all candidates, a closed form; 0: the tables
+  __shared__ uint8_t s_cw[NS][NR], s_placed[NS];
   // per region: output offset in the super-tile's, length, first byte not covered by an earlier
   // match (relative to the super-tile), kept count
   __shared__ uint4 s_reg[NS][NR];
@@ -4163,10 +4297,12 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     const uint8_t* psrc = L <= (uint32_t)kInlineMax ? p.pat : p.pat_ext;
     const uint8_t* rsrc = R <= (uint32_t)kInlineMax ? p.rep : p.rep_ext;
     for (uint32_t i = tid; i < L; i += kRegionThreads) ps[i] = psrc[i];
-    for (uint32_t i = tid; i < R + 16; i += kRegionThreads) rs[i] = R ? rsrc[i % R] : (uint8_t)0;
     if (R >= 1u && R <= 64u) {
+      for (uint32_t i = tid; i < R + 16; i += kRegionThreads) rs[i] = rsrc[mod_small(i, R, p.rmag)];
       uint8_t* t16 = smem + lay.tab16;
-      for (uint32_t i = tid; i < R * 16u; i += kRegionThreads) t16[i] = rsrc[((i >> 4) + (i & 15u)) % R];
+      for (uint32_t i = tid; i < R * 16u; i += kRegionThreads) t16[i] = rsrc[mod_small((i >> 4) + (i & 15u), R, p.rmag)];
+    } else {
+      for (uint32_t i = tid; i < R + 16; i += kRegionThreads) rs[i] = R ? rsrc[i < R ? i : i - R] : (uint8_t)0;
     }
   }
   if (NT == 0 && blockIdx.x == 0 && tid == 0) {  // nothing to emit: still report
@@ -4184,6 +4320,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     const uint32_t k = s_kind[slot][q];
     if (k == 0u) return 0u;
     if (k == 2u) return dense_region_entry(y, L);
+    if (k == 3u) return s_wcnt[slot][q] | (s_wend[slot][q] << 16);
     const uint8_t* const wt = smem + lay.wtab + slot * lay.wtab_set;
     if (L <= 4u) return reinterpret_cast<const uint32_t*>(wt)[q * L + y];
     const uint32_t v = reinterpret_cast<const uint16_t*>(wt)[q * L + y];
@@ -4296,23 +4433,76 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
           s_supx[slot][lane] = sup_carry;
         }
       } else {
-        uint8_t* const wrec = smem + lay.wrec + slot * lay.wrec_set;
-        for (uint32_t c = lane; c < L; c += 32u) {
-          uint32_t y = c, kc = 0;
-#pragma unroll 1
-          for (uint32_t q = 0; q < NR; ++q) {
-            wrec[q * L + c] = (uint8_t)y;
-            const uint32_t v = region_entry(slot, q, y);
-            kc += v & 0xFFFFu;
-            y = v >> 16;
+        // When every region's carry-out is the same for every carry (nearly always: a gap of L bytes
+        // without candidates is enough), each region's carry-in is its predecessor's carry-out and the lanes
+        // fold in parallel; otherwise a lane per carry goes through the regions one after the other.
+        uint32_t kc[2], kx[2];  // entries lane and lane + 32 of the super-tile's function
+        const uint32_t k = lane < NR ? s_kind[slot][lane] : 0u;
+        const bool same_out = __all_sync(0xffffffffu, k != 1u && k != 2u);
+        bool fixed = false;     // the kept count does not depend on the carry either
+        const bool dense = __all_sync(0xffffffffu, lane >= NR || k == 2u);  // a run from end to end: closed forms
+        if (dense) {
+#pragma unroll
+          for (uint32_t h = 0; h < 2u; ++h) {
+            const uint32_t c = lane + 32u * h;
+            kc[h] = ((uint32_t)S - c + L - 1u) / L;
+            kx[h] = c + kc[h] * L - (uint32_t)S;
           }
-          s_supc[slot][c] = kc;
-          s_supx[slot][c] = y;
-          if (t > 0) __stcg(p.agg + (unsigned long long)t * L + c, (unsigned long long)kc | ((unsigned long long)y << 32));
+        } else if (same_out) {
+          const uint32_t co = k >= 3u ? s_wend[slot][lane] : 0u;
+          uint32_t y = __shfl_up_sync(0xffffffffu, co, 1);
+          const uint32_t rest = __reduce_add_sync(
+              0xffffffffu, lane > 0u && lane < NR ? region_entry(slot, lane, y) & 0xFFFFu : 0u);
+          const uint32_t out = __shfl_sync(0xffffffffu, co, NR - 1u);
+          fixed = __shfl_sync(0xffffffffu, k, 0) != 4u;
+          if (lane > 0u && lane < NR) s_cw[slot][lane] = (uint8_t)y;
+#pragma unroll
+          for (uint32_t h = 0; h < 2u; ++h) {
+            const uint32_t c = lane + 32u * h;
+            kc[h] = rest + (region_entry(slot, 0, c < L ? c : 0u) & 0xFFFFu);
+            kx[h] = out;
+          }
+        } else {
+          uint8_t* const wrec = smem + lay.wrec + slot * lay.wrec_set;
+#pragma unroll
+          for (uint32_t h = 0; h < 2u; ++h) {
+            const uint32_t c = lane + 32u * h;
+            uint32_t y = c;
+            kc[h] = 0;
+#pragma unroll 1
+            for (uint32_t q = 0; q < NR && c < L; ++q) {
+              wrec[q * L + c] = (uint8_t)y;
+              const uint32_t v = region_entry(slot, q, y);
+              kc[h] += v & 0xFFFFu;
+              y = v >> 16;
+            }
+            kx[h] = y;
+          }
         }
+#pragma unroll
+        for (uint32_t h = 0; h < 2u; ++h) {
+          s_supc[slot][lane + 32u * h] = kc[h];
+          s_supx[slot][lane + 32u * h] = kx[h];
+        }
+        if (lane == 0) s_placed[slot] = dense ? 2u : (same_out ? 1u : 0u);
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&s_folded[slot]);
+          // (see RunningCarry; a count that depends on the carry is read from the table, so that goes first)
+          if (fixed) rec_store(p.rec, t, rec_word(tag, kStAgg, kc[0]), rec_word(tag, kStAgg, kx[0] | kRecSame | kRecFixed));
+        }
+#pragma unroll
+        for (uint32_t h = 0; h < 2u; ++h)
+          if (lane + 32u * h < L)
+            __stcg(p.agg + (unsigned long long)t * L + lane + 32u * h,
+                   (unsigned long long)kc[h] | ((unsigned long long)kx[h] << 32));
         __threadfence();
         __syncwarp();
-        if (t > 0 && lane == 0) st_release_u32(p.status + t, (p.epoch << 2) | kStAgg);
+        if (lane == 0) {
+          if (!fixed) rec_store(p.rec, t, rec_word(tag, kStAgg, kc[0]), rec_word(tag, kStAgg, kx[0] | (same_out ? kRecSame : (dense ? kRecDense : 0u))));
+          if (t > 0) st_release_u32(p.status + t, (p.epoch << 2) | kStAgg);
+        }
+        continue;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_folded[slot]);
@@ -4324,6 +4514,8 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     // ================================================================ look-back warps
     RunningSum run;  // kModeFree
     run.init();
+    RunningCarry runc;  // L > 4
+    runc.init(carry0);
 #pragma unroll 1
     for (uint32_t i = warp - kLookback;; i += kLookbacks) {
       const uint32_t slot = i % NS, par = (i / NS) & 1u;
@@ -4362,7 +4554,10 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
           olen = vb - min(x0 - qs, vb) - wc * L + over + wc * R;
           last1 = __reduce_max_sync(0xffffffffu, wc ? we - L + 1u : 0u);
         } else if (vb) {
-          const uint32_t cw = (smem + lay.wrec + slot * lay.wrec_set)[lane * L + c];
+          const uint32_t how = L > 4u ? s_placed[slot] : 0u;
+          const uint32_t cw = how == 1u   ? (lane ? s_cw[slot][lane] : c)
+                              : how == 2u ? dense_seg_carry(c, qs, L)
+                                          : (smem + lay.wrec + slot * lay.wrec_set)[lane * L + c];
           const uint32_t e = region_entry(slot, lane, cw);
           wc = e & 0xFFFFu;
           x0 = qs + cw;
@@ -4395,26 +4590,16 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
             ok = lookback_small_rec<3>(p, t, &K, &c, carry0);
           else if (L == 4u)
             ok = lookback_small_rec<4>(p, t, &K, &c, carry0);
-          else if (L <= 32u)
-            ok = lookback_table<1>(p, t, L, &K, &c, carry0);
           else
-            ok = lookback_table<2>(p, t, L, &K, &c, carry0);
+            ok = runc.reach(p, t, L, &K, &c, carry0);
         }
         if (!pipe_wait(p, &s_folded[slot], par)) break;
       }
       if (!ok) K = c = 0;
       const unsigned long long Kin = K + s_supc[slot][MODE == kModeFree ? 0u : c];
       const uint32_t cout = s_supx[slot][MODE == kModeFree ? 0u : c];
-      if (MODE == kModeSmall && lane == 0) {  // the inclusive prefix, for later super-tiles
-        if (use_rec) {
-          rec_store(p.rec, t, rec_word(tag, kStInc, Kin), rec_word(tag, kStInc, cout));
-        } else {
-          __stcg(&p.incl[t].kept, Kin);
-          __stcg(&p.incl[t].carry, cout);
-          __threadfence();
-          st_release_u32(p.status + t, (p.epoch << 2) | kStInc);
-        }
-      }
+      if (MODE == kModeSmall && use_rec && lane == 0)  // the inclusive prefix, for later super-tiles
+        rec_store(p.rec, t, rec_word(tag, kStInc, Kin), rec_word(tag, kStInc, cout));
       if (MODE == kModeSmall || c != 0u) place(c);
       // The output range starts len_bias bytes into out[], and the carry0 leading bytes covered by a match
       // kept before this buffer are not emitted here.
@@ -4433,9 +4618,11 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
         if (!fits) atomicExch(&p.res->overflow_epoch, p.epoch);
         if (MODE == kModeFree) record(t, O, total, last1, c, Kin);
         mbar_arrive(&s_ready[slot]);
-        if (MODE == kModeFree || use_rec) {  // (query_prefix reads these)
-          __stcg(&p.incl[t].kept, Kin);
-          __stcg(&p.incl[t].carry, cout);
+        __stcg(&p.incl[t].kept, Kin);  // (query_prefix reads these)
+        __stcg(&p.incl[t].carry, cout);
+        if (!use_rec) {  // ... and lookback_table
+          __threadfence();
+          st_release_u32(p.status + t, (p.epoch << 2) | kStInc);
         }
       }
       __syncwarp();
@@ -4445,7 +4632,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
 
   // ================================================================== worker warps
   const unsigned long long lim = (n_all >= L) ? min(n_all - L + 1, n) : 0ull;  // candidates p < lim
-  const uint32_t rmag = mod_magic(R), step512 = R ? 512u % R : 0u;
+  const uint32_t rmag = p.rmag, step512 = p.step512;
   // every pattern byte the same (kModeSmall: candidates are runs of one byte)
   const bool same = MODE == kModeFree ? L == 1u : p.same != 0u;
   uint32_t r[4];  // first pattern bytes, each in every byte
@@ -4556,14 +4743,52 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
               else
                 ks_warp_tables<4>(mask, p.inv_l, p.stride_mask, sr, wt4);
             } else {
-              // a lane per carry walks the segments that hold candidates
-              for (uint32_t c = lane; c < L; c += 32u) {
-                uint32_t x = c, kc = 0;
-                for (uint32_t sm = some; sm; sm &= sm - 1u) {
-                  const uint32_t s = (uint32_t)__ffs(sm) - 1u;
-                  x = walk_segment(x, s, row[s], L, &kc);
+              const uint64_t m0 = (uint64_t)__shfl_sync(0xffffffffu, (unsigned long long)mask, 0);
+              uint32_t ra = 0, rb = 0;
+              const bool one = single_run(mask, &ra, &rb);
+              if (!(m0 & low_bits(L))) {
+                // no carry reaches a candidate: one walk, by all lanes alike, settles the kept starts
+                uint64_t kept = 0;
+                uint32_t x = 0;
+                if (one) {
+                  kept = run_kept(mask, ra, L, p.stride_mask);
+                  x = ra + (rb - ra + L - 1u) / L * L;
+                } else {
+                  for (uint32_t sm = some; sm; sm &= sm - 1u) {
+                    const uint32_t s = (uint32_t)__ffs(sm) - 1u;
+                    const uint64_t m = (uint64_t)__shfl_sync(0xffffffffu, (unsigned long long)mask, s);
+                    const uint64_t kk = walk_kept(x > 64u * s ? x - 64u * s : 0u, m, L);
+                    if (kk) x = 64u * s + 63u - (uint32_t)__clzll((long long)kk) + L;
+                    if (s == lane) kept = kk;
+                  }
                 }
-                reinterpret_cast<uint16_t*>(wt)[wq * L + c] = (uint16_t)((kc << 6) | (x > kRegion ? x - kRegion : 0u));
+                row[lane] = kept;
+                kind = 3u;
+                cnt = __reduce_add_sync(0xffffffffu, (uint32_t)__popcll(kept));
+                end = x > kRegion ? x - kRegion : 0u;
+              } else {
+                // a lane per carry walks the segments that hold candidates
+                uint32_t lo = ~0u, hi = 0;  // smallest and largest carry-out
+                for (uint32_t c = lane; c < L; c += 32u) {
+                  uint32_t x = c, kc = 0;
+                  if (one) {
+                    x = c > ra ? c : ra;
+                    kc = x < rb ? (rb - x + L - 1u) / L : 0u;
+                    x += kc * L;
+                  } else {
+                    for (uint32_t sm = some; sm; sm &= sm - 1u) {
+                      const uint32_t s = (uint32_t)__ffs(sm) - 1u;
+                      x = walk_segment(x, s, row[s], L, &kc);
+                    }
+                  }
+                  x = x > kRegion ? x - kRegion : 0u;
+                  reinterpret_cast<uint16_t*>(wt)[wq * L + c] = (uint16_t)((kc << 6) | x);
+                  lo = x < lo ? x : lo;
+                  hi = x > hi ? x : hi;
+                }
+                lo = __reduce_min_sync(0xffffffffu, lo);
+                end = __reduce_max_sync(0xffffffffu, hi);
+                if (lo == end) kind = 4u;
               }
             }
           }
@@ -4576,6 +4801,10 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
         s_wend[slot][wq] = end;
       } else {
         s_kind[slot][wq] = (uint8_t)kind;
+        if (kind >= 3u) {
+          s_wcnt[slot][wq] = cnt;
+          s_wend[slot][wq] = end;
+        }
       }
     }
   };
@@ -4670,10 +4899,16 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       if (MODE == kModeSmall) {
         // the greedy from the exact carry into the region
         uint32_t xs = 0;  // carry into the lane's segment
-        if (s_kind[slot][wq] == 2u) {
+        const uint32_t kind = s_kind[slot][wq];
+        bool settled = kind == 3u;
+        if (kind == 2u) {
           xs = dense_seg_carry(c0, lane * 64u, L);
+        } else if (kind == 3u) {  // settled in pass A
         } else if (L <= 4u) {
           xs = (smem + lay.srec + slot * lay.srec_set)[(wq * 32u + lane) * L + c0];
+        } else if (uint32_t ra, rb; single_run(kept, &ra, &rb)) {
+          kept = run_kept(kept, c0 > ra ? c0 : ra, L, p.stride_mask);
+          settled = true;
         } else {
           uint32_t x = c0, kc = 0;
           for (uint32_t sm = __ballot_sync(0xffffffffu, kept != 0ull); sm; sm &= sm - 1u) {
@@ -4682,7 +4917,8 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
             x = walk_segment(x, s, row[s], L, &kc);
           }
         }
-        kept = L <= 4u ? (xs < 64u ? seg_walk(kept, xs, L, p.inv_l, p.stride_mask).kept : 0ull) : walk_kept(xs, kept, L);
+        if (!settled)
+          kept = L <= 4u ? (xs < 64u ? seg_walk(kept, xs, L, p.inv_l, p.stride_mask).kept : 0ull) : walk_kept(xs, kept, L);
         last1 = __reduce_max_sync(0xffffffffu, kept ? qs + lane * 64u + 64u - (uint32_t)__clzll((long long)kept) : 0u);
       }
       if (write || cut) {
@@ -5070,10 +5306,14 @@ cudaError_t launch_super_mode(const ReplaceParams& p, cudaStream_t st, int* grid
   long long grid = (long long)per_sm * device_sm_count();
   if (grid > (long long)p.num_tiles) grid = p.num_tiles;
   if (grid < 1) grid = 1;
-  if (region)
-    replace_region_kernel<MODE><<<(unsigned)grid, kRegionThreads, smem, st>>>(p);
-  else
+  if (region) {
+    ReplaceParams q = p;
+    q.rmag = mod_magic(p.R);
+    q.step512 = p.R ? 512u % p.R : 0u;
+    replace_region_kernel<MODE><<<(unsigned)grid, kRegionThreads, smem, st>>>(q);
+  } else {
     replace_super_kernel<MODE, false><<<(unsigned)grid, kThreads, smem, st>>>(p, SegLaunch{});
+  }
   if (grid_out) *grid_out = (int)grid;
   return cudaGetLastError();
 }

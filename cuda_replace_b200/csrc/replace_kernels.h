@@ -142,6 +142,7 @@ struct ReplaceParams {
   const uint32_t* presence;
   unsigned int presence_shift;
   unsigned int same;              // every pattern byte is the same
+  unsigned int rmag, step512;     // region kernel: ceil(2^32 / R) and 512 mod R (set by its launch)
   // Page-locked host memory that receives the results when the launch ends (region and super-tile
   // kernel; q_* and the scheduler's words are not written). nullptr: none.
   ApplyResult* res_mirror;
