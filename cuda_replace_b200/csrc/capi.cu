@@ -582,8 +582,12 @@ int apply_one(Session* s, const uint8_t* pat, int pat_len, const uint8_t* rep, i
     if (e != cudaSuccess) return (int)e;
     e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return (int)e;
-    const ApplyResult r = *s->res_host;
+    ApplyResult r = *s->res_host;
     if (r.error_epoch == p.epoch) return kErrUnknown;
+    if (out_last && p.nsub && r.kept && r.overflow_epoch != p.epoch) {  // only the device's block has the last kept start
+      e = cudaMemcpy(&r.last_tagged, &s->res->last_tagged, sizeof(r.last_tagged), cudaMemcpyDeviceToHost);
+      if (e != cudaSuccess) return (int)e;
+    }
     if (r.overflow_epoch == p.epoch) {
       if (attempt == 1) return kErrUnknown;
       e = dev_grow(&s->alt, &s->alt_cap, r.out_len, false, 0, s->stream);
@@ -737,7 +741,7 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
         p.presence_shift = s->pres_shift;
       }
     }
-    if (k == nst - 1) p.res_mirror = s->res_host;  // (epochs of earlier launches stay in the block)
+    p.res_mirror = s->res_host;  // (the last launch's lengths stay)
     if (tab_of[(size_t)k] >= 0) {
       p.multi = s->mtab + tab_of[(size_t)k];
       e = crb::launch_replace_multi(p, s->stream, nullptr);

@@ -324,8 +324,24 @@ struct OpMax {
   __device__ __forceinline__ uint32_t operator()(uint32_t a, uint32_t b) const { return a > b ? a : b; }
 };
 
+// What a launch reports, also written to the host's page-locked copy where the launch has one: the caller
+// then only waits for the stream, with no copy to enqueue and wait for.
 __device__ __forceinline__ void set_error(const ReplaceParams& p) {
   atomicExch(&p.res->error_epoch, p.epoch);
+  if (p.res_mirror) *const_cast<volatile unsigned int*>(&p.res_mirror->error_epoch) = p.epoch;
+}
+__device__ __forceinline__ void set_overflow(const ReplaceParams& p) {
+  atomicExch(&p.res->overflow_epoch, p.epoch);
+  if (p.res_mirror) *const_cast<volatile unsigned int*>(&p.res_mirror->overflow_epoch) = p.epoch;
+}
+__device__ __forceinline__ void report(const ReplaceParams& p, unsigned long long out_len, unsigned long long kept) {
+  p.res->out_len = out_len;
+  p.res->kept = kept;
+  if (p.res_mirror) {
+    volatile ApplyResult* m = p.res_mirror;
+    m->out_len = out_len;
+    m->kept = kept;
+  }
 }
 __device__ __forceinline__ bool aborted(const ReplaceParams& p) {
   return *reinterpret_cast<volatile unsigned int*>(&p.res->error_epoch) == p.epoch;
@@ -702,7 +718,7 @@ __global__ void __launch_bounds__(kThreads) replace_tiles_kernel(const __grid_co
       p.res->last_kept = __ldcg(&mine->last);
     }
     const bool fits = (O_t + tile_olen <= p.out_cap) && (O_t <= p.out_cap);
-    if (!fits && tid == 0) atomicExch(&p.res->overflow_epoch, p.epoch);
+    if (!fits && tid == 0) set_overflow(p);
     if (!fits || s_fail) continue;
 
     // ---- 7. assemble output windows in shared memory, store with TMA
@@ -2369,21 +2385,6 @@ __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32
   return true;
 }
 
-// The launch's results to the host's page-locked copy, by the thread that knows every CTA has written
-// its own (the caller then only waits for the stream: no copy to enqueue and wait for).
-__device__ __forceinline__ void mirror_result(const ReplaceParams& p) {
-  if (!p.res_mirror) return;
-  __threadfence();
-  const volatile ApplyResult* r = p.res;
-  volatile ApplyResult* m = p.res_mirror;
-  m->out_len = r->out_len;
-  m->kept = r->kept;
-  m->last_kept = r->last_kept;
-  m->error_epoch = r->error_epoch;
-  m->overflow_epoch = r->overflow_epoch;
-  m->last_tagged = r->last_tagged;
-}
-
 // Input length, output range and super-tile count of the job described by p.
 struct JobDims {
   unsigned long long n_all, n, n16;
@@ -2539,8 +2540,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     if (NT == 0 && blockIdx.x == 0 && threadIdx.x == 0) {  // nothing to emit: still report
       if (p.len_out) *p.len_out = p.len_bias;
       if (p.carry_out) *p.carry_out = carry0 > n ? carry0 - (uint32_t)n : 0u;
-      p.res->out_len = 0;
-      p.res->kept = 0;
+      report(p, 0, 0);
     }
   }
   uint32_t nscan = 0;  // block_excl_scan1 calls so far (selects the scratch buffer)
@@ -3077,7 +3077,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       const uint32_t total = cnt * R;
       noin_last1 = cnt ? m * (uint32_t)kTile + s_cout - L + 1u : 0u;
       const bool fits_t = (O + total <= p.out_cap) && (O <= p.out_cap);
-      if (!fits_t && tid == 0) atomicExch(&p.res->overflow_epoch, p.epoch);
+      if (!fits_t && tid == 0) set_overflow(p);
       if (fits_t && !failed && total) {
         const unsigned long long end = O + total;
         const unsigned long long s0 =
@@ -3147,7 +3147,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       // writes those)
       const bool odd = MODE != kModeFree && __any_sync(0xffffffffu, olen_r != wc * R && wc > 0u);
       const bool fits_t = (O + total <= p.out_cap) && (O <= p.out_cap);
-      if (!fits_t && tid == 0) atomicExch(&p.res->overflow_epoch, p.epoch);
+      if (!fits_t && tid == 0) set_overflow(p);
       if (odd && tid == 0) set_error(p);
       const bool write = fits_t && !odd && !failed;
 #pragma unroll 1
@@ -3376,7 +3376,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       // 0-7 of every warp hold the eight lengths, so the choice is the same in every warp.
       const bool warp_stage = stage_rounds ||
                               __reduce_max_sync(0xffffffffu, lane < 8u ? wolen : 0u) + 15u <= lay.wstage_cap;
-      if (!fits && tid == 0) atomicExch(&p.res->overflow_epoch, p.epoch);
+      if (!fits && tid == 0) set_overflow(p);
       // kModeMulti: the warp's own sum of its threads' lengths must equal the length its slot was
       // given from the pass-A sums, or it would write over its neighbour; a mismatch (which the
       // arithmetic rules out) is reported as an error and the warp writes nothing. The same in
@@ -3556,9 +3556,8 @@ __global__ void __launch_bounds__(kThreads, 3)
         if (lastt >= 0)
           atomicMax(&p.res->last_tagged, ((unsigned long long)p.epoch << 40) | (unsigned long long)(lastt + 1));
         if (t == NT - 1) {
-          p.res->out_len = O - p.len_bias;
           // (kModeMulti: the look-back sums are not match counts; no count is reported)
-          p.res->kept = MODE == kModeMulti ? 0ull : __ldcg(&p.incl[t].kept);
+          report(p, O - p.len_bias, MODE == kModeMulti ? 0ull : __ldcg(&p.incl[t].kept));
           if (p.len_out) *p.len_out = O;
           if (MODE != kModeMulti && p.carry_out) {
             // coverage past the output range n: by the last kept match, or by the carry into
@@ -3652,7 +3651,6 @@ __global__ void __launch_bounds__(kThreads, 3)
     if (d == gridDim.x - 1) {
       atomicExch(sched, 0u);
       atomicExch(sched + 1, 0u);
-      if (!SEG) mirror_result(p);
       __threadfence();
     }
   }
@@ -4308,8 +4306,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
   if (NT == 0 && blockIdx.x == 0 && tid == 0) {  // nothing to emit: still report
     if (p.len_out) *p.len_out = p.len_bias;
     if (p.carry_out) *p.carry_out = carry0 > n ? carry0 - (uint32_t)n : 0u;
-    p.res->out_len = 0;
-    p.res->kept = 0;
+    report(p, 0, 0);
   }
   __syncthreads();
 
@@ -4334,8 +4331,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     if (lastt >= 0)
       atomicMax(&p.res->last_tagged, ((unsigned long long)p.epoch << 40) | (unsigned long long)(lastt + 1));
     if (t == NT - 1) {
-      p.res->out_len = O + len - p.len_bias;
-      p.res->kept = kept;
+      report(p, O + len - p.len_bias, kept);
       if (p.len_out) *p.len_out = O + len;
       if (p.carry_out) {
         // coverage past the output range n: by the last kept match, or by the carry into
@@ -4378,7 +4374,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       marks += t == kNone ? 1u : 0u;
       ++issued;
     }
-    while (ok && done + marks < issued) finish();
+    while (MODE == kModeSmall && ok && done + marks < issued) finish();
     // after a wait that gave up: the loads in flight end before this CTA does
     for (uint32_t j = done; !ok && j < issued; ++j) (void)wait_tile(&s_full[j % NS], (j / NS) & 1u);
     if (lane == 0) {
@@ -4387,7 +4383,6 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       if (d == gridDim.x - 1) {
         atomicExch(&p.res->tile_counter, 0u);
         atomicExch(&p.res->done_ctas, 0u);
-        mirror_result(p);
       }
     }
     return;
@@ -4615,7 +4610,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       }
       __syncwarp();
       if (lane == 0) {
-        if (!fits) atomicExch(&p.res->overflow_epoch, p.epoch);
+        if (!fits) set_overflow(p);
         if (MODE == kModeFree) record(t, O, total, last1, c, Kin);
         mbar_arrive(&s_ready[slot]);
         __stcg(&p.incl[t].kept, Kin);  // (query_prefix reads these)
@@ -4836,7 +4831,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     } else {
       if (lane == 0) s_cutlen[slot] = len;
       const bool room = g0 <= p.out_cap && len <= p.out_cap - g0;
-      if (!room && lane == 0) atomicExch(&p.res->overflow_epoch, p.epoch);
+      if (!room && lane == 0) set_overflow(p);
       if (!room || !write) return;
     }
     gm[lane] = make_uint4((uint32_t)C, (uint32_t)kept, (uint32_t)(C >> 32), (uint32_t)(kept >> 32));

@@ -143,8 +143,8 @@ struct ReplaceParams {
   unsigned int presence_shift;
   unsigned int same;              // every pattern byte is the same
   unsigned int rmag, step512;     // region kernel: ceil(2^32 / R) and 512 mod R (set by its launch)
-  // Page-locked host memory that receives the results when the launch ends (region and super-tile
-  // kernel; q_* and the scheduler's words are not written). nullptr: none.
+  // Page-locked host memory that receives out_len, kept and the epochs of an error or overflow (region
+  // and super-tile kernel), complete when the launch is. nullptr: none.
   ApplyResult* res_mirror;
   uint8_t pat[kInlineMax];
   uint8_t rep[kInlineMax];
