@@ -693,8 +693,7 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
     s->lens_cap = cap;
   }
   if (tabs.size() > s->mtab_cap) {
-    if (s->pres) cudaFree(s->pres);
-  if (s->mtab) cudaFree(s->mtab);
+    if (s->mtab) cudaFree(s->mtab);
     if (s->mtab_host) cudaFreeHost(s->mtab_host);
     s->mtab = nullptr;
     s->mtab_host = nullptr;
