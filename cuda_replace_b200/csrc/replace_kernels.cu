@@ -1034,10 +1034,10 @@ __global__ void empty_pattern_kernel(const uint8_t* __restrict__ in, unsigned lo
 namespace {
 
 constexpr int kNBuf = 2;
-// Regions with up to this many matches are written as pieces: a piece costs about as many
-// instructions as an eighth of the scatter of a region (with 8 matches in most regions, 16 MiB of
-// ACGT took 58 us as pieces and 43 us scattered).
-constexpr uint32_t kPieceMax = 4;
+// Regions with up to this many matches are written as pieces, more by emit_gather (96 MiB with 1 / 2 / 3 / 4
+// matches planted per region: up to 4 as pieces 75.7 / 84.6 / 88.9 / 89.4 us, up to 2 77.2 / 83.3 / 85.3 / 85.8,
+// only 1 80.2 / 83.9 / 85.8 / 86.2).
+constexpr uint32_t kPieceMax = 2;
 constexpr int kMaxSub = 8;
 
 
@@ -2314,45 +2314,56 @@ __device__ __noinline__ bool warp_emit_pieces(uint8_t* out, const uint8_t* tb, u
 
 // Output of a warp region with few matches (at most kGatherMax, output at most kGatherBytes; R <= 64):
 // every 16-byte chunk of the output is taken by one lane, which copies it as if it began a literal
-// run (right up to the chunk's first match); the bytes from each match's replacement to the end of its
-// last chunk are then written over it one per lane. A chunk's source follows from the number of matches
-// that end before it: counted per chunk, then a scan. kept: the lane's kept starts in its segment of the
+// run (right up to the chunk's first match); then a few lanes per match write the bytes from its
+// replacement to the end of its last chunk over that. A chunk's source follows from the number of matches
+// that end before it: the last match to end before a chunk leaves its number there, and a chunk
+// takes the nearest mark below it. kept: the lane's kept starts in its segment of the
 // region at tb + qs; literal bytes [x0, end) (relative to tb); out[g0, g0 + total). scr: kGatherScratch
 // bytes of the warp's own. Returns false, writing nothing, when the lengths do not add up.
-// Bound by instruction issue: its cost grows with the matches, the scatter's does not. 24 MiB of random
-// bytes with 8 / 16 / 20 / 25 planted matches per region: 33.9 / 38.9 / 39.4 / 42.6 us, scattered 35.9
-// (more than 12 scattered) / 40.3 / 40.3 / 41.4 us; 32 MiB of rule lines 107 -> 83 us (pieces before).
-constexpr uint32_t kGatherMax = 20, kGatherBytes = 4064, kGatherScratch = 1024 + 2 * kGatherMax;
+// Bound by instruction issue: its cost grows with the matches, the scatter's does not. Counts per chunk, a
+// scan of them and the whole warp on one match after the other took 1379 instructions for a region of
+// 8 one-byte matches. Random bytes with 4 / 8 / 12 / 16 / 20 matches planted per region, us:
+//   24 MiB: before 32.9 / 34.3 / 37.4 / 39.3 / 40.2, so 29.8 / 30.0 / 32.0 / 35.8 / 39.6, scattered 40.5 / 42.0 / 41.8 / 41.9 / 41.9
+//   96 MiB: before  100 /  110 /  119 /  124 /  126, so 88.9 / 90.7 / 96.9 /  108 /  122, scattered  112 /  120 /  120 /  119 /  119
+constexpr uint32_t kGatherMax = 16, kGatherBytes = 4064, kGatherScratch = 256 + 2 * kGatherMax;
+static_assert(kGatherBytes + 30u < 256u * 16u && kGatherMax <= 32u, "a mark per chunk, a lane per match");
 __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32_t* scr, uint64_t kept, uint32_t qs,
                                          uint32_t x0, uint32_t end, unsigned long long g0, uint32_t total, uint32_t L,
                                          uint32_t R, const uint8_t* rs) {
   const uint32_t lane = threadIdx.x & 31u;
   const int grow = (int)R - (int)L;
-  uint16_t* const os = reinterpret_cast<uint16_t*>(scr + 256);  // output offset of every replacement
+  // mark[c]: replacements that end before chunk c, where that number differs from chunk c - 1's; else 0
+  uint8_t* const mark = reinterpret_cast<uint8_t*>(scr);
+  uint16_t* const os = reinterpret_cast<uint16_t*>(scr + 64);  // output offset of every replacement
   const uint32_t a0 = (uint32_t)g0 & 15u, nch = (total + a0 + 15u) >> 4;  // chunks touched, the first at g0 - a0
-  for (uint32_t c = lane; c < nch; c += 32u) scr[c] = 0;
+  scr[lane] = 0;
+  scr[lane + 32u] = 0;
   const uint32_t cnt = (uint32_t)__popcll(kept);
   const uint32_t incl = warp_incl_scan(cnt, OpSum());
   const uint32_t M = __shfl_sync(0xffffffffu, incl, 31);
-  __syncwarp();
   uint32_t k = incl - cnt;
-  for (uint64_t km = kept; km; km &= km - 1ull, ++k) {
-    const uint32_t o = (uint32_t)((int)(qs + 64u * lane + (uint32_t)__ffsll((long long)km) - 1u - x0) + (int)k * grow);
-    os[k] = (uint16_t)o;
-    const uint32_t ce = (o + R + a0 + 15u) >> 4;  // the first chunk that starts at or after its end
-    if (ce < nch) atomicAdd(scr + ce, 1u);
-  }
+  for (uint64_t km = kept; km; km &= km - 1ull, ++k)
+    os[k] = (uint16_t)((int)(qs + 64u * lane + (uint32_t)__ffsll((long long)km) - 1u - x0) + (int)k * grow);
   __syncwarp();
   {
     const uint32_t lo = os[M - 1u], last = (uint32_t)((int)(lo + x0) - (int)(M - 1u) * grow) + L;  // end of the last match
     if (lo + R + (end > last ? end - last : 0u) != total) return false;
   }
+  const uint32_t up = R + a0 + 15u;  // (os[i] + up) / 16: the first chunk that starts at or after replacement i's end
+  if (lane < M) {
+    const uint32_t ce = (os[lane] + up) >> 4;
+    if (ce < nch && (lane + 1u == M || ce != (os[lane + 1u] + up) >> 4)) mark[ce] = (uint8_t)(lane + 1u);
+  }
+  __syncwarp();
   uint8_t* const og = out + g0;
+  const uint32_t upto = 0xFFFFFFFFu >> (31u - lane);  // lanes 0 .. lane
   uint32_t j = 0, jb = 0;
 #pragma unroll 1
   for (uint32_t c0 = 0; c0 < nch; c0 += 32u) {
     const uint32_t c = c0 + lane;
-    j = jb + warp_incl_scan(c < nch ? scr[c] : 0u, OpSum());
+    const uint32_t v = mark[c], t = __ballot_sync(0xffffffffu, v != 0u) & upto;
+    j = __shfl_sync(0xffffffffu, v, 31 - __clz((int)t));  // the mark nearest below (or at) the chunk
+    j = t ? j : jb;
     jb = __shfl_sync(0xffffffffu, j, 31);
     if (16u * c >= a0 && 16u * c + 16u <= total + a0) {
       const uint32_t src = (uint32_t)((int)(x0 + 16u * c - a0) - (int)j * grow);
@@ -2374,12 +2385,16 @@ __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32
     if (ok) og[b] = tb[(uint32_t)((int)(x0 + b) - (lane < 16u ? 0 : (int)jt * grow))];
   }
   __syncwarp();
+  // from every replacement to the end of its last chunk (or the next one): 1 << lg lanes each
+  const uint32_t lg = R > 16u ? 3u : (M <= 8u ? 2u : 1u);
 #pragma unroll 1
-  for (uint32_t i = 0; i < M; ++i) {
+  for (uint32_t i = lane >> lg; i < M; i += 32u >> lg) {
     const uint32_t o = os[i], nx = i + 1u < M ? os[i + 1u] : total;
-    const uint32_t fe = ((o + R + a0 + 15u) & ~15u) - a0, to = fe < nx ? fe : nx;
-    for (uint32_t b = o + lane; b < to; b += 32u)
-      og[b] = b < o + R ? rs[b - o] : tb[(uint32_t)((int)(x0 + b) - (int)(i + 1u) * grow)];
+    const uint32_t fe = ((o + up) & ~15u) - a0, to = fe < nx ? fe : nx;
+    const int back = (int)x0 - (int)(i + 1u) * grow;
+#pragma unroll 1
+    for (uint32_t b = o + (lane & ((1u << lg) - 1u)); b < to; b += 1u << lg)
+      og[b] = *(b < o + R ? rs + (b - o) : tb + (uint32_t)((int)b + back));
   }
   __syncwarp();
   return true;
