@@ -325,6 +325,7 @@ int session_create(Session** out) {
   if (e == cudaSuccess) e = cudaMalloc(&s->res, sizeof(ApplyResult));
   if (e == cudaSuccess) e = cudaMemsetAsync(s->res, 0, sizeof(ApplyResult), s->stream);
   if (e == cudaSuccess) e = cudaMallocHost(&s->res_host, sizeof(ApplyResult));
+  if (e == cudaSuccess) memset(s->res_host, 0, sizeof(ApplyResult));  // (launches write only what they find)
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) {
     session_free(s);
