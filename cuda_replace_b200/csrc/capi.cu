@@ -611,7 +611,7 @@ int apply_one(Session* s, const uint8_t* pat, int pat_len, const uint8_t* rep, i
 
 // apply_batch with the lengths chained on the device: one launch per stage (one pair, or a run
 // of pairs applied in one pass) and a single read-back at the end, instead of a host round trip
-// per pair. Used when every pair fits the super-tile kernel with inline pattern bytes and the
+// per pair. Used when every pair has a kernel with super-tiles (nsub > 0), with inline pattern bytes, and the
 // worst-case lengths along the chain fit in memory; returns kFallback when the caller must use
 // one apply per pair.
 int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, const uint8_t** reps,
@@ -1148,7 +1148,7 @@ CR_EXPORT void cuda_replace_close(void* h) {
   session_free(s);
 }
 
-// unified() for a large page-locked input and a pattern the super-tile kernel takes: every
+// unified() for a large page-locked input and a pattern a kernel with super-tiles takes: every
 // chunk's upload is queued at once; each chunk is replaced as soon as it is on the device (its
 // last L - 1 bytes held back for the next chunk, the coverage carried across on the device)
 // into the session's output buffer, and its output is downloaded into the result while the

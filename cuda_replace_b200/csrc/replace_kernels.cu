@@ -6,7 +6,10 @@
 //   suppress  cuda_replace.cu:737-884, 905-968   (thread-0 / <<<1,1>>> serial greedy)
 //   scan      cuda_replace.cu:237-352, 1223-1244 (three-stage scan, 32-bit local offsets)
 //   scatter   cuda_replace.cu:1391-1608          (u16 padded array, range-sliced expand)
-// Here all four are one launch:
+// Here all four are one launch, of one of three kernels (super_nsub): the region kernel (inputs up to 64 MiB, and every
+// pattern of 5 to 64 bytes that overlaps itself), the super-tile kernel (larger inputs, segmented launches, stages
+// of several pairs), both described where they stand, and the tile kernel (longer patterns that overlap
+// themselves, and the entry point that allocates nothing):
 //   1. TMA (cp.async.bulk) stages a 16 KiB tile plus an (L-1)-byte halo in shared memory.
 //   2. Each thread owns 64 bytes; it compares the first min(L,4) pattern bytes at all 64
 //      positions with funnel shifts over 32-bit words and verifies the rest only for the
@@ -2920,7 +2923,8 @@ __global__ void __launch_bounds__(kThreads, 3)
   // out[g0, g0 + wtot). This thread's segment of the sub-tile at tb has the kept starts `kept`, its
   // first x_in bytes covered by an earlier match and V valid bytes. Equal lengths: the replacements
   // are written over the matches in shared memory and the region copied. At most kPieceMax
-  // matches: literal runs between replacements (emit_pieces). Otherwise the bytes are scattered
+  // matches: literal runs between replacements (warp_emit_pieces); at most kGatherMax: chunks gathered
+  // (emit_gather). Otherwise the bytes are scattered
   // into the warp's staging area (scatter_segments) and copied out, in rounds of as many segments
   // as fit it (a segment that alone outgrows it goes straight to global memory).
   // Lengths that do not add up to wtot (which the arithmetic rules out) report an error.

@@ -1,14 +1,14 @@
 // replace_kernels.h - launch interface between the session layer (capi.cu) and the
 // sm_100a kernels (replace_kernels.cu).
 //
-// One apply of (pattern P of length L, replacement R) over an input of n bytes is ONE
-// launch of replace_tiles_kernel. The input is cut into 16 KiB tiles; each CTA of a
-// persistent grid takes tiles in increasing order from an atomic counter, stages the
-// tile plus an (L-1)-byte halo in shared memory with a 1-D TMA bulk copy, finds the
-// candidate positions, publishes the tile's carry function, resolves its exact
-// carry-in with a decoupled look-back over the predecessors, and writes its output
-// bytes at a 64-bit offset with TMA bulk stores. The leftmost, non-overlapping rule
-// of bytes.replace is exact across every tile boundary; no second pass exists.
+// One apply of (pattern P of length L, replacement R) over an input of n bytes is ONE launch: of
+// replace_region_kernel (p.nsub == 1), replace_super_kernel (p.nsub sub-tiles of 16 KiB per super-tile) or
+// replace_tiles_kernel (p.nsub == 0). Each CTA of a persistent grid takes (super-)tiles in increasing order from an
+// atomic counter, stages them plus an (L-1)-byte halo in shared memory with 1-D TMA bulk copies, finds the
+// candidate positions, publishes the tile's carry function, resolves its exact carry-in with a
+// decoupled look-back over the predecessors, and writes its output bytes at a 64-bit offset.
+// The leftmost, non-overlapping rule of bytes.replace is exact across every tile boundary; no second
+// pass exists.
 #pragma once
 
 #include <cstdint>
@@ -108,7 +108,7 @@ struct ReplaceParams {
   unsigned int inv_l;             // ceil(65536 / L), for L < 64
   unsigned int query_limit;       // query kernel: tile-relative limit
   unsigned int query_tile;        // query kernel: tile index
-  unsigned int nsub;              // super-tile kernel: 16 KiB sub-tiles per super-tile (0 = tile kernel)
+  unsigned int nsub;              // super-tile kernel: 16 KiB sub-tiles per super-tile (1 = region kernel, 0 = tile kernel)
   unsigned long long query_limit64;  // super-tile query: absolute limit
   unsigned int* status;           // [num_tiles]
   TileIncl* incl;                 // [num_tiles]
