@@ -5266,14 +5266,16 @@ static_assert(kApplySub != kRegionSub, "nsub tells the kernel");
 // output, so on large inputs the look-back bounds it, where the super-tile kernel reads the input a second
 // time from L2. Microseconds, super-tile kernel / region kernel:
 //                      1 MiB      16 MiB     64 MiB     128 MiB
-//   entity in text   21.4/13.2  26.2/20.3  56.9/55.5  89.4/102
-//   binary deletion  16.0/12.7  26.3/17.5  45.3/41.0  74.1/73.6
-//   ACGT -> N        34.2/13.6  45.1/28.1   129/77.5   219/145 (150 with the gather)
-//   line ends, CRLF  32.4/14.3  39.9/33.2   101/88.7   178/159
-//   a run, L = 1     15.6/12.4  21.9/21.7  57.8/54.7  96.1/98.5
-//   a run, L = 2     15.8/14.8  18.4/21.6  32.1/47.8  55.5/84.9 (overlapping itself: up to 8 MiB)
+//   entity in text   19.6/12.9  24.1/21.0  50.3/54.9  80.3/102
+//   binary deletion  16.4/10.4  21.6/19.1  43.9/42.4  71.5/74.4
+//   ACGT -> N        25.9/15.4  32.7/28.4  80.4/69.3  129/127
+//   line ends, CRLF  28.9/15.4  35.7/32.9  92.1/88.6  151/157
+//   a random byte    25.7/13.8  30.0/25.6  69.4/64.4  112/116 (made two)
+//   a run, L = 1     16.8/10.9  22.0/21.5  57.4/57.2  98.3/102
+//   a run, L = 2     16.1/15.4  18.9/21.8  33.1/49.2  55.7/86.4 (overlapping itself: up to 8 MiB)
+//   AA in ACGT       42.5/22.8  50.9/42.3  130/117    223/214 (the same: by the slower loser, the run)
 // Bordered patterns of 5 to 64 bytes are always the region kernel's (64 MiB run of 6: 397 -> 122 us;
-// 32 MiB of rule lines, L = 40, which the tile kernel took before: 1020 -> 83 us).
+// 32 MiB of rule lines, L = 40, which the tile kernel took before: 1020 -> 64 us).
 uint32_t super_tile(const ReplaceParams& p) { return super_tile_bytes(p); }
 
 uint32_t super_nsub(uint32_t mode, uint32_t L, unsigned long long n) {
