@@ -204,7 +204,8 @@ cudaError_t dev_grow(uint8_t** ptr, size_t* cap, size_t need, bool keep, size_t 
   return cudaSuccess;
 }
 
-cudaError_t ensure_scratch(Session* s, size_t tiles, size_t entries_per_tile) {
+// Look-back scratch for launches of up to `tiles` (super-)tiles and `entries` table entries in all.
+cudaError_t ensure_scratch(Session* s, size_t tiles, size_t entries) {
   if (tiles > s->tiles_cap) {
     const size_t cap = tiles + tiles / 8 + 64;
     uint32_t* st = nullptr;
@@ -237,6 +238,8 @@ cudaError_t ensure_scratch(Session* s, size_t tiles, size_t entries_per_tile) {
     if (e != cudaSuccess) {
       cudaFree(st);
       cudaFree(in);
+      cudaFree(tl);
+      cudaFree(rc);
       return e;
     }
     if (s->status) cudaFree(s->status);
@@ -249,7 +252,6 @@ cudaError_t ensure_scratch(Session* s, size_t tiles, size_t entries_per_tile) {
     s->rec = rc;
     s->tiles_cap = cap;
   }
-  const size_t entries = tiles * entries_per_tile;
   if (entries > s->agg_cap) {
     const size_t cap = entries + entries / 8 + 1024;
     unsigned long long* a = nullptr;
@@ -539,7 +541,7 @@ int apply_one(Session* s, const uint8_t* pat, int pat_len, const uint8_t* rep, i
   const size_t tiles = (n + tile_bytes - 1) / tile_bytes;
   if (tiles > 0xFFFFFFF0ull) return (int)cudaErrorInvalidValue;
   p.num_tiles = (uint32_t)tiles;
-  e = ensure_scratch(s, tiles, p.agg_entries);
+  e = ensure_scratch(s, tiles, tiles * p.agg_entries);
   if (e != cudaSuccess) return (int)e;
   p.tile_last = s->tile_last;
   p.rec = s->rec;
@@ -675,9 +677,15 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
     k = k1;
   }
   if (maxb > std::max<size_t>(4 * s->len, s->len + (1ull << 30))) return kFallback;
-  cudaError_t e = dev_grow(&s->buf, &s->buf_cap, maxb ? maxb : 1, true, s->len, s->stream);
-  if (e == cudaSuccess) e = dev_grow(&s->alt, &s->alt_cap, maxb ? maxb : 1, false, 0, s->stream);
+  // The worst case need not fit where the lengths that occur do: one apply per pair then. (The buffer that
+  // holds the input grows last: left as it is when something does not fit, it leaves those applies the room.)
+  cudaError_t e = dev_grow(&s->alt, &s->alt_cap, maxb ? maxb : 1, false, 0, s->stream);
   if (e == cudaSuccess) e = ensure_scratch(s, tiles_max, entries_max);
+  if (e == cudaSuccess) e = dev_grow(&s->buf, &s->buf_cap, maxb ? maxb : 1, true, s->len, s->stream);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return kFallback;
+  }
   if (e != cudaSuccess) return (int)e;
   if ((size_t)count + 1 > s->lens_cap) {
     if (s->lens) cudaFree(s->lens);
@@ -1077,7 +1085,7 @@ CR_EXPORT int cuda_replace_apply_device_async(void* h, const uint8_t* d_in, size
   const size_t tiles = (n + tile_bytes - 1) / tile_bytes;
   if (tiles > 0xFFFFFFF0ull) return (int)cudaErrorInvalidValue;
   p.num_tiles = (uint32_t)tiles;
-  e = ensure_scratch(s, tiles, p.agg_entries);
+  e = ensure_scratch(s, tiles, tiles * p.agg_entries);
   if (e != cudaSuccess) return (int)e;
   p.tile_last = s->tile_last;
   p.rec = s->rec;
@@ -1196,7 +1204,8 @@ int unified_chunked(Session* s, const uint8_t* src, size_t n, const uint8_t* pat
   if (e == cudaSuccess && !s->olen_dev) e = cudaMalloc(&s->olen_dev, sizeof(unsigned long long));
   if (e == cudaSuccess) e = dev_grow(&s->buf, &s->buf_cap, n, false, 0, s->stream);
   if (e == cudaSuccess) e = dev_grow(&s->alt, &s->alt_cap, bound ? bound : 1, false, 0, s->stream);
-  if (e == cudaSuccess) e = ensure_scratch(s, (2 * chunk + P + tile_bytes - 1) / tile_bytes + 1, proto.agg_entries);
+  const size_t most_tiles = (2 * chunk + P + tile_bytes - 1) / tile_bytes + 1;
+  if (e == cudaSuccess) e = ensure_scratch(s, most_tiles, most_tiles * proto.agg_entries);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->carry2, 0, 2 * sizeof(unsigned int), s->stream);
   if (e != cudaSuccess) return (int)e;
   uint8_t* host = static_cast<uint8_t*>(pinned_pool().get(bound ? bound : 1, &e));
