@@ -69,7 +69,7 @@ class Arena {
   }
   cudaError_t init(size_t bytes) {
     bytes = rup(bytes, 2u << 20);
-    cudaError_t e = cudaMalloc(&base_, bytes);
+    cudaError_t e = crb::dev_malloc(&base_, bytes);
     if (e != cudaSuccess) return e;
     size_ = bytes;
     free_[0] = bytes;
@@ -261,12 +261,12 @@ struct Slot {
     drop_graphs();  // the graphs hold the old pointers
     free_scratch();
     const size_t cap = rup(need + need / 4 + 256, 1024);
-    cudaError_t e = cudaMalloc(&d_tile_job, cap * sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMalloc(&status, cap * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&incl, cap * sizeof(TileIncl));
-    if (e == cudaSuccess) e = cudaMalloc(&agg, cap * crb::kSegMaxL * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&tile_last, cap * sizeof(long long));
-    if (e == cudaSuccess) e = cudaMalloc(&rec, cap * 2 * sizeof(unsigned long long));
+    cudaError_t e = crb::dev_malloc(&d_tile_job, cap * sizeof(unsigned int));
+    if (e == cudaSuccess) e = crb::dev_malloc(&status, cap * sizeof(uint32_t));
+    if (e == cudaSuccess) e = crb::dev_malloc(&incl, cap * sizeof(TileIncl));
+    if (e == cudaSuccess) e = crb::dev_malloc(&agg, cap * crb::kSegMaxL * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = crb::dev_malloc(&tile_last, cap * sizeof(long long));
+    if (e == cudaSuccess) e = crb::dev_malloc(&rec, cap * 2 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemsetAsync(status, 0, cap * sizeof(uint32_t), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(rec, 0, cap * 2 * sizeof(unsigned long long), st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -285,17 +285,17 @@ struct Slot {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_meta, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreate(&ev_t0);
     if (e == cudaSuccess) e = cudaEventCreate(&ev_t1);
-    if (e == cudaSuccess) e = cudaMalloc(&d_jobs, tables * sizeof(SegJob));
+    if (e == cudaSuccess) e = crb::dev_malloc(&d_jobs, tables * sizeof(SegJob));
     if (e == cudaSuccess) e = cudaMallocHost(&h_jobs, tables * sizeof(SegJob));
-    if (e == cudaSuccess) e = cudaMalloc(&d_njobs, kMaxRounds * kClasses * sizeof(unsigned int));
+    if (e == cudaSuccess) e = crb::dev_malloc(&d_njobs, kMaxRounds * kClasses * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMallocHost(&h_njobs, kMaxRounds * kClasses * sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMalloc(&d_pairs, (size_t)max_jobs * kMaxRounds * sizeof(SegPair));
+    if (e == cudaSuccess) e = crb::dev_malloc(&d_pairs, (size_t)max_jobs * kMaxRounds * sizeof(SegPair));
     if (e == cudaSuccess) e = cudaMallocHost(&h_pairs, (size_t)max_jobs * kMaxRounds * sizeof(SegPair));
-    if (e == cudaSuccess) e = cudaMalloc(&d_res, (size_t)max_jobs * sizeof(ApplyResult));
+    if (e == cudaSuccess) e = crb::dev_malloc(&d_res, (size_t)max_jobs * sizeof(ApplyResult));
     if (e == cudaSuccess) e = cudaMallocHost(&h_res, (size_t)max_jobs * sizeof(ApplyResult));
-    if (e == cudaSuccess) e = cudaMalloc(&d_lens, (size_t)max_jobs * 2 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = crb::dev_malloc(&d_lens, (size_t)max_jobs * 2 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMallocHost(&h_lens, (size_t)max_jobs * 2 * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&d_ctl, 8 * sizeof(unsigned int));
+    if (e == cudaSuccess) e = crb::dev_malloc(&d_ctl, 8 * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMemsetAsync(d_ctl, 0, 8 * sizeof(unsigned int), st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     return e;
@@ -553,9 +553,9 @@ class Engine {
     const size_t n = 2u << 20;
     uint8_t* buf = nullptr;
     unsigned long long* lens = nullptr;
-    cudaError_t e = cudaMalloc(&buf, (size_t)nj * 2 * (n + 4096));
+    cudaError_t e = crb::dev_malloc(&buf, (size_t)nj * 2 * (n + 4096));
     if (e != cudaSuccess) return e;
-    e = cudaMalloc(&lens, (size_t)nj * 2 * sizeof(unsigned long long));
+    e = crb::dev_malloc(&lens, (size_t)nj * 2 * sizeof(unsigned long long));
     std::vector<uint8_t> host(n);
     uint32_t x = 12345u;
     for (size_t i = 0; i < n; ++i) {
@@ -1114,6 +1114,7 @@ CR_EXPORT int cuda_replace_server_open(void** srv, size_t hbm_budget, int max_jo
   auto* s = new (std::nothrow) Server(dev);
   if (!s) return -2;
   const int mj = max_jobs_per_batch > 0 ? std::min(max_jobs_per_batch, 65536) : 4096;
+  if (!hbm_budget) crb::dev_blocks_trim();  // (the idle blocks of finished streams count as free)
   const int rc = s->open(hbm_budget ? hbm_budget : default_budget(), mj);
   if (rc != 0) {
     delete s;
@@ -1222,6 +1223,7 @@ CR_EXPORT int cuda_replace_jobs(int njobs, const uint8_t** srcs, const size_t* s
       cuda_replace_server_close(g_jobs_srv[dev]);
       g_jobs_srv[dev] = nullptr;
     }
+    crb::dev_blocks_trim();
     const size_t budget = std::min(default_budget(), std::max(want, (size_t)256 << 20));
     int rc = cuda_replace_server_open(&g_jobs_srv[dev], budget, 4096);
     if (rc != 0) {
@@ -1268,4 +1270,5 @@ CR_EXPORT void cuda_replace_jobs_release(void) {
       g_jobs_srv[d] = nullptr;
       g_jobs_budget[d] = 0;
     }
+  crb::dev_blocks_trim();
 }

@@ -179,13 +179,11 @@ cudaError_t dev_grow(uint8_t** ptr, size_t* cap, size_t need, bool keep, size_t 
   if (*cap >= need && *ptr) return cudaSuccess;
   const size_t new_cap = round_up(need + need / 8 + 4096, kAllocQuantum);
   uint8_t* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, new_cap);
+  cudaError_t e = crb::dev_malloc(&p, new_cap);
   if (e != cudaSuccess) {
-    cudaGetLastError();
-    crb::dev_blocks_trim();
     // retry without headroom before giving up
     const size_t tight = round_up(need + 4096, 4096);
-    e = cudaMalloc(&p, tight);
+    e = crb::dev_malloc(&p, tight);
     if (e != cudaSuccess) return e;
     *cap = tight;
   } else {
@@ -211,21 +209,21 @@ cudaError_t ensure_scratch(Session* s, size_t tiles, size_t entries) {
     uint32_t* st = nullptr;
     TileIncl* in = nullptr;
     long long* tl = nullptr;
-    cudaError_t e = cudaMalloc(&st, cap * sizeof(uint32_t));
+    cudaError_t e = crb::dev_malloc(&st, cap * sizeof(uint32_t));
     if (e != cudaSuccess) return e;
-    e = cudaMalloc(&in, cap * sizeof(TileIncl));
+    e = crb::dev_malloc(&in, cap * sizeof(TileIncl));
     if (e != cudaSuccess) {
       cudaFree(st);
       return e;
     }
-    e = cudaMalloc(&tl, cap * sizeof(long long));
+    e = crb::dev_malloc(&tl, cap * sizeof(long long));
     if (e != cudaSuccess) {
       cudaFree(st);
       cudaFree(in);
       return e;
     }
     unsigned long long* rc = nullptr;
-    e = cudaMalloc(&rc, cap * 2 * sizeof(unsigned long long));
+    e = crb::dev_malloc(&rc, cap * 2 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemsetAsync(rc, 0, cap * 2 * sizeof(unsigned long long), s->stream);
     if (e != cudaSuccess) {
       cudaFree(st);
@@ -255,7 +253,7 @@ cudaError_t ensure_scratch(Session* s, size_t tiles, size_t entries) {
   if (entries > s->agg_cap) {
     const size_t cap = entries + entries / 8 + 1024;
     unsigned long long* a = nullptr;
-    cudaError_t e = cudaMalloc(&a, cap * sizeof(unsigned long long));
+    cudaError_t e = crb::dev_malloc(&a, cap * sizeof(unsigned long long));
     if (e != cudaSuccess) return e;
     if (s->agg) cudaFree(s->agg);
     s->agg = a;
@@ -324,7 +322,7 @@ int session_create(Session** out) {
   if (!s) return -2;
   cudaError_t e = cudaGetDevice(&s->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&s->res, sizeof(ApplyResult));
+  if (e == cudaSuccess) e = crb::dev_malloc(&s->res, sizeof(ApplyResult));
   if (e == cudaSuccess) e = cudaMemsetAsync(s->res, 0, sizeof(ApplyResult), s->stream);
   if (e == cudaSuccess) e = cudaMallocHost(&s->res_host, sizeof(ApplyResult));
   if (e == cudaSuccess) memset(s->res_host, 0, sizeof(ApplyResult));  // (launches write only what they find)
@@ -452,7 +450,7 @@ cudaError_t upload_ext(Session* s, const uint8_t* pat, uint32_t L, const uint8_t
     cudaStreamSynchronize(s->stream);
     if (s->ext) cudaFree(s->ext);
     s->ext = nullptr;
-    cudaError_t e = cudaMalloc(&s->ext, need);
+    cudaError_t e = crb::dev_malloc(&s->ext, need);
     if (e != cudaSuccess) return e;
     s->ext_cap = need;
   }
@@ -682,10 +680,7 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
   cudaError_t e = dev_grow(&s->alt, &s->alt_cap, maxb ? maxb : 1, false, 0, s->stream);
   if (e == cudaSuccess) e = ensure_scratch(s, tiles_max, entries_max);
   if (e == cudaSuccess) e = dev_grow(&s->buf, &s->buf_cap, maxb ? maxb : 1, true, s->len, s->stream);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    return kFallback;
-  }
+  if (e == cudaErrorMemoryAllocation) return kFallback;
   if (e != cudaSuccess) return (int)e;
   if ((size_t)count + 1 > s->lens_cap) {
     if (s->lens) cudaFree(s->lens);
@@ -693,7 +688,7 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
     s->lens = nullptr;
     s->lens_host = nullptr;
     const size_t cap = (size_t)count + 64;
-    e = cudaMalloc(&s->lens, cap * sizeof(unsigned long long));
+    e = crb::dev_malloc(&s->lens, cap * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMallocHost(&s->lens_host, cap * sizeof(unsigned long long));
     if (e != cudaSuccess) {
       s->lens_cap = 0;
@@ -707,7 +702,7 @@ int apply_batch_chained(Session* s, const uint8_t** pats, const int* pat_lens, c
     s->mtab = nullptr;
     s->mtab_host = nullptr;
     const size_t cap = tabs.size() + 8;
-    e = cudaMalloc(&s->mtab, cap * sizeof(crb::MultiTable));
+    e = crb::dev_malloc(&s->mtab, cap * sizeof(crb::MultiTable));
     if (e == cudaSuccess) e = cudaMallocHost(&s->mtab_host, cap * sizeof(crb::MultiTable));
     if (e != cudaSuccess) {
       s->mtab_cap = 0;
@@ -948,7 +943,7 @@ CR_EXPORT int cuda_replace_build_index(void* h, size_t chunk_size) {
     if (s->pres) cudaFree(s->pres);
     s->pres = nullptr;
     s->pres_cap = 0;
-    cudaError_t e = cudaMalloc(&s->pres, chunks * 8 * sizeof(uint32_t));
+    cudaError_t e = crb::dev_malloc(&s->pres, chunks * 8 * sizeof(uint32_t));
     if (e != cudaSuccess) return (int)e;
     s->pres_cap = chunks * 8;
   }
@@ -1200,8 +1195,8 @@ int unified_chunked(Session* s, const uint8_t* src, size_t n, const uint8_t* pat
     if (e == cudaSuccess && !s->ev_done[k]) e = cudaEventCreateWithFlags(&s->ev_done[k], cudaEventDisableTiming);
     if (e == cudaSuccess && dst && !s->ev_dl[k]) e = cudaEventCreateWithFlags(&s->ev_dl[k], cudaEventDisableTiming);
   }
-  if (e == cudaSuccess && !s->carry2) e = cudaMalloc(&s->carry2, 2 * sizeof(unsigned int));
-  if (e == cudaSuccess && !s->olen_dev) e = cudaMalloc(&s->olen_dev, sizeof(unsigned long long));
+  if (e == cudaSuccess && !s->carry2) e = crb::dev_malloc(&s->carry2, 2 * sizeof(unsigned int));
+  if (e == cudaSuccess && !s->olen_dev) e = crb::dev_malloc(&s->olen_dev, sizeof(unsigned long long));
   if (e == cudaSuccess) e = dev_grow(&s->buf, &s->buf_cap, n, false, 0, s->stream);
   if (e == cudaSuccess) e = dev_grow(&s->alt, &s->alt_cap, bound ? bound : 1, false, 0, s->stream);
   const size_t most_tiles = (2 * chunk + P + tile_bytes - 1) / tile_bytes + 1;

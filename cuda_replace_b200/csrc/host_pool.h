@@ -326,6 +326,13 @@ void host_arena_register(HostArena* a);
 void host_arena_close(HostArena* a);
 // Give the idle device blocks of finished streams back to the driver (stream.cu).
 void dev_blocks_trim();
+// cudaMalloc of this library: when memory has run out, the idle blocks go back and it is tried once more. An
+// error is reported by the return value only (a later launch's cudaGetLastError does not see it).
+cudaError_t dev_malloc_bytes(void** p, size_t n);
+template <typename T>
+cudaError_t dev_malloc(T** p, size_t n) {
+  return dev_malloc_bytes(reinterpret_cast<void**>(p), n);
+}
 // Release a block handed to a caller: into its host area, else into the pool.
 void host_free(void* p);
 

@@ -64,7 +64,8 @@ bool is_pinned(const void* p) {
 // Device blocks of finished streams, kept for the next one: allocating and freeing some thirty of them
 // took 5 ms of every call. At most kMaxIdle bytes are kept, the blocks idle the longest go first; a
 // block is put here only when no stream uses it any more, and all of them go back to the driver when an
-// allocation of this library fails (dev_blocks_trim).
+// allocation of device memory by this library fails (dev_malloc), when a server sizes itself by the free memory,
+// and by cuda_replace_jobs_release.
 class DevBlocks {
  public:
   cudaError_t get(void** p, size_t n) {
@@ -86,13 +87,7 @@ class DevBlocks {
         return cudaSuccess;
       }
     }
-    *p = nullptr;
-    e = cudaMalloc(p, n);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      trim();
-      e = cudaMalloc(p, n);
-    }
+    e = crb::dev_malloc_bytes(p, n);
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> g(mu_);
     live_[*p] = Block{*p, n, dev};
@@ -157,6 +152,20 @@ DevBlocks& blocks() {
 
 namespace crb {
 void dev_blocks_trim() { blocks().trim(); }
+
+cudaError_t dev_malloc_bytes(void** p, size_t n) {
+  *p = nullptr;
+  cudaError_t e = cudaMalloc(p, n);
+  if (e == cudaSuccess) return e;
+  cudaGetLastError();
+  blocks().trim();
+  e = cudaMalloc(p, n);
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();
+  }
+  return e;
+}
 }  // namespace crb
 
 namespace {

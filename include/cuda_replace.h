@@ -331,7 +331,8 @@ int cuda_replace_jobs(int njobs, const uint8_t** srcs, const size_t* src_lens, c
                       const uint8_t** pats, const int* pat_lens, const uint8_t** reps, const int* rep_lens,
                       uint8_t** out_hosts, size_t* out_lens);
 /* Close the server that cuda_replace_jobs keeps and release its device and page-locked memory
- * (the next call opens a new one). */
+ * (the next call opens a new one). Idle device memory that finished streams left for the next one
+ * (at most 1 GiB) is released too. */
 void cuda_replace_jobs_release(void);
 
 #ifdef __cplusplus
