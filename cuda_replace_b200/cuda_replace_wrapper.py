@@ -428,7 +428,10 @@ class Session:
                            stream: int = 0) -> None:
         """Enqueue a replace of device memory d_in[0, n) into d_out on a CUDA stream handle."""
         _need_bytes(pat, rep)
-        rc = self.lib._async(self.h, d_in, n, pat, len(pat), rep, len(rep), d_out, out_cap, stream)
+        # (addresses by way of c_void_p(): an argument declared as one would take a bytes object or an array for its
+        # own address, and the kernel would be given host memory)
+        rc = self.lib._async(self.h, c_void_p(d_in), c_size_t(n), pat, len(pat), rep, len(rep), c_void_p(d_out),
+                             c_size_t(out_cap), c_void_p(stream))
         if rc != 0:
             raise RuntimeError(f"cuda_replace_apply_device_async failed rc={rc}")
 
