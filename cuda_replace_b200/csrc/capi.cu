@@ -378,10 +378,10 @@ cudaError_t upload_host(Session* s, uint8_t* dst, const uint8_t* src, size_t len
 }
 
 // The session buffer to caller memory dst[0, s->len): a large pageable dst by way of a pooled page-locked
-// block. Up to 32 MiB each piece is copied into dst on the host threads as soon as it lands while the next
-// ones download (12 MiB into a fresh bytes object 0.73 -> 0.38 ms); above, one copy after the download
-// is the faster (64 MiB: 3.3 ms against 5.0 ms in pieces, whose first touches of dst's pages collide with
-// the downloads).
+// block in four pieces, each copied into dst on the host threads while the next one downloads. Into fresh
+// memory, whose first touches bound the copies, ms for 1 / 2 / 4 / 8 / 16 pieces: 4 MiB 0.51 / 0.19 / 0.21 / 0.21 / 0.21,
+// 8 MiB 1.15 / 0.68 / 0.30 / 0.35 / 0.35, 16 MiB 1.80 / 0.79 / 0.46 / 0.46 / 0.60, 64 MiB 3.8 / 2.9 / 3.0 / 3.4 / 4.6, 128 MiB
+// 7.4 / 5.3 / 5.6 / 6.5 / 7.0. Smaller pieces than 1 MiB are no work for several threads.
 cudaError_t download_host(Session* s, uint8_t* dst) {
   cudaError_t e = cudaSuccess;
   if (s->len < (3u << 20) || host_is_pinned(dst)) {
@@ -391,16 +391,8 @@ cudaError_t download_host(Session* s, uint8_t* dst) {
   }
   uint8_t* host = static_cast<uint8_t*>(pinned_pool().get(s->len, &e));
   if (!host) return e;
-  if (s->len > ((size_t)32 << 20)) {
-    e = cudaMemcpyAsync(host, s->buf, s->len, cudaMemcpyDeviceToHost, s->stream);
-    const cudaError_t se = cudaStreamSynchronize(s->stream);
-    if (e == cudaSuccess) e = se;
-    if (e == cudaSuccess) crb::parallel_memcpy(dst, host, s->len);
-    pinned_pool().put(host);
-    return e;
-  }
-  // (a piece per event, at most kUnifiedChunks)
-  const size_t piece = std::max<size_t>((size_t)1 << 20, round_up((s->len + kUnifiedChunks - 1) / kUnifiedChunks, (size_t)1 << 18));
+  const size_t piece = std::max<size_t>((size_t)1 << 20, round_up((s->len + 3) / 4, (size_t)1 << 18));
+  static_assert(kUnifiedChunks >= 4, "an event per piece");
   CopyOut copyout;
   copyout.open(s->device);
   for (size_t off = 0, k = 0; e == cudaSuccess && off < s->len; off += piece, ++k) {

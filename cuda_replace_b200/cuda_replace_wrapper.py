@@ -81,12 +81,14 @@ def _bytes_at(ptr, n: int, lib: Optional[C.CDLL] = None) -> bytes:
     """Copy n bytes of library-owned memory into a new bytes object. Large results are copied
     by the library on several host threads into a bytes object created uninitialised (the
     page faults of fresh memory, not the copy, bound a single-threaded copy); ctypes.string_at
-    is not used because its size is a C int, which results of 2 GiB and more overflow."""
+    takes only the small ones, because its size is a C int, which results of 2 GiB and more overflow."""
     if not n:
         return b""
+    if n < _PARALLEL_COPY_MIN:
+        return C.string_at(ptr, n)
     addr = C.cast(ptr, c_void_p).value
     copy = getattr(lib, "cuda_replace_host_copy", None) if lib is not None else None
-    if copy is None or n < _PARALLEL_COPY_MIN:
+    if copy is None:
         return memoryview((C.c_uint8 * n).from_address(addr)).cast("B").tobytes()
     out = _new_bytes(None, n)  # uninitialised, filled below before anyone else sees it
     dst = _bytes_buffer(out)
@@ -386,7 +388,11 @@ class Session:
         return int(kept.value), int(last.value)
 
     def result(self) -> bytes:
-        n = self.length()
+        out_len = c_size_t()
+        rc = self.lib.lib.cuda_replace_length(self.h, C.byref(out_len))
+        if rc != 0:
+            raise RuntimeError(f"cuda_replace_result failed rc={rc}")
+        n = out_len.value
         if n >= _PARALLEL_COPY_MIN:  # straight into the bytes object, the copies behind the download
             def fill(addr, cap):
                 got = c_size_t()
@@ -401,7 +407,6 @@ class Session:
             except _Outgrown:
                 pass
         out_ptr = c_uint8_p()
-        out_len = c_size_t()
         rc = self.lib.lib.cuda_replace_result(self.h, C.byref(out_ptr), C.byref(out_len))
         if rc != 0:
             raise RuntimeError(f"cuda_replace_result failed rc={rc}")

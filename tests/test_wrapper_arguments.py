@@ -39,3 +39,10 @@ def test_patterns_are_bytes(calls, bad):
                 with pytest.raises(TypeError):
                     call()
     assert not seen
+
+
+def test_result_of_a_closed_session_names_the_call(fake_lib_path):
+    s = Wr.Session(Wr.CudaReplaceLib(fake_lib_path), b"abc")
+    s.close()
+    with pytest.raises(RuntimeError, match="cuda_replace_result failed"):
+        s.result()
