@@ -30,7 +30,9 @@ class PinnedPool {
     {
       std::lock_guard<std::mutex> g(mu_);
       auto it = idle_.lower_bound(want);
-      if (it != idle_.end() && it->first <= want + want / 2 + (64ull << 20)) {
+      // (a request of a few bytes takes no large block from the transfers: pinning that anew costs far more)
+      const size_t slack = want <= kSmall ? want : want / 2 + (64ull << 20);
+      if (it != idle_.end() && it->first <= want + slack) {
         void* p = it->second.first;
         idle_bytes_ -= it->first;
         lru_.erase(it->second.second);
@@ -84,6 +86,7 @@ class PinnedPool {
 
  private:
   static constexpr size_t kMaxIdle = 24ull << 30;
+  static constexpr size_t kSmall = 64u << 10;
   std::mutex mu_;
   std::multimap<size_t, std::pair<void*, unsigned long long>> idle_;  // size -> (block, put order)
   std::map<unsigned long long, std::pair<size_t, void*>> lru_;        // put order -> (size, block)
