@@ -2175,7 +2175,10 @@ __device__ __forceinline__ void sts8(uint32_t a, uint32_t v) { asm volatile("st.
 // Bound by instruction issue; before, each lane walked its own matches and emitted words one after
 // the other, which cost a warp as much as its busiest lane at every step: 64 MiB of text, every
 // blank replaced by three bytes, 340 -> 115 us; line ends made CRLF, 149 -> 97 us.
-// ONE: L = 1 and every byte valid (literal = not kept). RC: R, or 5 for any R > 4.
+// A replacement of 17 bytes and more is stored by the whole warp, match by match (its own lane writing it byte by
+// byte held the others up: 64 matches per region made 20 / 48 / 64 bytes, 16 MiB: 133 / 264 / 340 us, so 71 / 79 / 78;
+// the word-by-word walk before this kernel 57 / 64 / 69, which emit_gather beats for up to 128 matches).
+// ONE: L = 1 and every byte valid (literal = not kept). RC: R, 5 for 5 to 16 bytes, 6 for more.
 template <bool ONE, int RC>
 __device__ __forceinline__ void scatter_half(uint32_t stg, uint32_t base, uint32_t v, uint32_t C, uint32_t K, uint32_t below,
                                              uint32_t R, uint32_t rep4, uint32_t rs) {
@@ -2188,12 +2191,22 @@ __device__ __forceinline__ void scatter_half(uint32_t stg, uint32_t base, uint32
     d += ONE ? (uint32_t)__popc(~K & below) : (uint32_t)__popc(C & below);
   } else {
     const uint32_t kb = (uint32_t)__popc(K & below);
-    d += (ONE ? (threadIdx.x & 31u) - kb : (uint32_t)__popc(C & below)) + (RC == 5 ? kb * R : kb * (uint32_t)RC);
+    d += (ONE ? (threadIdx.x & 31u) - kb : (uint32_t)__popc(C & below)) + (RC >= 5 ? kb * R : kb * (uint32_t)RC);
   }
   const bool mat = (K & bit) != 0u, lit = ONE ? !mat : (C & bit) != 0u;
   if (RC == 0) {
     if (lit) sts8(d, v);
   } else {
+    if (RC == 6) {  // the replacements by the whole warp, one match after the other
+      if (lit) sts8(d, v);
+      uint32_t at = stg + base;
+      for (uint32_t km = K; km; km &= km - 1u, at += R) {
+        const uint32_t lo = (km & (0u - km)) - 1u;  // the bytes before the match
+        const uint32_t o = at + (ONE ? (uint32_t)__popc(~K & lo) : (uint32_t)__popc(C & lo));
+        for (uint32_t r = threadIdx.x & 31u; r < R; r += 32u) sts8(o + r, lds8(rs + r));
+      }
+      return;
+    }
     if (lit || mat) sts8(d, mat ? rep4 : v);
     if (RC >= 2 && mat) {
       sts8(d + 1u, rep4 >> 8);
@@ -2231,14 +2244,14 @@ __device__ __noinline__ void scatter_direct(uint8_t* out, const uint8_t* src, co
   const uint32_t b = __shfl_sync(0xffffffffu, pk, s);
   for (uint32_t h = 0; h < 2u; ++h) {
     const uint32_t C = h ? q.z : q.x, K = h ? q.w : q.y;
-    uint8_t* d = out + (b & 0xFFFFu) + (h ? b >> 16 : 0u) + __popc(C & below) + (uint32_t)__popc(K & below) * R;
-    if (C & bit) *d = src[64u * s + 32u * h + lane];
-    if (K & bit)
-      for (uint32_t r = 0; r < R; ++r) d[r] = rs[r];
+    uint8_t* d = out + (b & 0xFFFFu) + (h ? b >> 16 : 0u);
+    if (C & bit) d[__popc(C & below) + (uint32_t)__popc(K & below) * R] = src[64u * s + 32u * h + lane];
+    for (uint32_t km = K; km; km &= km - 1u, d += R)  // the whole warp on one match after the other
+      for (uint32_t r = lane; r < R; r += 32u) d[__popc(C & ((km & (0u - km)) - 1u)) + r] = rs[r];
   }
 }
 
-// scatter_segments by R and shape, kept out of line: its twelve loops would crowd the kernel's instruction
+// scatter_segments by R and shape, kept out of line: its fourteen loops would crowd the kernel's instruction
 // cache (inlined, sparse inputs measured 3-4% slower). Shared-memory addresses, 32 bits each.
 __device__ __noinline__ void scatter_any(uint32_t stg, uint32_t src, uint32_t gm, uint32_t pk, uint32_t s0, uint32_t s1,
                                          uint32_t R, uint32_t rs, bool one) {
@@ -2249,13 +2262,14 @@ __device__ __noinline__ void scatter_any(uint32_t stg, uint32_t src, uint32_t gm
     else                                                                \
       scatter_segments<false, RC>(stg, src, gm, pk, s0, s1, R, rs);     \
     break;
-  switch (R < 5u ? R : 5u) {  // the same in every lane
+  switch (R < 5u ? R : (R <= 16u ? 5u : 6u)) {  // the same in every lane
     CRB_SCATTER(0)
     CRB_SCATTER(1)
     CRB_SCATTER(2)
     CRB_SCATTER(3)
     CRB_SCATTER(4)
     CRB_SCATTER(5)
+    CRB_SCATTER(6)
   }
 #undef CRB_SCATTER
 }
@@ -2315,7 +2329,7 @@ __device__ __noinline__ bool warp_emit_pieces(uint8_t* out, const uint8_t* tb, u
   }
 }
 
-// Output of a warp region with few matches (at most kGatherMax, output at most kGatherBytes; R <= 64):
+// Output of a warp region of few matches or of a moderate number of long replacements (`gathers`):
 // every 16-byte chunk of the output is taken by one lane, which copies it as if it began a literal
 // run (right up to the chunk's first match); then a few lanes per match write the bytes from its
 // replacement to the end of its last chunk over that. A chunk's source follows from the number of matches
@@ -2328,8 +2342,19 @@ __device__ __noinline__ bool warp_emit_pieces(uint8_t* out, const uint8_t* tb, u
 // 8 one-byte matches. Random bytes with 4 / 8 / 12 / 16 / 20 matches planted per region, us:
 //   24 MiB: before 32.9 / 34.3 / 37.4 / 39.3 / 40.2, so 29.8 / 30.0 / 32.0 / 35.8 / 39.6, scattered 40.5 / 42.0 / 41.8 / 41.9 / 41.9
 //   96 MiB: before  100 /  110 /  119 /  124 /  126, so 88.9 / 90.7 / 96.9 /  108 /  122, scattered  112 /  120 /  120 /  119 /  119
-constexpr uint32_t kGatherMax = 16, kGatherBytes = 4064, kGatherScratch = 256 + 2 * kGatherMax;
-static_assert(kGatherBytes + 30u < 256u * 16u && kGatherMax <= 32u, "a mark per chunk, a lane per match");
+// Replacements of 5 bytes and more, 16 MiB, the word-by-word walk and (up to 6 KiB of output per region) staging
+// of a warp before / scattered with a lane per match / so: 26 matches per region made 20 bytes 57 / 70 / 35, 64 bytes
+// 64 / 148 / 43, 200 bytes 146 / (in pieces) 79 / 67; 41 made 5 bytes 66 / 57 / 37, 30 bytes 72 / 130 / 47; 64 made 10 bytes
+// 55 / 90 / 45, 64 bytes 69 / 340 / 64; 102 made 10 bytes 68 / 90 / 55, 30 bytes 79 / 186 / 71.
+constexpr uint32_t kGatherMax = 128, kGatherBytes = 8128, kGatherScratch = 512 + 2 * kGatherMax;
+constexpr uint32_t kScatterR = 1024;  // longest replacement scattered (16-bit lengths of 32 bytes' output)
+// Whether a region of M matches and `total` output bytes is gathered. Up to four bytes per match the scatter's fixed
+// stores are the faster from 17 matches on (64 matches made 1 byte, 72 MiB: 119 gathered, 100 scattered). (R: a chunk
+// inside a replacement reads that far past the region.)
+__device__ __forceinline__ bool gathers(uint32_t M, uint32_t total, uint32_t R) {
+  return M <= (R > 4u ? kGatherMax : 16u) && total <= kGatherBytes && R <= 256u;
+}
+static_assert(kGatherBytes + 30u < 512u * 16u && kGatherMax <= 255u, "a mark per chunk, of 8 bits");
 __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32_t* scr, uint64_t kept, uint32_t qs,
                                          uint32_t x0, uint32_t end, unsigned long long g0, uint32_t total, uint32_t L,
                                          uint32_t R, const uint8_t* rs) {
@@ -2337,10 +2362,11 @@ __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32
   const int grow = (int)R - (int)L;
   // mark[c]: replacements that end before chunk c, where that number differs from chunk c - 1's; else 0
   uint8_t* const mark = reinterpret_cast<uint8_t*>(scr);
-  uint16_t* const os = reinterpret_cast<uint16_t*>(scr + 64);  // output offset of every replacement
+  uint16_t* const os = reinterpret_cast<uint16_t*>(scr + 128);  // output offset of every replacement
   const uint32_t a0 = (uint32_t)g0 & 15u, nch = (total + a0 + 15u) >> 4;  // chunks touched, the first at g0 - a0
   scr[lane] = 0;
   scr[lane + 32u] = 0;
+  if (nch > 256u) scr[lane + 64u] = scr[lane + 96u] = 0;
   const uint32_t cnt = (uint32_t)__popcll(kept);
   const uint32_t incl = warp_incl_scan(cnt, OpSum());
   const uint32_t M = __shfl_sync(0xffffffffu, incl, 31);
@@ -2353,9 +2379,9 @@ __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32
     if (lo + R + (end > last ? end - last : 0u) != total) return false;
   }
   const uint32_t up = R + a0 + 15u;  // (os[i] + up) / 16: the first chunk that starts at or after replacement i's end
-  if (lane < M) {
-    const uint32_t ce = (os[lane] + up) >> 4;
-    if (ce < nch && (lane + 1u == M || ce != (os[lane + 1u] + up) >> 4)) mark[ce] = (uint8_t)(lane + 1u);
+  for (uint32_t i = lane; i < M; i += 32u) {
+    const uint32_t ce = (os[i] + up) >> 4;
+    if (ce < nch && (i + 1u == M || ce != (os[i + 1u] + up) >> 4)) mark[ce] = (uint8_t)(i + 1u);
   }
   __syncwarp();
   uint8_t* const og = out + g0;
@@ -2389,7 +2415,8 @@ __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32
   }
   __syncwarp();
   // from every replacement to the end of its last chunk (or the next one): 1 << lg lanes each
-  const uint32_t lg = R > 16u ? 3u : (M <= 8u ? 2u : 1u);
+  // (as many as about three rounds write it in: 64 bytes by 8 / 16 / 32 lanes, 26 matches, 16 MiB: 49.7 / 43.3 / 47.8 us)
+  const uint32_t lg = R > 64u ? 5u : R > 32u ? 4u : R > 16u ? 3u : (M <= 8u || R > 4u ? 2u : 1u);
 #pragma unroll 1
   for (uint32_t i = lane >> lg; i < M; i += 32u >> lg) {
     const uint32_t o = os[i], nx = i + 1u < M ? os[i + 1u] : total;
@@ -2921,17 +2948,18 @@ __global__ void __launch_bounds__(kThreads, 3)
 
   // Output of one warp region (kModeFree, kModeSmall) that mixes literal bytes and replacements:
   // out[g0, g0 + wtot). This thread's segment of the sub-tile at tb has the kept starts `kept`, its
-  // first x_in bytes covered by an earlier match and V valid bytes. Equal lengths: the replacements
-  // are written over the matches in shared memory and the region copied. At most kPieceMax
-  // matches: literal runs between replacements (warp_emit_pieces); at most kGatherMax: chunks gathered
-  // (emit_gather). Otherwise the bytes are scattered
+  // first x_in bytes covered by an earlier match and V valid bytes. Equal lengths up to 64 bytes: the replacements
+  // are written over the matches in shared memory and the region copied (a longer one by one lane,
+  // byte by byte, held the warp up: 72 MiB of text, one match of 200 bytes in three regions of four, 345 us, gathered
+  // 174). At most kPieceMax matches, or replacements beyond kScatterR: literal runs between
+  // replacements (warp_emit_pieces). As `gathers` says: chunks gathered (emit_gather). Otherwise the bytes are scattered
   // into the warp's staging area (scatter_segments) and copied out, in rounds of as many segments
   // as fit it (a segment that alone outgrows it goes straight to global memory).
   // Lengths that do not add up to wtot (which the arithmetic rules out) report an error.
   auto emit_region = [&](const uint8_t* tb, uint64_t kept, unsigned long long gseg, uint32_t x_in, uint32_t V,
                          unsigned long long g0, uint32_t wtot) {
     const uint32_t x0r = __shfl_sync(0xffffffffu, x_in, 0);
-    if (R == L) {
+    if (R == L && L <= 64u) {
       uint8_t* w = const_cast<uint8_t*>(tb) + sb;  // (a match may run past the segment: those bytes are its own)
       for (uint64_t km = kept; km; km &= km - 1ull) {
         const uint32_t b = (uint32_t)(__ffsll((long long)km) - 1);
@@ -2944,12 +2972,13 @@ __global__ void __launch_bounds__(kThreads, 3)
     }
     const uint32_t vend = __reduce_add_sync(0xffffffffu, V);
     const uint32_t M = __reduce_add_sync(0xffffffffu, (uint32_t)__popcll(kept)), q0 = warp * 2048u;
-    if (M <= kPieceMax) {
+    const bool gather = gathers(M, wtot, R);
+    if (M <= kPieceMax || (R > kScatterR && !gather)) {
       if (!warp_emit_pieces(p.out, tb, kept, q0, q0 + x0r, q0 + vend, g0, wtot, L, R, rs) && lane == 0)
         set_error(p);  // (the arithmetic rules it out)
       return;
     }
-    if (R <= 64u && wtot <= kGatherBytes && M <= kGatherMax) {
+    if (gather) {
       if (!emit_gather(p.out, tb, reinterpret_cast<uint32_t*>(ob) + (size_t)warp * lay.wstage_words, kept, q0, q0 + x0r,
                        q0 + vend, g0, wtot, L, R, rs) &&
           lane == 0)
@@ -3079,8 +3108,8 @@ __global__ void __launch_bounds__(kThreads, 3)
     unsigned long long O =
         p.len_bias + (unsigned long long)((long long)(tstart + cin) - (long long)carry0 + dprefix);
     const bool failed = s_fail != 0;
-    // a region's output of any length is staged in rounds (emit_region)
-    const bool stage_rounds = MODE != kModeMulti && R <= 64u;
+    // a region's output of any length and any R has its path (emit_region)
+    constexpr bool stage_rounds = MODE != kModeMulti;
 
     // ================= pass B, table-driven: every warp region of this whole super-tile is a run of
     // replacements, empty, or (mode 2) a copy of its input. Mode 2: lane r stands for region
@@ -3502,7 +3531,8 @@ __global__ void __launch_bounds__(kThreads, 3)
           }
         }
         }  // kModeMulti, more than 16 matches
-      } else if (fits && !failed) {
+      } else if (MODE == kModeMulti && fits && !failed) {
+        if constexpr (MODE == kModeMulti) {
         // very large expansions: windows of the sub-tile output, byte by byte (the windows
         // share the staging area with the warps' own staging, which the block barrier at the
         // end of every sub-tile keeps apart)
@@ -3524,17 +3554,11 @@ __global__ void __launch_bounds__(kThreads, 3)
               copy_clip(obw, o, src + pos, nk - pos, w0, w1);
               o += nk - pos;
               if (nk >= V) break;
-              if constexpr (MODE == kModeMulti) {  // this match's own replacement
-                const int k = multi_identify(MT, src + nk, n_all - (gseg + nk));
-                if (k < 0) break;  // cannot happen: pass A found this pattern here
-                copy_clip(obw, o, MT.rep[k], MT.R[k], w0, w1);
-                o += MT.R[k];
-                pos = nk + MT.L[k];
-                continue;
-              }
-              copy_clip(obw, o, rs, R, w0, w1);
-              o += R;
-              pos = nk + L;
+              const int k = multi_identify(MT, src + nk, n_all - (gseg + nk));  // this match's own replacement
+              if (k < 0) break;  // cannot happen: pass A found this pattern here
+              copy_clip(obw, o, MT.rep[k], MT.R[k], w0, w1);
+              o += MT.R[k];
+              pos = nk + MT.L[k];
             }
           }
           fence_proxy_async_smem();
@@ -3555,6 +3579,7 @@ __global__ void __launch_bounds__(kThreads, 3)
           }
           if (tid == 0) bulk_wait_read_all();
           __syncthreads();
+        }
         }
       }
       }  // !done
@@ -3710,7 +3735,7 @@ __host__ __device__ constexpr uint32_t region_count(uint32_t mode) { return mode
 __host__ __device__ constexpr uint32_t region_slots(uint32_t mode) { return mode == kModeFree ? 6u : 3u; }
 __host__ __device__ constexpr uint32_t region_tile(uint32_t mode) { return region_count(mode) * kRegion; }
 __host__ __device__ constexpr uint32_t region_slot(uint32_t mode) { return region_tile(mode) + kHaloMax + 48u; }
-static_assert(kGatherScratch <= 1040u + 512u, "emit_gather works in the staging area and the masks behind it");
+static_assert(kGatherScratch <= 1040u, "emit_gather works in the staging area and the masks behind it");
 
 struct LayoutW {
   uint32_t slots, masks, scratch, pat, rep, tab16, srec, wtab, wrec, total;
@@ -4955,7 +4980,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
           x_in = ee > lane * 64u ? ee - lane * 64u : 0u;
         }
         const uint32_t V = vb > lane * 64u ? min(vb - lane * 64u, 64u) : 0u;
-        if (!cut && R == L && L <= kHaloMax) {
+        if (!cut && R == L && L <= 64u) {
           // equal lengths: written over the matches in shared memory, then copied (a match may run
           // past the region: those bytes are its own)
           uint8_t* const w = tb + qs + 64u * lane;
@@ -4966,10 +4991,10 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
           fence_proxy_async_smem();  // the slot is loaded again by the async proxy
           __syncwarp();
           warp_emit_literal(p.out, tb, g0, e.y, e.z);
-        } else if (!cut && (R > 64u || e.w <= kRegionPieces)) {
+        } else if (!cut && (e.w <= kRegionPieces || (R > kScatterR && !gathers(e.w, e.y, R)))) {
           if (!warp_emit_pieces(p.out, tb, kept, qs, e.z, qs + vb, g0, e.y, L, R, rs) && lane == 0)
             set_error(p);  // (the arithmetic rules it out)
-        } else if (!cut && e.w <= kGatherMax && e.y <= kGatherBytes) {
+        } else if (!cut && gathers(e.w, e.y, R)) {
           if (!emit_gather(p.out, tb, reinterpret_cast<uint32_t*>(stg), kept, qs, e.z, qs + vb, g0, e.y, L, R, rs) &&
               lane == 0)
             set_error(p);  // (the arithmetic rules it out)
