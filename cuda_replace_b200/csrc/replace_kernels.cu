@@ -39,7 +39,7 @@ namespace {
 
 constexpr unsigned long long kSpinLimitNs = 2000000000ull;  // 2 s per bounded wait
 
-__host__ __device__ __forceinline__ uint32_t align_up_u32(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
+__host__ __device__ __forceinline__ constexpr uint32_t align_up_u32(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
 // ---------------------------------------------------------------- shared memory layout
 struct Layout {
@@ -1055,10 +1055,13 @@ struct LayoutS {
 };
 
 // ratio: kModeMulti, output staging per input byte (1..3). The other modes stage 2 KiB per warp
-// whatever R is: a region whose output is larger is staged and written in rounds.
+// whatever R is: a region whose output is larger is staged and written in rounds. One apply of a pattern of 3 or 4
+// bytes that overlaps itself stages 1.5 KiB: with its tables, 2 KiB left an SM two CTAs of three (256 MiB of text, an absent
+// pattern of 3 bytes 217 -> 188 us, of 4 bytes 240 -> 208; 2 bytes fit three either way and are the slower for the second
+// round: `AA` in a sequence 561 us with 2 KiB, 587 with 1.5).
 // sets: per-super-tile tables held at once (2 when one super-tile's pass A overlaps the
 // previous one's look-back and pass B).
-__host__ __device__ __forceinline__ LayoutS make_layout_s(uint32_t mode, uint32_t L, uint32_t R, uint32_t nsub,
+__host__ __device__ __forceinline__ constexpr LayoutS make_layout_s(uint32_t mode, uint32_t L, uint32_t R, uint32_t nsub,
                                                           uint32_t ratio = 1, uint32_t sets = 1) {
   LayoutS s{};
   uint32_t off = 0;
@@ -1066,7 +1069,7 @@ __host__ __device__ __forceinline__ LayoutS make_layout_s(uint32_t mode, uint32_
   s.in0 = off;
   off += kNBuf * s.inbytes;
   {
-    const uint32_t words = (2048u * ratio + 48u) / 4u;
+    const uint32_t words = ((mode == kModeSmall && L > 2u && sets > 1u ? 1504u : 2048u * ratio) + 48u) / 4u;
     s.wstage_words = mode == kModeMulti ? words + words / 32u + 2u : words;  // (a multiple of 4: 16-byte rows)
     s.wstage_cap = words * 4u;
   }
@@ -5284,6 +5287,10 @@ void prepare_pattern_fields(ReplaceParams& p, const uint8_t* pat, uint32_t L) {
 uint32_t tile_kernel_smem_bytes(uint32_t mode, uint32_t L, uint32_t R) { return make_layout(mode, L, R).total; }
 // The super-tile kernel's super-tiles in a single apply and in a multi-pattern stage: 64 KiB.
 constexpr uint32_t kApplySub = 4;
+// Three CTAs of the super-tile kernel fit an SM (228 KiB; each takes 1 KiB more, and 0.9 or 1.3 KiB of static memory).
+static_assert(3u * (make_layout_s(kModeSmall, 4, 16, kApplySub, 1, 2).total + 2048u) <= 228u * 1024u, "L = 4");
+static_assert(3u * (make_layout_s(kModeSmall, 2, 16, kApplySub, 1, 2).total + 2048u) <= 228u * 1024u, "L = 2");
+static_assert(3u * (make_layout_s(kModeFree, 64, 64, kApplySub, 1, 2).total + 3072u) <= 228u * 1024u, "free");
 static_assert(kApplySub != kRegionSub, "nsub tells the kernel");
 
 // Which kernel takes an input. The region kernel has the shorter path for one super-tile and more of
