@@ -5306,14 +5306,21 @@ static_assert(kApplySub != kRegionSub, "nsub tells the kernel");
 //   a run, L = 1     16.8/10.9  22.0/21.5  57.4/57.2  98.3/102
 //   a run, L = 2     16.1/15.4  18.9/21.8  33.1/49.2  55.7/86.4 (overlapping itself: up to 8 MiB)
 //   AA in ACGT       42.5/22.8  50.9/42.3  130/117    223/214 (the same: by the slower loser, the run)
-// Bordered patterns of 5 to 64 bytes are always the region kernel's (64 MiB run of 6: 397 -> 122 us;
-// 32 MiB of rule lines, L = 40, which the tile kernel took before: 1020 -> 64 us).
+// Free patterns longer than 64 bytes in text, one in three regions of four (its search walks to the next match of any
+// region before, and a region's matches are verified by one lane each, which its few warps per SM hide less):
+//                      8 MiB      16 MiB     24 MiB     32 MiB     48 MiB     64 MiB
+//   200 bytes        63.7/45.9  67.4/65.8  72.8/93.4   112/101    124/150    170/191    (up to 16 MiB)
+//   64 bytes         38.9/30.5  41.3/40.4  45.5/51.7  62.5/58.7  70.3/79.6  92.6/102
+// Bordered patterns of 5 to 64 bytes are always the region kernel's: the super-tile kernel's tables over carries cost more
+// than a second read at any size, for sparse matches too. Before / in the region kernel, 64 MiB: `papap` in text, one in 4 KiB,
+// 185/95, `ACACA` in a sequence 219/112, `mumumumumumu` 250/116, a 32-byte rule line 832/96, a run of 6 391/60; 512 MiB:
+// 1152/635, 1416/822, 1593/799, 6362/675, 2497/346. 40 bytes, which the tile kernel took, 32 MiB: 1020/64.
 uint32_t super_tile(const ReplaceParams& p) { return super_tile_bytes(p); }
 
 uint32_t super_nsub(uint32_t mode, uint32_t L, unsigned long long n) {
   if (mode == kModeMulti) return kApplySub;
   if (mode == kModeSmall && L > 4u) return kRegionSub;
-  const unsigned long long most = mode == kModeFree ? 64ull << 20 : 8ull << 20;
+  const unsigned long long most = (mode == kModeFree ? (L <= 64u ? 64ull : 16ull) : 8ull) << 20;
   if (mode == kModeFree || (mode == kModeSmall && L >= 2u)) return n <= most ? kRegionSub : kApplySub;
   return 0;
 }
