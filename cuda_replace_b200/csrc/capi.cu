@@ -378,10 +378,12 @@ cudaError_t upload_host(Session* s, uint8_t* dst, const uint8_t* src, size_t len
 }
 
 // The session buffer to caller memory dst[0, s->len): a large pageable dst by way of a pooled page-locked
-// block in four pieces, each copied into dst on the host threads while the next one downloads. Into fresh
-// memory, whose first touches bound the copies, ms for 1 / 2 / 4 / 8 / 16 pieces: 4 MiB 0.51 / 0.19 / 0.21 / 0.21 / 0.21,
-// 8 MiB 1.15 / 0.68 / 0.30 / 0.35 / 0.35, 16 MiB 1.80 / 0.79 / 0.46 / 0.46 / 0.60, 64 MiB 3.8 / 2.9 / 3.0 / 3.4 / 4.6, 128 MiB
-// 7.4 / 5.3 / 5.6 / 6.5 / 7.0. Smaller pieces than 1 MiB are no work for several threads.
+// block in pieces, each copied into dst on the host threads while the next one downloads. Eight up to 24 MiB, so that a
+// piece lands before the copy threads go to sleep (four took 0.49 or 0.71 ms for 16 MiB, from run to run), four above,
+// where the first touches of dst's pages bound the copies. Median ms into fresh memory, one download and one
+// copy / 4 / 8 / 16 pieces: 8 MiB 1.31 / 0.32 to 0.57 / 0.35 / 0.35, 16 MiB 0.55 / 0.67 / 0.46 / 0.58, 24 MiB 0.70 / 0.59 / 0.57 / 0.60,
+// 32 MiB 1.78 / 1.57 / 1.81 / -, 64 MiB 3.8 / 3.0 / 3.4 / 4.6, 128 MiB 6.6 / 5.6 / 6.5 / 7.0. Pieces below 1 MiB are no work
+// for several threads.
 cudaError_t download_host(Session* s, uint8_t* dst) {
   cudaError_t e = cudaSuccess;
   if (s->len < (3u << 20) || host_is_pinned(dst)) {
@@ -391,8 +393,9 @@ cudaError_t download_host(Session* s, uint8_t* dst) {
   }
   uint8_t* host = static_cast<uint8_t*>(pinned_pool().get(s->len, &e));
   if (!host) return e;
-  const size_t piece = std::max<size_t>((size_t)1 << 20, round_up((s->len + 3) / 4, (size_t)1 << 18));
-  static_assert(kUnifiedChunks >= 4, "an event per piece");
+  const size_t pieces = s->len <= ((size_t)24 << 20) ? 8 : 4;
+  const size_t piece = std::max<size_t>((size_t)1 << 20, round_up((s->len + pieces - 1) / pieces, (size_t)1 << 18));
+  static_assert(kUnifiedChunks >= 8, "an event per piece");
   CopyOut copyout;
   copyout.open(s->device);
   for (size_t off = 0, k = 0; e == cudaSuccess && off < s->len; off += piece, ++k) {

@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 MiB = 1 << 20
 
 
-@pytest.mark.parametrize("n", [1, 3 * MiB - 1, 3 * MiB, 4 * MiB - 1, 4 * MiB, 4 * MiB + 1, 5 * MiB - 7, 33 * MiB + 5, 96 * MiB + 1])
+@pytest.mark.parametrize("n", [1, 3 * MiB - 1, 3 * MiB, 4 * MiB - 1, 4 * MiB, 4 * MiB + 1, 5 * MiB - 7, 24 * MiB, 24 * MiB + 1, 33 * MiB + 5, 96 * MiB + 1])
 def test_result_and_unified_into(cr_lib, n):
     base = np.random.default_rng(n).integers(0, 255, size=MiB + 13, dtype=np.uint8)
     src = np.resize(base, n).tobytes()
