@@ -345,21 +345,34 @@ bool host_is_pinned(const void* p) {
   return a.type == cudaMemoryTypeHost;
 }
 
-// Pieces of a pageable transfer staged through page-locked memory: large enough to copy on all host
-// threads, small enough that the copy of one hides behind the link's work on the one before.
+// Staged transfers of pageable memory under way in the process. One or two are cut into pieces, so that
+// their copies on the host threads hide behind their own work on the link; one among more goes in one piece (up to
+// 32 MiB), whose copy hides behind the others'. Sessions that load, replace and read back 12 / 24 MiB documents in a loop, ms,
+// one piece of up to 32 MiB always / pieces always / so: one thread 2.8, 3.9 / 1.0, 1.7 / 1.0, 1.7; two 2.0, 2.9 / 1.4, 2.4 /
+// 1.5, 2.5; four 2.0, 4.4 / 2.2, 4.4 / 1.8, 4.1; eight 4.2, 9.0 / 4.7, 8.6 / 3.7, 8.1.
+std::atomic<int> g_staged{0};
+struct StagedTransfer {
+  const bool in_pieces = g_staged.fetch_add(1, std::memory_order_relaxed) < 2;
+  ~StagedTransfer() { g_staged.fetch_sub(1, std::memory_order_relaxed); }
+};
+
+// Upload pieces: large enough to copy on all host threads, small enough to pipeline.
 size_t stage_piece(size_t len) {
-  return std::min<size_t>((size_t)32 << 20, std::max<size_t>((size_t)1 << 20, round_up(len / 16, (size_t)1 << 18)));
+  const size_t piece = len <= ((size_t)16 << 20) ? std::max<size_t>((size_t)1 << 20, len / 8) : std::max<size_t>((size_t)2 << 20, len / 16);
+  return std::min<size_t>((size_t)32 << 20, round_up(piece, (size_t)1 << 18));
 }
 
-// Host -> device copy of len bytes. A large pageable source is staged piece by piece through three
+// Host -> device copy of len bytes. A large pageable source is staged piece by piece through up to three
 // page-locked slots filled by the host threads (a pageable cudaMemcpy goes through the driver's
 // single-threaded staging; in pieces of 32 MiB the first copy hid behind nothing: 12 MiB took 2.1 ms,
-// now 0.5, 64 MiB 4.0 ms, now 2.5; the copies and the link share the host's memory bandwidth).
+// now 0.5, 64 MiB 4.0 ms, now 2.5; the copies and the link share the host's memory bandwidth). Below 5 MiB the driver's
+// staging is as fast, and leaves the host threads to others.
 cudaError_t upload_host(Session* s, uint8_t* dst, const uint8_t* src, size_t len, cudaStream_t st) {
-  if (len < (3u << 20) || host_is_pinned(src)) return cudaMemcpyAsync(dst, src, len, cudaMemcpyHostToDevice, st);
-  const size_t piece = stage_piece(len);
+  if (len < (5u << 20) || host_is_pinned(src)) return cudaMemcpyAsync(dst, src, len, cudaMemcpyHostToDevice, st);
+  const StagedTransfer transfer;
+  const size_t piece = transfer.in_pieces ? stage_piece(len) : std::min<size_t>(round_up(len, (size_t)1 << 18), (size_t)32 << 20);
   cudaError_t e = cudaSuccess;
-  uint8_t* stage = static_cast<uint8_t*>(pinned_pool().get(3 * piece, &e));
+  uint8_t* stage = static_cast<uint8_t*>(pinned_pool().get(std::min<size_t>(3, (len + piece - 1) / piece) * piece, &e));
   if (!stage) return e;
   for (int b = 0; b < 3 && e == cudaSuccess; ++b)
     if (!s->ev_stage[b]) e = cudaEventCreateWithFlags(&s->ev_stage[b], cudaEventDisableTiming);
@@ -393,6 +406,15 @@ cudaError_t download_host(Session* s, uint8_t* dst) {
   }
   uint8_t* host = static_cast<uint8_t*>(pinned_pool().get(s->len, &e));
   if (!host) return e;
+  const StagedTransfer transfer;
+  if (!transfer.in_pieces && s->len <= ((size_t)32 << 20)) {
+    e = cudaMemcpyAsync(host, s->buf, s->len, cudaMemcpyDeviceToHost, s->stream);
+    const cudaError_t se = cudaStreamSynchronize(s->stream);
+    if (e == cudaSuccess) e = se;
+    if (e == cudaSuccess) crb::parallel_memcpy(dst, host, s->len);
+    pinned_pool().put(host);
+    return e;
+  }
   const size_t pieces = s->len <= ((size_t)24 << 20) ? 8 : 4;
   const size_t piece = std::max<size_t>((size_t)1 << 20, round_up((s->len + pieces - 1) / pieces, (size_t)1 << 18));
   static_assert(kUnifiedChunks >= 8, "an event per piece");
