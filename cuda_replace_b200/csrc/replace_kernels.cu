@@ -781,9 +781,8 @@ __global__ void __launch_bounds__(kThreads) replace_tiles_kernel(const __grid_co
 }
 
 // ============================================================================ query kernel
-// One CTA re-derives the kept starts of one tile from the tile records of the last apply
-// (exact carry-in from the predecessor's inclusive prefix) and counts those before limit.
-template <int MODE>
+// One CTA re-derives the kept starts of one tile from the tile records of the last apply by the tile
+// kernel (kModeLarge; exact carry-in from the predecessor's inclusive prefix) and counts those before limit.
 __global__ void __launch_bounds__(kThreads) query_tile_kernel(const __grid_constant__ ReplaceParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t s_bar;
@@ -850,15 +849,9 @@ __global__ void __launch_bounds__(kThreads) query_tile_kernel(const __grid_const
     for (uint32_t seg = 0; seg < (uint32_t)kThreads; ++seg) {
       const uint32_t base = seg * 64u;
       if (base >= lim) break;
-      uint64_t kept;
-      uint32_t xn;
-      if (MODE == kModeFree) {
-        kept = masks[seg];
-        xn = 0;
-      } else if (x >= 64u) {
-        kept = 0;
-        xn = x - 64u;
-      } else {
+      uint64_t kept = 0;
+      uint32_t xn = x - 64u;
+      if (x < 64u) {
         const Walk w = seg_walk(masks[seg], x, L, p.inv_l, p.stride_mask);
         kept = w.kept;
         xn = w.end > 64u ? w.end - 64u : 0u;
@@ -2694,7 +2687,7 @@ __global__ void __launch_bounds__(kThreads, 3)
           ks_warp_tables<3>(mask, p.inv_l, p.stride_mask, srec + tid * 3u, wtab, &s_dense[set][j * kWarps + warp]);
         } else if (L == 4u) {
           ks_warp_tables<4>(mask, p.inv_l, p.stride_mask, srec + tid * 4u, wtab, &s_dense[set][j * kWarps + warp]);
-        } else {
+        } else if constexpr (SEG) {
           // segment tables in shared memory, then lanes-over-carries walks of the warp's
           // own 32 segments (only rows of this warp are read: a warp barrier suffices)
           uint16_t* segtab = reinterpret_cast<uint16_t*>(smem + lay.segtab);
@@ -2723,7 +2716,7 @@ __global__ void __launch_bounds__(kThreads, 3)
 
     // ================= fold the sub-tiles into the super-tile function
     // (warp 1, so that warp 0 can start the previous super-tile's look-back at the same time)
-    const bool use_rec = kFreeLike || L <= 4u;
+    const bool use_rec = kFreeLike || !SEG || L <= 4u;  // (one apply: bordered patterns up to 4 bytes)
     const uint32_t tag = p.epoch & 0xFFFFFFu;
     unsigned long long fr_cnt = 0;  // kModeFree: lane 0 of warp 1
     long long fr_lco = 0;
@@ -2803,14 +2796,14 @@ __global__ void __launch_bounds__(kThreads, 3)
       const uint32_t* wt = reinterpret_cast<const uint32_t*>(wtab_b);
       bool bad = false;    // some region is not covered from some carry
       bool mixed = false;  // some region is neither covered nor free of kept starts
-      if (use_rec && m <= 4u) {
+      if (!SEG || (use_rec && m <= 4u)) {
         if (L == 2u)
           fold_small_rec<2>(wt, s_dense[set], wrec_b, subrec_b, m, whole, &bad, &mixed, &sup_cnt, &sup_carry);
         else if (L == 3u)
           fold_small_rec<3>(wt, s_dense[set], wrec_b, subrec_b, m, whole, &bad, &mixed, &sup_cnt, &sup_carry);
         else
           fold_small_rec<4>(wt, s_dense[set], wrec_b, subrec_b, m, whole, &bad, &mixed, &sup_cnt, &sup_carry);
-      } else
+      } else if constexpr (SEG) {
 #pragma unroll 1
       for (uint32_t j = 0; j < m; ++j) {
         uint8_t* wrec = wrec_b + (size_t)j * kWarps * L;
@@ -2841,6 +2834,7 @@ __global__ void __launch_bounds__(kThreads, 3)
         const uint32_t tx = __shfl_sync(0xffffffffu, y, sup_carry);
         sup_cnt += tc;
         sup_carry = tx;
+      }
       }
       noin = !whole ? 0u : (!__any_sync(0xffffffffu, bad) ? 1u : (!__any_sync(0xffffffffu, mixed) ? 2u : 0u));
       if (use_rec) {
@@ -3044,7 +3038,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     uint8_t* const wtab_b = smem + lay.wtab + set * lay.wtab_set;
     uint8_t* const wrec_b = smem + lay.wrec + set * lay.wrec_set;
     uint8_t* const subrec_b = smem + lay.subrec + set * lay.subrec_set;
-    const bool use_rec = kFreeLike || L <= 4u;
+    const bool use_rec = kFreeLike || !SEG || L <= 4u;  // (one apply: bordered patterns up to 4 bytes)
     const uint32_t tag = p.epoch & 0xFFFFFFu;
     // ================= look back, publish the inclusive prefix
     if (warp == 0) {
@@ -3060,7 +3054,7 @@ __global__ void __launch_bounds__(kThreads, 3)
           ok = lookback_small_rec<3>(p, t, &K, &c, carry0);
         else if (L == 4u)
           ok = lookback_small_rec<4>(p, t, &K, &c, carry0);
-        else
+        else if constexpr (SEG)
           ok = lookback_small(p, t, L, &K, &c, carry0);
       }
       if (!ok) {
@@ -4324,8 +4318,8 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       s_cutlen[s] = 0;
     }
     fence_mbar_init();
-    // one super-tile when every CTA gets at most one (none is taken from a CTA that starts late),
-    // else up to three ahead
+    // one super-tile when every CTA gets at most one (none is taken from a CTA that starts late), else the CTA's
+    // share of the launch, at most one per slot: for this first fill only, later ones are claimed as slots come free
     const uint32_t share = (NT + gridDim.x - 1u) / gridDim.x;
     const uint32_t depth = share < NS ? (share ? share : 1u) : NS;
     for (; issued < depth && !marks; ++issued) {
@@ -5236,8 +5230,8 @@ cudaError_t launch_mode(const ReplaceParams& p, cudaStream_t st, int* grid_out) 
       cudaError_t e = cudaFuncSetAttribute(replace_tiles_kernel<MODE>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       if (e != cudaSuccess) return e;
-      e = cudaFuncSetAttribute(query_tile_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               200 * 1024);
+      if (MODE == kModeLarge)
+        e = cudaFuncSetAttribute(query_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       if (e != cudaSuccess) return e;
       attr_dev_mask |= 1 << (dev & 31);
     }
@@ -5294,9 +5288,9 @@ static_assert(3u * (make_layout_s(kModeFree, 64, 64, kApplySub, 1, 2).total + 30
 static_assert(kApplySub != kRegionSub, "nsub tells the kernel");
 
 // Which kernel takes an input. The region kernel has the shorter path for one super-tile and more of
-// the chip at work on small inputs; its slots hold a super-tile for its load, its look-back and its
-// output, so on large inputs the look-back bounds it, where the super-tile kernel reads the input a second
-// time from L2. Microseconds, super-tile kernel / region kernel:
+// the chip at work on small inputs; on large ones it falls behind the super-tile kernel, which reads the input a
+// second time from L2 (the region kernel's slots hold a super-tile through load, look-back and output; which of
+// them holds it up has not been measured). Microseconds, super-tile kernel / region kernel:
 //                      1 MiB      16 MiB     64 MiB     128 MiB
 //   entity in text   19.6/12.9  24.1/21.0  50.3/54.9  80.3/102
 //   binary deletion  16.4/10.4  21.6/19.1  43.9/42.4  71.5/74.4
@@ -5399,12 +5393,8 @@ cudaError_t launch_replace(const ReplaceParams& p, cudaStream_t st, int* grid_ct
 
 cudaError_t launch_query(const ReplaceParams& p, cudaStream_t st) {
   const uint32_t smem = make_layout(kModeFree, p.L, p.R).total;
-  // the attribute is set by the first launch_replace of the same mode on this device
-  switch (p.mode) {
-    case kModeFree: query_tile_kernel<kModeFree><<<1, kThreads, smem, st>>>(p); break;
-    case kModeSmall: query_tile_kernel<kModeSmall><<<1, kThreads, smem, st>>>(p); break;
-    default: query_tile_kernel<kModeLarge><<<1, kThreads, smem, st>>>(p); break;
-  }
+  // the attribute is set by the first launch_replace of this mode on this device
+  query_tile_kernel<<<1, kThreads, smem, st>>>(p);
   return cudaGetLastError();
 }
 
