@@ -2247,7 +2247,7 @@ __device__ __noinline__ void scatter_direct(uint8_t* out, const uint8_t* src, co
   }
 }
 
-// scatter_segments by R and shape, kept out of line: its fourteen loops would crowd the kernel's instruction
+// scatter_segments by R and shape, kept out of line: its twelve loops would crowd the kernel's instruction
 // cache (inlined, sparse inputs measured 3-4% slower). Shared-memory addresses, 32 bits each.
 __device__ __noinline__ void scatter_any(uint32_t stg, uint32_t src, uint32_t gm, uint32_t pk, uint32_t s0, uint32_t s1,
                                          uint32_t R, uint32_t rs, bool one) {
@@ -2258,16 +2258,21 @@ __device__ __noinline__ void scatter_any(uint32_t stg, uint32_t src, uint32_t gm
     else                                                                \
       scatter_segments<false, RC>(stg, src, gm, pk, s0, s1, R, rs);     \
     break;
-  switch (R < 5u ? R : (R <= 16u ? 5u : 6u)) {  // the same in every lane
+  switch (R < 5u ? R : 5u) {  // the same in every lane
     CRB_SCATTER(0)
     CRB_SCATTER(1)
     CRB_SCATTER(2)
     CRB_SCATTER(3)
     CRB_SCATTER(4)
     CRB_SCATTER(5)
-    CRB_SCATTER(6)
   }
 #undef CRB_SCATTER
+}
+
+// The same for R > 16, apart so that the loops above stay together.
+__device__ __noinline__ void scatter_long(uint32_t stg, uint32_t src, uint32_t gm, uint32_t pk, uint32_t s0, uint32_t s1,
+                                          uint32_t R, uint32_t rs) {
+  scatter_segments<false, 6>(stg, src, gm, pk, s0, s1, R, rs);
 }
 
 // A warp's staged bytes to out[g0, g0 + len): staging byte (g0 & 15) + i holds output byte i. Whole
@@ -2351,18 +2356,22 @@ __device__ __forceinline__ bool gathers(uint32_t M, uint32_t total, uint32_t R) 
   return M <= (R > 4u ? kGatherMax : 16u) && total <= kGatherBytes && R <= 256u;
 }
 static_assert(kGatherBytes + 30u < 512u * 16u && kGatherMax <= 255u, "a mark per chunk, of 8 bits");
-__device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32_t* scr, uint64_t kept, uint32_t qs,
+// MANY: more than four bytes per replacement (up to kGatherMax matches); otherwise at most 16 matches. (Apart, as
+// scatter_long is: with one body for both, and its loops among scatter_any's, the region kernel took 3 to 7% more on sparse
+// matches, `mumumumumumu` in text, 512 MiB, 802 -> 843 us.)
+template <bool MANY>
+__device__ __noinline__ bool emit_gather_as(uint8_t* out, const uint8_t* tb, uint32_t* scr, uint64_t kept, uint32_t qs,
                                          uint32_t x0, uint32_t end, unsigned long long g0, uint32_t total, uint32_t L,
                                          uint32_t R, const uint8_t* rs) {
   const uint32_t lane = threadIdx.x & 31u;
   const int grow = (int)R - (int)L;
   // mark[c]: replacements that end before chunk c, where that number differs from chunk c - 1's; else 0
   uint8_t* const mark = reinterpret_cast<uint8_t*>(scr);
-  uint16_t* const os = reinterpret_cast<uint16_t*>(scr + 128);  // output offset of every replacement
+  uint16_t* const os = reinterpret_cast<uint16_t*>(scr + (MANY ? 128 : 64));  // output offset of every replacement
   const uint32_t a0 = (uint32_t)g0 & 15u, nch = (total + a0 + 15u) >> 4;  // chunks touched, the first at g0 - a0
   scr[lane] = 0;
   scr[lane + 32u] = 0;
-  if (nch > 256u) scr[lane + 64u] = scr[lane + 96u] = 0;
+  if (MANY && nch > 256u) scr[lane + 64u] = scr[lane + 96u] = 0;
   const uint32_t cnt = (uint32_t)__popcll(kept);
   const uint32_t incl = warp_incl_scan(cnt, OpSum());
   const uint32_t M = __shfl_sync(0xffffffffu, incl, 31);
@@ -2375,9 +2384,14 @@ __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32
     if (lo + R + (end > last ? end - last : 0u) != total) return false;
   }
   const uint32_t up = R + a0 + 15u;  // (os[i] + up) / 16: the first chunk that starts at or after replacement i's end
-  for (uint32_t i = lane; i < M; i += 32u) {
+  auto mark_end = [&](uint32_t i) {
     const uint32_t ce = (os[i] + up) >> 4;
     if (ce < nch && (i + 1u == M || ce != (os[i + 1u] + up) >> 4)) mark[ce] = (uint8_t)(i + 1u);
+  };
+  if (MANY) {
+    for (uint32_t i = lane; i < M; i += 32u) mark_end(i);
+  } else if (lane < M) {
+    mark_end(lane);
   }
   __syncwarp();
   uint8_t* const og = out + g0;
@@ -2412,7 +2426,7 @@ __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32
   __syncwarp();
   // from every replacement to the end of its last chunk (or the next one): 1 << lg lanes each
   // (as many as about three rounds write it in: 64 bytes by 8 / 16 / 32 lanes, 26 matches, 16 MiB: 49.7 / 43.3 / 47.8 us)
-  const uint32_t lg = R > 64u ? 5u : R > 32u ? 4u : R > 16u ? 3u : (M <= 8u || R > 4u ? 2u : 1u);
+  const uint32_t lg = MANY ? (R > 64u ? 5u : R > 32u ? 4u : R > 16u ? 3u : 2u) : (M <= 8u ? 2u : 1u);
 #pragma unroll 1
   for (uint32_t i = lane >> lg; i < M; i += 32u >> lg) {
     const uint32_t o = os[i], nx = i + 1u < M ? os[i + 1u] : total;
@@ -2424,6 +2438,13 @@ __device__ __noinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32
   }
   __syncwarp();
   return true;
+}
+
+__device__ __forceinline__ bool emit_gather(uint8_t* out, const uint8_t* tb, uint32_t* scr, uint64_t kept, uint32_t qs,
+                                            uint32_t x0, uint32_t end, unsigned long long g0, uint32_t total, uint32_t L,
+                                            uint32_t R, const uint8_t* rs) {
+  return R > 4u ? emit_gather_as<true>(out, tb, scr, kept, qs, x0, end, g0, total, L, R, rs)
+                : emit_gather_as<false>(out, tb, scr, kept, qs, x0, end, g0, total, L, R, rs);
 }
 
 // Input length, output range and super-tile count of the job described by p.
@@ -3016,6 +3037,8 @@ __global__ void __launch_bounds__(kThreads, 3)
       __syncwarp();  // the masks (and the last round's copies) are done
       if (direct)
         scatter_direct(p.out + (gr & ~15ull), src, gm, pk, s0, R, rs);
+      else if (R > 16u)
+        scatter_long(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs));
       else
         scatter_any(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs), one);
       __syncwarp();
@@ -3722,7 +3745,9 @@ constexpr uint32_t kLoader = kWorkers, kPublisher = kWorkers + 1, kLookback = kW
 constexpr uint32_t kRegionThreads = (kWorkers + 2 + kLookbacks) * 32;
 constexpr uint32_t kRegionSub = 1;   // nsub of an apply that takes the region kernel (its super-tiles: region_tile)
 constexpr uint32_t kHaloMax = 272;   // bytes after a super-tile held with it
-constexpr uint32_t kRegionPieces = 1;  // regions with up to this many matches are written as pieces
+// Regions with up to this many matches are written as pieces, and of replacements over 64 bytes up to twice as many
+// (rule lines of 40 bytes made 100, mostly one or two per region, 256 MiB: 341 us, with two gathered 383).
+constexpr uint32_t kRegionPieces = 1;
 constexpr unsigned long long kPipeLimitNs = 6000000000ull;  // bounded wait inside a CTA (a look-back may take 2 s)
 // Regions of a super-tile (a worker warp each; 24 workers are one or two teams) and slots. A slot is
 // held from its load's start to its output's end, some 10,000 cycles of which the look-back and the load are
@@ -4890,6 +4915,8 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       __syncwarp();  // the masks are written, the last round's bytes read
       if (direct)
         scatter_direct(p.out + (gr & ~15ull), src, gm, pk, s0, R, rs);
+      else if (R > 16u)
+        scatter_long(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs));
       else
         scatter_any(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs), one);
       __syncwarp();
@@ -4988,12 +5015,15 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
           fence_proxy_async_smem();  // the slot is loaded again by the async proxy
           __syncwarp();
           warp_emit_literal(p.out, tb, g0, e.y, e.z);
-        } else if (!cut && (e.w <= kRegionPieces || (R > kScatterR && !gathers(e.w, e.y, R)))) {
+        } else if (!cut && e.w <= (R > 64u ? 2u * kRegionPieces : kRegionPieces)) {
           if (!warp_emit_pieces(p.out, tb, kept, qs, e.z, qs + vb, g0, e.y, L, R, rs) && lane == 0)
             set_error(p);  // (the arithmetic rules it out)
         } else if (!cut && gathers(e.w, e.y, R)) {
           if (!emit_gather(p.out, tb, reinterpret_cast<uint32_t*>(stg), kept, qs, e.z, qs + vb, g0, e.y, L, R, rs) &&
               lane == 0)
+            set_error(p);  // (the arithmetic rules it out)
+        } else if (!cut && R > kScatterR) {
+          if (!warp_emit_pieces(p.out, tb, kept, qs, e.z, qs + vb, g0, e.y, L, R, rs) && lane == 0)
             set_error(p);  // (the arithmetic rules it out)
         } else {
           emit_scatter(tb + qs, kept, x_in, V, g0, e.y, !cut, write, slot);
