@@ -6,8 +6,8 @@
 //   suppress  cuda_replace.cu:737-884, 905-968   (thread-0 / <<<1,1>>> serial greedy)
 //   scan      cuda_replace.cu:237-352, 1223-1244 (three-stage scan, 32-bit local offsets)
 //   scatter   cuda_replace.cu:1391-1608          (u16 padded array, range-sliced expand)
-// Here all four are one launch, of one of three kernels (super_nsub): the region kernel (inputs up to 64 MiB, and every
-// pattern of 5 to 64 bytes that overlaps itself), the super-tile kernel (larger inputs, segmented launches, stages
+// Here all four are one launch, of one of three kernels (super_nsub): the region kernel (inputs up to 64, 16 or 8 MiB by
+// pattern, and every pattern of 5 to 64 bytes that overlaps itself), the super-tile kernel (larger inputs, segmented launches, stages
 // of several pairs), both described where they stand, and the tile kernel (longer patterns that overlap
 // themselves, and the entry point that allocates nothing):
 //   1. TMA (cp.async.bulk) stages a 16 KiB tile plus an (L-1)-byte halo in shared memory.
@@ -3743,9 +3743,8 @@ namespace {
 
 constexpr uint32_t kRegion = 2048;
 constexpr uint32_t kWorkers = 24;  // worker warps
-// control warps (the look-backs of successive super-tiles alternate between two warps: one takes
-// most of the 4400 cycles that two super-tiles take at DRAM speed, nearly all of it the round trip to the
-// records)
+// control warps (the look-backs of successive super-tiles alternate between two warps: with one, a look-back, 2,300
+// cycles and more of round trips to the records, held up the next; a third changed nothing)
 constexpr uint32_t kLoader = kWorkers, kPublisher = kWorkers + 1, kLookback = kWorkers + 2, kLookbacks = 2;
 constexpr uint32_t kRegionThreads = (kWorkers + 2 + kLookbacks) * 32;
 constexpr uint32_t kRegionSub = 1;   // nsub of an apply that takes the region kernel (its super-tiles: region_tile)
@@ -3755,8 +3754,8 @@ constexpr uint32_t kHaloMax = 272;   // bytes after a super-tile held with it
 constexpr uint32_t kRegionPieces = 1;
 constexpr unsigned long long kPipeLimitNs = 6000000000ull;  // bounded wait inside a CTA (a look-back may take 2 s)
 // Regions of a super-tile (a worker warp each; 24 workers are one or two teams) and slots. A slot is
-// held from its load's start to its output's end, some 10,000 cycles of which the look-back and the load are
-// most, so many small super-tiles in flight keep DRAM busier than few large ones; the functions of
+// held from its load's start to its output's end. Many small super-tiles in flight measured faster than few large
+// ones (12 regions in six slots, with the running sums, against 24 in three: 64 MiB of random bytes 47 -> 41 us); the functions of
 // bordered patterns cost the control warps more per super-tile, so theirs are the larger ones.
 __host__ __device__ constexpr uint32_t region_count(uint32_t mode) { return mode == kModeFree ? 12u : 24u; }
 __host__ __device__ constexpr uint32_t region_slots(uint32_t mode) { return mode == kModeFree ? 6u : 3u; }
