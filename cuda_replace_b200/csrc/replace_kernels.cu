@@ -2171,10 +2171,10 @@ __device__ __forceinline__ void sts8(uint32_t a, uint32_t v) { asm volatile("st.
 // Bound by instruction issue; before, each lane walked its own matches and emitted words one after
 // the other, which cost a warp as much as its busiest lane at every step: 64 MiB of text, every
 // blank replaced by three bytes, 340 -> 115 us; line ends made CRLF, 149 -> 97 us.
-// A replacement of 17 bytes and more is stored by the whole warp, match by match (its own lane writing it byte by
-// byte held the others up: 64 matches per region made 20 / 48 / 64 bytes, 16 MiB: 133 / 264 / 340 us, so 71 / 79 / 78;
-// the word-by-word walk before this kernel 57 / 64 / 69, which emit_gather beats for up to 128 matches).
-// ONE: L = 1 and every byte valid (literal = not kept). RC: R, 5 for 5 to 16 bytes, 6 for more.
+// Long replacements are stored by the whole warp, match by match, unless they are many (scatters_long; their own lane
+// writing them byte by byte holds the others up: 64 matches per region made 20 / 48 / 64 bytes, 16 MiB: 133 / 264 / 340 us, so
+// 71 / 79 / 78; the word-by-word walk before this kernel 57 / 64 / 69, which emit_gather beats for up to 200 matches).
+// ONE: L = 1 and every byte valid (literal = not kept). RC: R, 5 for any R > 4 (each by its own lane), 6 by the whole warp.
 template <bool ONE, int RC>
 __device__ __forceinline__ void scatter_half(uint32_t stg, uint32_t base, uint32_t v, uint32_t C, uint32_t K, uint32_t below,
                                              uint32_t R, uint32_t rep4, uint32_t rs) {
@@ -2197,8 +2197,7 @@ __device__ __forceinline__ void scatter_half(uint32_t stg, uint32_t base, uint32
       if (lit) sts8(d, v);
       uint32_t at = stg + base;
       for (uint32_t km = K; km; km &= km - 1u, at += R) {
-        const uint32_t lo = (km & (0u - km)) - 1u;  // the bytes before the match
-        const uint32_t o = at + (ONE ? (uint32_t)__popc(~K & lo) : (uint32_t)__popc(C & lo));
+        const uint32_t o = at + (uint32_t)__popc(C & ((km & (0u - km)) - 1u));
         for (uint32_t r = threadIdx.x & 31u; r < R; r += 32u) sts8(o + r, lds8(rs + r));
       }
       return;
@@ -2269,7 +2268,12 @@ __device__ __noinline__ void scatter_any(uint32_t stg, uint32_t src, uint32_t gm
 #undef CRB_SCATTER
 }
 
-// The same for R > 16, apart so that the loops above stay together.
+// Whether M replacements of R bytes are stored by the whole warp, one match after the other, or each by its own
+// lane: some 12 instructions and 4 for every 32 bytes per match, against 2.4 for every byte from the fifth on in each of the
+// region's 64 halves (253 matches made 17 / 40 bytes, 16 MiB: warp 135 / 167, lane 110 / 224 us; 512 made 20: 236, 142).
+__device__ __forceinline__ bool scatters_long(uint32_t M, uint32_t R) { return R > 16u && M * (96u + R) < 1232u * (R - 4u); }
+
+// The same by the whole warp, apart so that the loops above stay together.
 __device__ __noinline__ void scatter_long(uint32_t stg, uint32_t src, uint32_t gm, uint32_t pk, uint32_t s0, uint32_t s1,
                                           uint32_t R, uint32_t rs) {
   scatter_segments<false, 6>(stg, src, gm, pk, s0, s1, R, rs);
@@ -2346,8 +2350,9 @@ __device__ __noinline__ bool warp_emit_pieces(uint8_t* out, const uint8_t* tb, u
 // Replacements of 5 bytes and more, 16 MiB, the word-by-word walk and (up to 6 KiB of output per region) staging
 // of a warp before / scattered with a lane per match / so: 26 matches per region made 20 bytes 57 / 70 / 35, 64 bytes
 // 64 / 148 / 43, 200 bytes 146 / (in pieces) 79 / 67; 41 made 5 bytes 66 / 57 / 37, 30 bytes 72 / 130 / 47; 64 made 10 bytes
-// 55 / 90 / 45, 64 bytes 69 / 340 / 64; 102 made 10 bytes 68 / 90 / 55, 30 bytes 79 / 186 / 71.
-constexpr uint32_t kGatherMax = 128, kGatherBytes = 8128, kGatherScratch = 512 + 2 * kGatherMax;
+// 55 / 90 / 45, 64 bytes 69 / 340 / 64; 102 made 10 bytes 68 / 90 / 55, 30 bytes 79 / 186 / 71; 128 made 5 / 12 bytes, 64 MiB:
+// 323 / 181 / 130, 349 / 286 / 162. 253 made 5 / 7 bytes, 64 MiB: scattered 158 / 182, gathered 182 / 198.
+constexpr uint32_t kGatherMax = 200, kGatherBytes = 8128, kGatherScratch = 512 + 2 * kGatherMax;
 constexpr uint32_t kScatterR = 1024;  // longest replacement scattered (16-bit lengths of 32 bytes' output)
 // Whether a region of M matches and `total` output bytes is gathered. Up to four bytes per match the scatter's fixed
 // stores are the faster from 17 matches on (64 matches made 1 byte, 72 MiB: 119 gathered, 100 scattered). (R: a chunk
@@ -3027,7 +3032,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     uint4* gm = reinterpret_cast<uint4*>(smem + lay.gmask) + warp * 32u;
     uint8_t* stg = ob + (size_t)warp * lay.wstage_words * 4u;
     gm[lane] = make_uint4((uint32_t)C, (uint32_t)kept, (uint32_t)(C >> 32), (uint32_t)(kept >> 32));
-    const bool one = __all_sync(0xffffffffu, L == 1u && V == 64u && x_in == 0u);
+    const bool one = __all_sync(0xffffffffu, L == 1u && V == 64u && x_in == 0u), by_warp = scatters_long(M, R);
     const uint8_t* src = tb + warp * 2048u;
 #pragma unroll 1
     for (uint32_t s0 = 0; s0 < 32u;) {
@@ -3042,7 +3047,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       __syncwarp();  // the masks (and the last round's copies) are done
       if (direct)
         scatter_direct(p.out + (gr & ~15ull), src, gm, pk, s0, R, rs);
-      else if (R > 16u)
+      else if (by_warp)
         scatter_long(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs));
       else
         scatter_any(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs), one);
@@ -4906,6 +4911,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
     }
     gm[lane] = make_uint4((uint32_t)C, (uint32_t)kept, (uint32_t)(C >> 32), (uint32_t)(kept >> 32));
     const bool one = __all_sync(0xffffffffu, L == 1u && V == 64u && x_in == 0u);
+    const bool by_warp = scatters_long(s_reg[slot][wq].w, R);
 #pragma unroll 1
     for (uint32_t s0 = 0; s0 < 32u;) {  // rounds of as many segments as fit the staging area
       const uint32_t from = __shfl_sync(0xffffffffu, start, s0);
@@ -4919,7 +4925,7 @@ __global__ void __launch_bounds__(kRegionThreads, 1) replace_region_kernel(const
       __syncwarp();  // the masks are written, the last round's bytes read
       if (direct)
         scatter_direct(p.out + (gr & ~15ull), src, gm, pk, s0, R, rs);
-      else if (R > 16u)
+      else if (by_warp)
         scatter_long(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs));
       else
         scatter_any(smem_u32(stg), smem_u32(src), smem_u32(gm), pk, s0, s1, R, smem_u32(rs), one);

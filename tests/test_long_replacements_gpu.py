@@ -10,7 +10,7 @@ from cuda_replace_b200.cuda_replace_wrapper import Session
 pytestmark = pytest.mark.gpu
 
 KiB, MiB = 1 << 10, 1 << 20
-COUNTS = [0, 1, 2, 3, 15, 16, 17, 31, 33, 64, 100, 127, 128, 129, 300, 2048]
+COUNTS = [0, 1, 2, 3, 15, 16, 17, 31, 33, 64, 100, 128, 199, 200, 201, 300, 2048]
 A, B = b"\x80", b"\x81"
 PATTERNS = [A, A + B, A + A, A + B + A, A * 5, A + b"\x82" * 30 + B, A * 40, A + b"\x82" * 62 + B, A + b"\x82" * 63 + B,
             A + b"\x82" * 298 + B]
