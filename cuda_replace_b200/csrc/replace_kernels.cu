@@ -5097,7 +5097,7 @@ __global__ void __launch_bounds__(kThreads) query_super_kernel(const __grid_cons
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ uint32_t s_scan[kWarps];
-  __shared__ uint32_t s_x;
+  __shared__ uint32_t s_x, s_some[kWarps];
   __shared__ unsigned long long s_k;
   __shared__ long long s_last;
   __shared__ uint32_t s_ok;
@@ -5154,35 +5154,31 @@ __global__ void __launch_bounds__(kThreads) query_super_kernel(const __grid_cons
     }
     if (L > 4) mask = verify_tail(mask, tb + sb, ps, L);
     masks[tid] = mask;
+    const uint32_t some = __ballot_sync(0xffffffffu, mask != 0ull);  // segments with candidates: few, mostly
+    if ((tid & 31u) == 0) s_some[tid >> 5] = some;
     __syncthreads();
     if (tid == 0) {
       const unsigned long long lim = rel - (unsigned long long)j * kTile;  // limit relative to this sub-tile
-      uint32_t x = s_x;
+      uint32_t y = s_x;  // blocked until, relative to this sub-tile
       unsigned long long K = s_k;
       long long last = s_last;
-      for (uint32_t seg = 0; seg < (uint32_t)kThreads; ++seg) {
-        const unsigned long long base = (unsigned long long)seg * 64u;
-        uint64_t kept;
-        uint32_t xn;
-        if (MODE == kModeFree) {
-          kept = masks[seg];
-          xn = 0;
-        } else if (x >= 64u) {
-          kept = 0;
-          xn = x - 64u;
-        } else {
-          const Walk w = seg_walk(masks[seg], x, L, p.inv_l, p.stride_mask);
-          kept = w.kept;
-          xn = w.end > 64u ? w.end - 64u : 0u;
+      for (uint32_t w = 0; w < (uint32_t)kWarps; ++w)
+        for (uint32_t sm = s_some[w]; sm; sm &= sm - 1u) {
+          const uint32_t seg = 32u * w + (uint32_t)__ffs((int)sm) - 1u, base = 64u * seg;
+          uint64_t kept = masks[seg];
+          if (MODE != kModeFree) {
+            const uint32_t x = y > base ? y - base : 0u;
+            const Walk k = seg_walk(kept, x < 64u ? x : 64u, L, p.inv_l, p.stride_mask);
+            kept = k.kept;
+            if (kept) y = base + k.end;
+          }
+          if ((unsigned long long)base < lim) {
+            const uint64_t kb = kept & low_bits(lim - base < 64ull ? (uint32_t)(lim - base) : 64u);
+            K += (unsigned long long)__popcll(kb);
+            if (kb) last = (long long)(sstart + base + 63u - (uint32_t)__clzll((long long)kb));
+          }
         }
-        if (base < lim) {
-          const uint64_t kb = kept & low_bits(lim - base < 64ull ? (uint32_t)(lim - base) : 64u);
-          K += (unsigned long long)__popcll(kb);
-          if (kb) last = (long long)(sstart + base + 63u - (uint32_t)__clzll((long long)kb));
-        }
-        x = xn;
-      }
-      s_x = x;
+      s_x = y > (uint32_t)kTile ? y - (uint32_t)kTile : 0u;
       s_k = K;
       s_last = last;
     }
